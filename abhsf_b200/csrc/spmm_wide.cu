@@ -346,11 +346,11 @@ bool spmm_f64_wide(const abhsf_matrix& a, int k, const double* X, int64_t ldx, d
             launch_wide<16, 32>(a, rows, nrows, X + j, ldx, Y + j, ldy, st);
         else if (nrows > 0)
             launch_wide<16, 16>(a, rows, nrows, X + j, ldx, Y + j, ldy, st);
-        if (sliced) {
-            slices_begin(a, p, X + j, ldx, Y + j, ldy, st, cols);
-            slices_end(a, p, X + j, ldx, Y + j, ldy, st, cols);
-        }
         j += cols;
+    }
+    if (sliced) {
+        slices_begin(a, p, X, ldx, Y, ldy, st, k);
+        slices_end(a, p, X, ldx, Y, ldy, st, k);
     }
     return true;
 }

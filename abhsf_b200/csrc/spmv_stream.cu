@@ -27,10 +27,9 @@
 // onto its row's sum in column order, starting from y: the order of the
 // reference CSR's spmv_naive (spmv/bottlenecks/spmv.cpp:58-64), so y is
 // bitwise the same.  A chain (its own kernel, on a side stream forked from
-// the caller's so that it runs beside the others): the lanes form 32
-// products at a time, kChainAhead steps ahead, and every lane adds them in
-// order.  Slices and chains are dealt to warps at
-// preparation time, longest first.  No waits: nothing here can stall on
+// the caller's so that it runs beside the others): 512 products at a time,
+// a segment a lane, added in order to the bit by the rule of chain_sum.cuh.
+// Slices and chains are dealt to warps at preparation time, longest first.  No waits: nothing here can stall on
 // another warp.
 #include <algorithm>
 #include <cstdlib>
@@ -41,6 +40,7 @@
 
 #include <cub/cub.cuh>
 
+#include "chain_sum.cuh"
 #include "common.cuh"
 #include "internal.cuh"
 
@@ -54,7 +54,11 @@ constexpr int kUnroll = 4;        // elements a lane loads per step of a sliced 
 constexpr int kChainWarps = 4;    // warps per CTA of the chain kernel
 constexpr int kChainCtasPerSm = 4;  // register bound of the chain kernel (128 a thread)
 constexpr int kChainGridPerSm = 1;  // chain CTAs per SM in the grid: the rest of the SM is left to the others
-constexpr int kChainAhead = 8;    // chain: steps of 32 products in flight ahead of the sums
+constexpr int kSliceGridPerSm = 3;  // sliced-row CTAs per SM beside chains
+constexpr int kChainGroup = 512;  // chain: elements a warp sums at a time, 16 a lane
+constexpr int kChainTurn = 4;     // chain: a last group of so few segments of 16 is added in turn
+constexpr int kMmCols = 4;        // columns a warp of the SpMM kernels serves
+constexpr int kMmAhead = 2;       // steps a lane of the sliced-row SpMM loads at a time
 constexpr uint32_t kChain = 1u;   // dc_slice::geo: a one-row chain
 constexpr int kMidShift = 20;     // dc_slice::geo: matrix index of a batch
 constexpr int kLenBits = 8;       // lane record: row offset << kLenBits | (length - 1)
@@ -98,6 +102,14 @@ __device__ __forceinline__ double wide(double v) { return v; }
 __device__ __forceinline__ float wide(float v) { return v; }
 __device__ __forceinline__ float wide(uint16_t b) { return __uint_as_float((uint32_t)b << 16); }
 
+// Shared memory of one warp of the chain kernel: two halves of a group's x and
+// values, each lane's 16 padded by 16 bytes.
+template <typename T, typename V>
+__host__ __device__ constexpr int chain_smem_warp()
+{
+    return 2 * 32 * (16 * (int)(sizeof(T) + sizeof(V)) + 32);
+}
+
 // Streamed once: loaded with the evict-first hint so that x stays in L2.
 __device__ __forceinline__ uint32_t ld_stream(const uint32_t* p) { return __ldcs(p); }
 __device__ __forceinline__ double ld_stream(const double* p) { return __ldcs(p); }
@@ -122,14 +134,15 @@ struct dc_args {
     dc_mat A;                // the matrix (B = false)
     const void* x;
     void* y;
-    int64_t ldx, ldy;        // x[i * ldx], y[i * ldy]
+    int64_t ldx, ldy;        // SpMM: x[i * ldx + column], y[i * ldy + column]
+    int cols;                // SpMM: columns
     const dc_mat* mats;      // a batch (B = true): matrix i's arrays, x and y
     const void* const* xs;
     void* const* ys;
 };
 
-// Eight consecutive products from shared memory (every lane the same
-// address: a broadcast), in two or four 16-byte loads.
+// Eight consecutive values from shared memory (16-byte aligned), in two or
+// four 16-byte loads.
 __device__ __forceinline__ void load8(const double* q, double (&t)[8])
 {
 #pragma unroll
@@ -151,41 +164,26 @@ __device__ __forceinline__ void load8(const float* q, float (&t)[8])
     }
 }
 
-// Adds the first nv products of q (shared memory, 16-byte aligned) onto run
-// in order.  The loads of the next eight are issued before the adds of the
-// current eight, so that nothing but the adds themselves lies on the chain.
-template <int N, typename T>
-__device__ __forceinline__ T add_products(T run, const T* q, int nv)
+// Adds nseg runs of 16 products, `stride` values apart in shared memory, onto
+// run one after another (every lane the same: broadcast loads).  Eight
+// products are loaded while the eight before them are added, so that nothing
+// but the adds lies on the chain.
+template <typename T>
+__device__ __forceinline__ T add_in_turn(T run, const T* q, int stride, int nseg)
 {
-    T t[2][8];
-    load8(q, t[0]);
-#pragma unroll
-    for (int b = 0; b < N / 8; ++b) {
-        if (8 * b >= nv)
-            break;
-        if (b + 1 < N / 8)
-            load8(q + 8 * (b + 1), t[(b + 1) & 1]);
+    T t[8], u[8];
+    load8(q, t);
+#pragma unroll 1
+    for (int b = 0; b < nseg; ++b, q += stride) {
+        load8(q + 8, u);
 #pragma unroll
         for (int k = 0; k < 8; ++k)
-            if (8 * b + k < nv)
-                run = dadd(run, t[b & 1][k]);
-    }
-    return run;
-}
-
-// All N products, no tests in the chain.
-template <int N, typename T>
-__device__ __forceinline__ T add_products_full(T run, const T* q)
-{
-    T t[2][8];
-    load8(q, t[0]);
-#pragma unroll
-    for (int b = 0; b < N / 8; ++b) {
-        if (b + 1 < N / 8)
-            load8(q + 8 * (b + 1), t[(b + 1) & 1]);
+            run = dadd(run, t[k]);
+        if (b + 1 < nseg)
+            load8(q + stride, t);
 #pragma unroll
         for (int k = 0; k < 8; ++k)
-            run = dadd(run, t[b & 1][k]);
+            run = dadd(run, u[k]);
     }
     return run;
 }
@@ -225,13 +223,12 @@ __global__ void __launch_bounds__(32 * kWarpsPerCta, kCtasPerSm) k_spmv_slices(d
         const dc_mat& M = mat(sl);
         const T* X = static_cast<const T*>(B ? P.xs[mid] : P.x);
         T* Y = static_cast<T*>(B ? P.ys[mid] : P.y);
-        const int64_t ldx = B ? 1 : P.ldx, ldy = B ? 1 : P.ldy;
         const uint32_t* W = M.words + sl.base + lane;
         const V* Vv = static_cast<const V*>(M.vals) + sl.base + lane;
         // one row per lane, element k of the lane's row at slot 32 k + lane
         const int len = lane < (int)sl.lanes ? (int)(rec & kLenMask) + 1 : 0;
         const int64_t row = (int64_t)sl.brow * S + (int64_t)(rec >> kLenBits);
-        T acc = len ? Y[row * ldy] : T(0);
+        T acc = len ? Y[row] : T(0);
         uint32_t col = 0;
         // values stay in their stored type until their product: a widening
         // at the load would wait for the prefetch it belongs to
@@ -256,7 +253,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerCta, kCtasPerSm) k_spmv_slices(d
 #pragma unroll
             for (int u = 0; u < U; ++u) {
                 col += w[u];
-                x[u] = k0 + u < len ? __ldg(X + (int64_t)col * ldx) : T(0);
+                x[u] = k0 + u < len ? __ldg(X + col) : T(0);
             }
 #pragma unroll
             for (int u = 0; u < U; ++u)
@@ -269,113 +266,238 @@ __global__ void __launch_bounds__(32 * kWarpsPerCta, kCtasPerSm) k_spmv_slices(d
             }
         }
         if (len)
-            Y[row * ldy] = acc;
+            Y[row] = acc;
         sl = nx;
         nx = nn;
         rec = rec_n;
     }
 }
 
+// Asynchronous 4- or 8-byte copy of one element to shared memory.
+template <typename T>
+__device__ __forceinline__ void cp_async(T* dst, const T* src)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;\n" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src),
+                 "n"(sizeof(T))
+                 : "memory");
+}
+
+// The 16 values of a lane's segment (16-byte aligned in shared memory).
+template <typename V>
+__device__ __forceinline__ void load16(const V* q, V (&t)[16])
+{
+    constexpr int N = 16 / (int)sizeof(V);  // values of one 16-byte read
+#pragma unroll
+    for (int k = 0; k < 16 / N; ++k) {
+        union {
+            uint4 u;
+            V v[N];
+        } c;
+        c.u = reinterpret_cast<const uint4*>(q)[k];
+#pragma unroll
+        for (int i = 0; i < N; ++i)
+            t[N * k + i] = c.v[i];
+    }
+}
+
+// A chain as a warp walks it, kChainGroup elements at a time.
+template <typename T, typename V>
+struct chain_pos {
+    int64_t si;   // its place in the schedule
+    int b0, len;  // first element of the group; the row's elements
+    const uint32_t* W;
+    const V* Vv;
+    const T* X;
+    T* y;
+};
+
+template <int S, bool B, typename T, typename V>
+__device__ __forceinline__ void chain_at(const dc_args& P, const dc_slice& sl, chain_pos<T, V>& c)
+{
+    const int mid = (int)(sl.geo >> kMidShift);
+    const dc_mat& M = B ? P.mats[mid] : P.A;
+    c.b0 = 0;
+    c.len = (int)sl.steps;
+    c.W = M.words + sl.base;
+    c.Vv = static_cast<const V*>(M.vals) + sl.base;
+    c.X = static_cast<const T*>(B ? P.xs[mid] : P.x);
+    c.y = static_cast<T*>(B ? P.ys[mid] : P.y) + (int64_t)sl.brow * S + sl.meta;
+}
+
 // The chains: one warp per row, the row's elements in order (each word the
-// absolute column).  Lane l forms the product of element 32 j + l of a group
-// of kChainAhead x 32 and stores it in the warp's shared buffer; every lane
-// then adds the group's products in order, read back by broadcast loads (a
-// shuffle per product would cost more issue slots than the add it feeds).
-// The values and gathered x of the next group are in flight meanwhile, so
-// that the chain of adds -- the one thing that must run in sequence -- does
-// not wait on memory.
+// absolute column), 512 at a time.  Lane l holds elements 16 l .. 16 l + 15 of
+// a group: its segment of chain::sum_group, which adds the group in order
+// without a chain of 512 additions (8.2 cycles each in FP64).  Where that gives
+// up -- a sum that keeps crossing binades, near zero -- every lane adds the
+// products in turn from shared memory.  A warp's rows form one stream of
+// groups: while one is summed, the values and gathered x of the next are on
+// their way into the other half of the warp's shared buffer (cp.async: they
+// take no registers), and so are the words of the one after, whichever rows
+// they belong to.  The places of a group past its row's end hold -0, which
+// leaves any sum as it is.
+// Bound by latency: one warp issues 408 instructions a group, 4.8 cycles each
+// (a lone row of 98,304 ones 0.49 -> 0.20 ms, of N(0,1) products 0.49 -> 0.37,
+// against additions in turn).  R-MAT scale 22 (chains and sliced rows
+// together) 0.574 -> 0.368 ms, the 256-matrix batch 0.861 -> 0.787 ms.  Two
+// CTAs an SM, or the sliced rows two, were slower on the batch (0.87 ms).
 template <int S, int VT, bool B>
 __global__ void __launch_bounds__(32 * kChainWarps, kChainCtasPerSm) k_spmv_chains(dc_args P)
 {
     using T = typename vt_of<VT>::T;
     using V = typename vt_of<VT>::V;
-    constexpr int AH = kChainAhead, G = 32 * AH;
-    __shared__ __align__(16) T sbuf[kChainWarps][G];
+    constexpr int L = 16, G = kChainGroup;
+    static_assert(G == 32 * L, "a segment a lane");
+    // segments 16 bytes apart, so that the lanes' 16-byte reads meet no bank twice
+    constexpr int STX = L + 16 / (int)sizeof(T), STV = L + 16 / (int)sizeof(V);
+    extern __shared__ __align__(16) uint8_t chain_smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int gw = blockIdx.x * kChainWarps + warp;
     if (gw >= P.warps)
         return;
-    T* buf = sbuf[warp];
+    T* xb = reinterpret_cast<T*>(chain_smem + warp * chain_smem_warp<T, V>());
+    V* vb = reinterpret_cast<V*>(xb + 2 * 32 * STX);
     const int64_t s1 = P.wbeg[gw + 1];
+    chain_pos<T, V> cur{}, nxt{}, ahead;  // summed; copied; its words loaded
+    ahead.si = P.wbeg[gw];
+    if (ahead.si >= s1)
+        return;
+    chain_at<S, B>(P, P.slices[ahead.si], ahead);
+    dc_slice after = ahead.si + 1 < s1 ? P.slices[ahead.si + 1] : P.slices[ahead.si];
+    uint32_t w[L];
+    V vq[sizeof(V) < 4 ? L : 1];  // 2-byte values cannot be copied asynchronously
+    auto load_words = [&] {
+        const uint32_t* W = ahead.W + ahead.b0 + lane;
+        const int left = ahead.len - ahead.b0 - lane;  // elements of the row from this lane's first on
+        if (ahead.len - ahead.b0 >= G) {
+#pragma unroll
+            for (int j = 0; j < L; ++j)
+                w[j] = ld_stream(W + 32 * j);
+        } else {
+#pragma unroll
+            for (int j = 0; j < L; ++j)
+                w[j] = 32 * j < left ? ld_stream(W + 32 * j) : 0u;
+        }
+    };
+    auto advance = [&] {  // ahead: the next group (si = s1 at the end)
+        ahead.b0 += G;
+        if (ahead.b0 >= ahead.len && ++ahead.si < s1) {
+            chain_at<S, B>(P, after, ahead);
+            if (ahead.si + 1 < s1)
+                after = P.slices[ahead.si + 1];
+        }
+    };
+    // element 32 j + lane of a group is value lane % 16 of segment 2 j + lane / 16
+    T* const x_to = xb + (lane / L) * STX + lane % L;
+    V* const v_to = vb + (lane / L) * STV + lane % L;
+    auto copy_one = [&](int half, int j, const V* Vv) {
+        cp_async(x_to + half * 32 * STX + 2 * j * STX, nxt.X + w[j]);
+        if constexpr (sizeof(V) >= 4)
+            cp_async(v_to + half * 32 * STV + 2 * j * STV, Vv + 32 * j);
+        else
+            vq[j] = ld_stream(Vv + 32 * j);
+    };
+    auto copy = [&](int half) {  // nxt's values and x
+        const V* Vv = nxt.Vv + nxt.b0 + lane;
+        const int left = nxt.len - nxt.b0 - lane;
+        if (nxt.len - nxt.b0 >= G) {
+#pragma unroll
+            for (int j = 0; j < L; ++j)
+                copy_one(half, j, Vv);
+        } else {
+#pragma unroll
+            for (int j = 0; j < L; ++j)
+                if (32 * j < left)
+                    copy_one(half, j, Vv);
+        }
+    };
+    load_words();
+    nxt = ahead;
+    T y_nxt = *nxt.y;
+    advance();
+    copy(0);
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+    if (ahead.si < s1)
+        load_words();
+    T run = T(0);
+    int half = 0;
 #pragma unroll 1
-    for (int64_t si = P.wbeg[gw]; si < s1; ++si) {
-        const dc_slice sl = P.slices[si];
-        const int mid = (int)(sl.geo >> kMidShift);
-        const dc_mat& M = B ? P.mats[mid] : P.A;
-        const T* X = static_cast<const T*>(B ? P.xs[mid] : P.x);
-        T* Y = static_cast<T*>(B ? P.ys[mid] : P.y);
-        const int64_t ldx = B ? 1 : P.ldx, ldy = B ? 1 : P.ldy;
-        const uint32_t* W = M.words + sl.base;
-        const V* Vv = static_cast<const V*>(M.vals) + sl.base;
-        const int64_t row = (int64_t)sl.brow * S + sl.meta;
-        const int len = (int)sl.steps;
-        // slot j: the value and x of element 32 j + lane of the current
-        // group; the word of the same element of the next group
-        uint32_t wq[AH];
-        V vq[AH];  // widened at the product (see k_spmv_slices)
-        T xq[AH];
+    for (;;) {
+        cur = nxt;
+        if (cur.b0 == 0)
+            run = y_nxt;
+        if constexpr (sizeof(V) < 4) {
 #pragma unroll
-        for (int j = 0; j < AH; ++j) {
-            const int e = 32 * j + lane;
-            wq[j] = e < len ? ld_stream(W + e) : 0u;
+            for (int j = 0; j < L; ++j)
+                v_to[half * 32 * STV + 2 * j * STV] = vq[j];
         }
-#pragma unroll
-        for (int j = 0; j < AH; ++j) {
-            const int e = 32 * j + lane;
-            vq[j] = e < len ? ld_stream(Vv + e) : V(0);
-            xq[j] = e < len ? __ldg(X + (int64_t)wq[j] * ldx) : T(0);
-            wq[j] = e + G < len ? ld_stream(W + e + G) : 0u;
+        const bool more = ahead.si < s1;
+        if (more) {
+            nxt = ahead;
+            if (nxt.b0 == 0)
+                y_nxt = *nxt.y;
+            advance();
+            copy(half ^ 1);
+            if (ahead.si < s1)
+                load_words();
         }
-        T run = Y[row * ldy];
-        // whole groups: the refills clamped to the row (what they fetch past
-        // its end is never used)
-        int b0 = 0;
-#pragma unroll 1
-        for (; b0 + G <= len; b0 += G) {
-            __syncwarp();  // the previous group's products are read
+        asm volatile("cp.async.commit_group;\ncp.async.wait_group 1;\n" ::: "memory");
+        __syncwarp();  // every lane's copies of the current group have landed
+        T p[L];
+        T* xs = xb + half * 32 * STX + lane * STX;
+        {
+            V v[L];
+            load16(xs, p);
+            load16(vb + half * 32 * STV + lane * STV, v);
 #pragma unroll
-            for (int j = 0; j < AH; ++j) {
-                buf[32 * j + lane] = dmul(wide(vq[j]), xq[j]);
-                const int e = b0 + G + 32 * j + lane;  // the same element of the next group
-                vq[j] = ld_stream(Vv + min(e, len - 1));
-                xq[j] = __ldg(X + (int64_t)wq[j] * ldx);
-                wq[j] = ld_stream(W + min(e + G, len - 1));
-            }
+            for (int i = 0; i < L; ++i)
+                p[i] = dmul(wide(v[i]), p[i]);
+        }
+        const int have = cur.len - cur.b0 - L * lane;  // of the lane's segment
+        if (cur.len - cur.b0 < G) {
+#pragma unroll
+            for (int i = 0; i < L; ++i)
+                p[i] = i < have ? p[i] : T(-0.0);
+        }
+        const int nseg = min(32, (cur.len - cur.b0 + L - 1) / L);
+        // a short last group is as fast in turn
+        if (nseg <= kChainTurn || !chain::sum_group<1, L>(run, p, lane)) {
+#pragma unroll
+            for (int i = 0; i < L; ++i)
+                xs[i] = p[i];
             __syncwarp();
-            run = add_products_full<G>(run, buf);
+            run = add_in_turn(run, xb + half * 32 * STX, STX, nseg);
         }
-        // the last, partial group
-        const int rem = len - b0;
-        if (rem > 0) {
-            __syncwarp();
-#pragma unroll
-            for (int j = 0; j < AH; ++j)
-                buf[32 * j + lane] = 32 * j + lane < rem ? dmul(wide(vq[j]), xq[j]) : T(0);
-            __syncwarp();
-            run = add_products<G>(run, buf, rem);
-        }
-        if (lane == 0)
-            Y[row * ldy] = run;
+        if (cur.b0 + G >= cur.len && lane == 0)
+            *cur.y = run;
+        __syncwarp();  // this half is read before it is filled again
+        if (!more)
+            break;
+        half ^= 1;
     }
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
 }
 
-// Y += A X over K columns of X and Y (FP64, K = 2 .. 32), sliced rows.  Lane
-// (g, h) = (lane / K, lane % K) keeps the sums of column h for rows g, g + G,
-// ... of the slice (G = 32 / K): the group of K lanes reads one row of X, K
-// contiguous values, per product.  Each step loads the slice's 32 words and
-// values as the SpMV does (lane r: row r); lane r keeps row r's running
-// column, and the groups take column and value by shuffles.  Every (row,
-// column) sum adds its products in the row's column order from Y's value:
-// column j of Y is bitwise the SpMV of column j of X.
-template <int K>
-__global__ void __launch_bounds__(32 * kWarpsPerCta) k_spmm_slices(dc_args P, int S)
+// Y += A X over k > 1 columns (FP64), kMmCols = 4 of them a warp (blockIdx.x
+// names the four): one 32-byte sector of a row of X.  Lane (g, h) = (lane / 4,
+// lane % 4) keeps the sums of column h for rows g, g + 8, g + 16, g + 24 of
+// the slice and reads those rows' words and values itself (four lanes the same
+// address: a broadcast), so nothing is exchanged between lanes.  The next
+// kMmAhead steps' words and values are in flight while the gathers of the
+// current ones return.  Every (row, column) sum adds its products in the
+// row's column order from Y's value: column j of Y is bitwise the SpMV of
+// column j of X.
+// Bound by the latency of the gathers (eight a lane in flight); one launch
+// whatever k is.  R-MAT scale 18, 7 columns: passes of 4, 2 and 1 columns, each
+// with up to four gathers a lane in flight and column and value by shuffles,
+// took 415 us of kernel time, this 77 us (with the chains: 1,305 -> 113 us).
+template <int S>
+__global__ void __launch_bounds__(32 * kWarpsPerCta, 2) k_spmm_slices(dc_args P)
 {
-    constexpr int G = 32 / K;
-    constexpr int CH = K < 8 ? K : 8;  // rows whose gathers are in flight together
+    constexpr int R = kMmCols, U = kMmAhead;  // rows a lane (32 rows x 4 columns over 32 lanes); steps a round
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int g = lane / K, h = lane % K;
-    const int gw = blockIdx.x * kWarpsPerCta + warp;
-    if (gw >= P.warps)
+    const int g = lane / kMmCols, h = blockIdx.x * kMmCols + lane % kMmCols;
+    const int gw = blockIdx.y * kWarpsPerCta + warp;
+    if (gw >= P.warps || h >= P.cols)
         return;
     const double* X = static_cast<const double*>(P.x) + h;
     double* Y = static_cast<double*>(P.y) + h;
@@ -383,103 +505,128 @@ __global__ void __launch_bounds__(32 * kWarpsPerCta) k_spmm_slices(dc_args P, in
 #pragma unroll 1
     for (int64_t si = P.wbeg[gw]; si < s1; ++si) {
         const dc_slice sl = P.slices[si];
-        const uint32_t* W = P.A.words + sl.base;
-        const double* Vv = static_cast<const double*>(P.A.vals) + sl.base;
-        const uint32_t rec = lane < (int)sl.lanes ? P.A.lane[sl.meta + lane] : 0u;
-        const int len = lane < (int)sl.lanes ? (int)(rec & kLenMask) + 1 : 0;
-        const uint32_t off = rec >> kLenBits;  // lane r: row r's offset from the slice's first row
-        const int64_t row0 = (int64_t)sl.brow * S;
-        double acc[K];
+        const uint32_t* W = P.A.words + sl.base + g;
+        const double* Vv = static_cast<const double*>(P.A.vals) + sl.base + g;
+        int len[R];
+        double* y[R];
+        double acc[R];
+        uint32_t col[R], w[U][R];
+        double v[U][R];
 #pragma unroll
-        for (int i = 0; i < K; ++i) {
-            const int r = g + G * i;
-            const uint32_t oi = __shfl_sync(0xffffffffu, off, r);
-            acc[i] = r < (int)sl.lanes ? Y[(row0 + oi) * P.ldy] : 0.0;
+        for (int i = 0; i < R; ++i) {
+            const int r = g + 8 * i;
+            const uint32_t rec = r < (int)sl.lanes ? P.A.lane[sl.meta + r] : 0u;
+            len[i] = r < (int)sl.lanes ? (int)(rec & kLenMask) + 1 : 0;
+            y[i] = Y + ((int64_t)sl.brow * S + (int64_t)(rec >> kLenBits)) * P.ldy;
+            col[i] = 0;
         }
-        uint32_t col = 0;  // lane r: row r's column
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+            for (int i = 0; i < R; ++i) {
+                w[u][i] = u < len[i] ? __ldg(W + 32 * u + 8 * i) : 0u;
+                v[u][i] = u < len[i] ? __ldg(Vv + 32 * u + 8 * i) : 0.0;
+            }
+#pragma unroll
+        for (int i = 0; i < R; ++i)
+            acc[i] = len[i] ? *y[i] : 0.0;
 #pragma unroll 1
-        for (int k = 0; k < (int)sl.steps; ++k) {
-            const bool on = k < len;
-            const int64_t slot = (int64_t)k * 32 + lane;
-            col += on ? ld_stream(W + slot) : 0u;
-            const double v = on ? ld_stream(Vv + slot) : 0.0;
-            const uint32_t act = __ballot_sync(0xffffffffu, on);
+        for (int k0 = 0; k0 < (int)sl.steps; k0 += U) {
+            double x[U][R];
 #pragma unroll
-            for (int i0 = 0; i0 < K; i0 += CH) {
-                double x[CH], vv[CH];
+            for (int u = 0; u < U; ++u)
 #pragma unroll
-                for (int i = 0; i < CH; ++i) {
-                    const int r = g + G * (i0 + i);
-                    const uint32_t c = __shfl_sync(0xffffffffu, col, r);
-                    vv[i] = __shfl_sync(0xffffffffu, v, r);
-                    x[i] = (act >> r) & 1u ? __ldg(X + (int64_t)c * P.ldx) : 0.0;
+                for (int i = 0; i < R; ++i) {
+                    col[i] += w[u][i];
+                    x[u][i] = k0 + u < len[i] ? __ldg(X + (int64_t)col[i] * P.ldx) : 0.0;
+                    w[u][i] = k0 + U + u < len[i] ? __ldg(W + 32 * (k0 + U + u) + 8 * i) : 0u;
                 }
 #pragma unroll
-                for (int i = 0; i < CH; ++i)
-                    if ((act >> (g + G * (i0 + i))) & 1u)
-                        acc[i0 + i] = dadd(acc[i0 + i], dmul(vv[i], x[i]));
-            }
+            for (int u = 0; u < U; ++u)
+#pragma unroll
+                for (int i = 0; i < R; ++i) {
+                    if (k0 + u < len[i])
+                        acc[i] = dadd(acc[i], dmul(v[u][i], x[u][i]));
+                    v[u][i] = k0 + U + u < len[i] ? __ldg(Vv + 32 * (k0 + U + u) + 8 * i) : 0.0;
+                }
         }
 #pragma unroll
-        for (int i = 0; i < K; ++i) {
-            const int r = g + G * i;
-            const uint32_t oi = __shfl_sync(0xffffffffu, off, r);
-            if (r < (int)sl.lanes)
-                Y[(row0 + oi) * P.ldy] = acc[i];
-        }
+        for (int i = 0; i < R; ++i)
+            if (len[i])
+                *y[i] = acc[i];
     }
 }
 
-// Y += A X over K columns, the chains: one row per warp, lane h (of the first
-// K; the others repeat them and store nothing) keeps column h's sum and adds
-// the row's products one after another, 32 elements' words and values loaded
-// at a time (the next 32 in flight meanwhile) and taken by shuffles.
-template <int K>
-__global__ void __launch_bounds__(32 * kChainWarps, kChainCtasPerSm) k_spmm_chains(dc_args P, int S)
+// Y += A X over k > 1 columns, the chains: one row and kMmCols = 4 columns a
+// warp, 128 elements at a time.  Lane (g, h) holds elements 16 g .. 16 g + 15
+// for column h: its segment of column h's chain in chain::sum_group (four
+// chains of eight segments at once).  The words and values are loaded by the
+// quad (lane (g, h) elements 16 g + 4 j + h) and handed round by shuffles, so
+// that the 16 gathers of X a lane has in flight are one sector each for the
+// quad.  Where sum_group gives up, the segments are added one after another.
+// R-MAT scale 18, 7 columns: three passes with eight gathers in flight a warp
+// step took 1,236 us of kernel time, this 92 us.
+template <int S>
+__global__ void __launch_bounds__(32 * kChainWarps, kChainCtasPerSm) k_spmm_chains(dc_args P)
 {
+    constexpr int L = 16, G = 8 * L, Q = L / kMmCols;
+    constexpr unsigned full = 0xffffffffu;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int h = lane % K;
-    const int gw = blockIdx.x * kChainWarps + warp;
+    const int g = lane / kMmCols, q = lane % kMmCols, h = blockIdx.x * kMmCols + q;
+    const int gw = blockIdx.y * kChainWarps + warp;
     if (gw >= P.warps)
         return;
-    const double* X = static_cast<const double*>(P.x) + h;
-    double* Y = static_cast<double*>(P.y) + h;
+    const bool live = h < P.cols;  // the last columns' warps may hold fewer than four
+    const double* X = static_cast<const double*>(P.x) + (live ? h : 0);
+    double* Y = static_cast<double*>(P.y) + (live ? h : 0);
     const int64_t s1 = P.wbeg[gw + 1];
 #pragma unroll 1
     for (int64_t si = P.wbeg[gw]; si < s1; ++si) {
         const dc_slice sl = P.slices[si];
         const uint32_t* W = P.A.words + sl.base;
         const double* Vv = static_cast<const double*>(P.A.vals) + sl.base;
-        const int64_t row = (int64_t)sl.brow * S + sl.meta;
-        const int len = (int)sl.steps;
-        double acc = Y[row * P.ldy];
-        uint32_t c = lane < len ? ld_stream(W + lane) : 0u;
-        double v = lane < len ? ld_stream(Vv + lane) : 0.0;
-#pragma unroll 1
-        for (int e0 = 0; e0 < len; e0 += 32) {
-            const int n = min(32, len - e0);
-            const int en = e0 + 32 + lane;
-            const uint32_t cn = en < len ? ld_stream(W + en) : 0u;
-            const double vn = en < len ? ld_stream(Vv + en) : 0.0;
+        const int len = (int)sl.steps, e0 = L * g + q;
+        double* y = Y + ((int64_t)sl.brow * S + sl.meta) * P.ldy;
+        uint32_t w[Q];
+        double v[Q], x[L], run = *y;
 #pragma unroll
-            for (int j0 = 0; j0 < 32; j0 += 8) {
-                double x[8], vv[8];
+        for (int j = 0; j < Q; ++j)
+            w[j] = ld_stream(W + min(e0 + kMmCols * j, len - 1));
 #pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    const uint32_t cj = __shfl_sync(0xffffffffu, c, j0 + j);
-                    vv[j] = __shfl_sync(0xffffffffu, v, j0 + j);
-                    x[j] = j0 + j < n ? __ldg(X + (int64_t)cj * P.ldx) : 0.0;
-                }
+        for (int i = 0; i < L; ++i)
+            x[i] = __ldg(X + (int64_t)__shfl_sync(full, w[i / kMmCols], kMmCols * g + i % kMmCols) * P.ldx);
 #pragma unroll
-                for (int j = 0; j < 8; ++j)
-                    if (j0 + j < n)
-                        acc = dadd(acc, dmul(vv[j], x[j]));
-            }
-            c = cn;
-            v = vn;
+        for (int j = 0; j < Q; ++j) {
+            v[j] = ld_stream(Vv + min(e0 + kMmCols * j, len - 1));
+            w[j] = ld_stream(W + min(e0 + G + kMmCols * j, len - 1));
         }
-        if (lane < K)
-            Y[row * P.ldy] = acc;
+#pragma unroll 1
+        for (int b0 = 0; b0 < len; b0 += G) {
+            double p[L];
+#pragma unroll
+            for (int i = 0; i < L; ++i) {
+                const double vi = __shfl_sync(full, v[i / kMmCols], kMmCols * g + i % kMmCols);
+                p[i] = b0 + L * g + i < len ? dmul(vi, x[i]) : -0.0;
+                x[i] = __ldg(X + (int64_t)__shfl_sync(full, w[i / kMmCols], kMmCols * g + i % kMmCols) * P.ldx);
+            }
+#pragma unroll
+            for (int j = 0; j < Q; ++j) {
+                v[j] = ld_stream(Vv + min(b0 + G + e0 + kMmCols * j, len - 1));
+                w[j] = ld_stream(W + min(b0 + 2 * G + e0 + kMmCols * j, len - 1));
+            }
+            if (!chain::sum_group<kMmCols, L>(run, p, lane)) {
+                const int nseg = min(8, (len - b0 + L - 1) / L);
+#pragma unroll 1
+                for (int s = 0; s < nseg; ++s) {
+#pragma unroll
+                    for (int i = 0; i < L; ++i)
+                        run = g == s ? dadd(run, p[i]) : run;
+                    run = __shfl_sync(full, run, kMmCols * s + q);
+                }
+            }
+        }
+        if (g == 0 && live)
+            *y = run;
     }
 }
 
@@ -638,7 +785,7 @@ int stream_grid_warps(int64_t items, bool chains, bool beside_chains, bool besid
     int dev = 0, nsm = 0;
     ABHSF_CUDA(cudaGetDevice(&dev));
     ABHSF_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    const int ctas = beside_ring ? 1 : kCtasPerSm - (beside_chains ? 1 : 0);
+    const int ctas = beside_ring ? 1 : beside_chains ? kSliceGridPerSm : kCtasPerSm;
     const int64_t full = chains ? (int64_t)nsm * kChainGridPerSm * kChainWarps : (int64_t)nsm * ctas * kWarpsPerCta;
     return (int)std::max<int64_t>(1, std::min<int64_t>(full, items));
 }
@@ -660,10 +807,14 @@ void make_side(cudaStream_t& side, cudaEvent_t& fork, cudaEvent_t& join)
 }
 
 // Time a slice takes, for the deal: a sliced one walks its longest row, a
-// chain adds its products one after another.
+// chain takes about 2,400 cycles a group while its sum is near zero (where
+// groups are added in turn more often) and 1,700 later, and its first loads.
 inline uint64_t slice_weight(const abhsf_matrix::dc_slice_host& p)
 {
-    return p.chain ? 8ull * p.steps + 64u : 32ull * p.steps + 64u;
+    if (!p.chain)
+        return 32ull * p.steps + 64u;
+    const uint64_t groups = (p.steps + kChainGroup - 1) / kChainGroup;
+    return 1700u * groups + 700u * std::min<uint64_t>(groups, 8) + 500u;
 }
 
 }  // namespace
@@ -951,12 +1102,12 @@ namespace {
 // it L1) takes no CTA that needs some until it drains, so the chains would
 // wait for the sliced rows instead of running beside them: every kernel here
 // asks for the same split of L1 and shared memory.
-constexpr int kCarveoutPct = 25;
+constexpr int kCarveoutPct = 40;  // a chain CTA takes 73 KB
 
 // Sets the split for kernel Kern once per device (the attribute belongs to
 // the device's context).
 template <auto Kern>
-void same_carveout()
+void same_carveout(int smem = 0)
 {
     static std::atomic<uint64_t> done{0};
     int dev = 0;
@@ -965,6 +1116,8 @@ void same_carveout()
     if (done.load(std::memory_order_relaxed) & bit)
         return;
     ABHSF_CUDA(cudaFuncSetAttribute(Kern, cudaFuncAttributePreferredSharedMemoryCarveout, kCarveoutPct));
+    if (smem > 48 * 1024)
+        ABHSF_CUDA(cudaFuncSetAttribute(Kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     done.fetch_or(bit, std::memory_order_relaxed);
 }
 
@@ -972,9 +1125,10 @@ template <int S, int VT, bool B>
 void launch_kind(bool chains, const dc_args& P, cudaStream_t st)
 {
     if (chains) {
-        same_carveout<k_spmv_chains<S, VT, B>>();
+        constexpr int smem = kChainWarps * chain_smem_warp<typename vt_of<VT>::T, typename vt_of<VT>::V>();
+        same_carveout<k_spmv_chains<S, VT, B>>(smem);
         const unsigned grid = (unsigned)((P.warps + kChainWarps - 1) / kChainWarps);
-        k_spmv_chains<S, VT, B><<<grid, 32 * kChainWarps, 0, st>>>(P);
+        k_spmv_chains<S, VT, B><<<grid, 32 * kChainWarps, smem, st>>>(P);
     } else {
         same_carveout<k_spmv_slices<S, VT, B>>();
         const unsigned grid = (unsigned)((P.warps + kWarpsPerCta - 1) / kWarpsPerCta);
@@ -1011,7 +1165,7 @@ void launch(int s, int vt, bool batch, bool chains, const dc_args& P, cudaStream
 dc_mat mat_of(const abhsf_matrix& a) { return dc_mat{a.dc_words.get(), a.dc_vals.get(), a.dc_lane.get(), a.m}; }
 
 dc_args args_of(const abhsf_matrix& a, const uint8_t* sched, const int64_t* wbeg, int warps, const void* x,
-                int64_t ldx, void* y, int64_t ldy)
+                int64_t ldx, void* y, int64_t ldy, int cols)
 {
     dc_args P{};
     P.slices = reinterpret_cast<const dc_slice*>(sched);
@@ -1022,6 +1176,7 @@ dc_args args_of(const abhsf_matrix& a, const uint8_t* sched, const int64_t* wbeg
     P.y = y;
     P.ldx = ldx;
     P.ldy = ldy;
+    P.cols = cols;
     return P;
 }
 
@@ -1036,48 +1191,56 @@ dc_args batch_args(const abhsf_batch& b, const uint8_t* sched, const int64_t* wb
     P.xs = reinterpret_cast<const void* const*>(xs);
     P.ys = reinterpret_cast<void* const*>(ys);
     P.ldx = P.ldy = 1;
+    P.cols = 1;
     return P;
 }
 
-template <int K>
-void launch_mm_k(bool chains, int s, const dc_args& P, cudaStream_t st)
+// Column groups first in the grid: the groups of one slice run side by side
+// and share its words and values in L2.
+template <int S>
+void launch_mm(bool chains, const dc_args& P, cudaStream_t st)
 {
-    same_carveout<k_spmm_chains<K>>();
-    same_carveout<k_spmm_slices<K>>();
+    same_carveout<k_spmm_chains<S>>();
+    same_carveout<k_spmm_slices<S>>();
+    const unsigned groups = (unsigned)((P.cols + kMmCols - 1) / kMmCols);
+    const int per = chains ? kChainWarps : kWarpsPerCta;
+    const dim3 grid(groups, (unsigned)((P.warps + per - 1) / per));
     if (chains)
-        k_spmm_chains<K><<<(unsigned)((P.warps + kChainWarps - 1) / kChainWarps), 32 * kChainWarps, 0, st>>>(P, s);
+        k_spmm_chains<S><<<grid, 32 * kChainWarps, 0, st>>>(P);
     else
-        k_spmm_slices<K><<<(unsigned)((P.warps + kWarpsPerCta - 1) / kWarpsPerCta), 32 * kWarpsPerCta, 0, st>>>(P, s);
+        k_spmm_slices<S><<<grid, 32 * kWarpsPerCta, 0, st>>>(P);
     ABHSF_CUDA(cudaGetLastError());
 }
 
-// One pass over `cols` columns: the SpMV kernels for one, the K-column ones
-// (FP64) otherwise.
-void launch_cols(int cols, int s, int vt, bool chains, const dc_args& P, cudaStream_t st)
+// P.cols columns: the SpMV kernels for one, the SpMM ones (FP64) for more and
+// for one that is a column of a wider X or Y.
+void launch_cols(int s, int vt, bool chains, const dc_args& P, cudaStream_t st)
 {
     if (P.warps == 0)
         return;
-    switch (cols) {
-    case 1: launch(s, vt, false, chains, P, st); break;
-    case 2: launch_mm_k<2>(chains, s, P, st); break;
-    case 4: launch_mm_k<4>(chains, s, P, st); break;
-    case 8: launch_mm_k<8>(chains, s, P, st); break;
-    case 16: launch_mm_k<16>(chains, s, P, st); break;
-    case 32: launch_mm_k<32>(chains, s, P, st); break;
-    default: fail(ABHSF_ERROR_UNSUPPORTED, "slices: a pass of 1, 2, 4, 8, 16 or 32 columns");
+    if (P.cols == 1 && P.ldx == 1 && P.ldy == 1) {
+        launch(s, vt, false, chains, P, st);
+        return;
+    }
+    switch (s) {
+    case 16: launch_mm<16>(chains, P, st); break;
+    case 32: launch_mm<32>(chains, P, st); break;
+    case 64: launch_mm<64>(chains, P, st); break;
+    case 128: launch_mm<128>(chains, P, st); break;
+    default: launch_mm<256>(chains, P, st); break;
     }
 }
 
 // Chains on the side stream, after everything queued on st so far.
 void fork_chains(cudaStream_t st, cudaStream_t side, cudaEvent_t fork, cudaEvent_t join, int s, int vt, bool batch,
-                 const dc_args& P, int cols = 1)
+                 const dc_args& P)
 {
     ABHSF_CUDA(cudaEventRecord(fork, st));
     ABHSF_CUDA(cudaStreamWaitEvent(side, fork, 0));
     if (batch)
         launch(s, vt, batch, true, P, side);
     else
-        launch_cols(cols, s, vt, true, P, side);
+        launch_cols(s, vt, true, P, side);
     ABHSF_CUDA(cudaEventRecord(join, side));
 }
 
@@ -1113,9 +1276,9 @@ void slices_begin(const abhsf_matrix& a, const dc_plan& p, const void* x, int64_
     ABHSF_CUDA(cudaEventRecord(a.dc_fork, st));
     ABHSF_CUDA(cudaStreamWaitEvent(a.dc_side, a.dc_fork, 0));
     if (beside)  // first, so that its CTAs take their place before the ring's fill the SMs
-        launch(a.s, a.value_type, false, false, args_of(a, p.sched, p.wbeg, p.warps, x, ldx, y, ldy), a.dc_side);
+        launch(a.s, a.value_type, false, false, args_of(a, p.sched, p.wbeg, p.warps, x, ldx, y, ldy, 1), a.dc_side);
     if (p.cwarps)
-        launch_cols(cols, a.s, a.value_type, true, args_of(a, p.csched, p.cwbeg, p.cwarps, x, ldx, y, ldy),
+        launch_cols(a.s, a.value_type, true, args_of(a, p.csched, p.cwbeg, p.cwarps, x, ldx, y, ldy, cols),
                     a.dc_side);
     ABHSF_CUDA(cudaEventRecord(a.dc_join, a.dc_side));
 }
@@ -1125,7 +1288,7 @@ void slices_end(const abhsf_matrix& a, const dc_plan& p, const void* x, int64_t 
 {
     const bool beside = sliced_beside(a, p, cols);
     if (p.warps && !beside)
-        launch_cols(cols, a.s, a.value_type, false, args_of(a, p.sched, p.wbeg, p.warps, x, ldx, y, ldy), st);
+        launch_cols(a.s, a.value_type, false, args_of(a, p.sched, p.wbeg, p.warps, x, ldx, y, ldy, cols), st);
     if (p.cwarps || beside)
         ABHSF_CUDA(cudaStreamWaitEvent(st, a.dc_join, 0));
 }
