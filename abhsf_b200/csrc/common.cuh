@@ -68,7 +68,12 @@ inline std::atomic<int64_t>& dbuf_allocations()
     return count;
 }
 
-// Owning device allocation (cudaMalloc / cudaFree).
+// Device memory (alloc.cu): usable on any stream at once, given back after the
+// device has been waited for.  pool_dev: what device_free needs with it.
+void* device_alloc(size_t bytes, int& pool_dev);
+void device_free(void* ptr, int pool_dev) noexcept;
+
+// Owning device allocation.
 template <typename T>
 class dbuf {
   public:
@@ -77,12 +82,12 @@ class dbuf {
     ~dbuf() { reset(); }
     dbuf(const dbuf&) = delete;
     dbuf& operator=(const dbuf&) = delete;
-    dbuf(dbuf&& o) noexcept : p_(o.p_), n_(o.n_) { o.p_ = nullptr; o.n_ = 0; }
+    dbuf(dbuf&& o) noexcept : p_(o.p_), n_(o.n_), pool_dev_(o.pool_dev_) { o.p_ = nullptr; o.n_ = 0; }
     dbuf& operator=(dbuf&& o) noexcept
     {
         if (this != &o) {
             reset();
-            p_ = o.p_; n_ = o.n_;
+            p_ = o.p_; n_ = o.n_; pool_dev_ = o.pool_dev_;
             o.p_ = nullptr; o.n_ = 0;
         }
         return *this;
@@ -92,24 +97,24 @@ class dbuf {
         reset();
         if (count == 0)
             count = 1;
-        ABHSF_CUDA(cudaMalloc(reinterpret_cast<void**>(&p_), count * sizeof(T)));
+        p_ = static_cast<T*>(device_alloc(count * sizeof(T), pool_dev_));
         dbuf_allocations().fetch_add(1, std::memory_order_relaxed);
         n_ = count;
     }
     void reset()
     {
         if (p_)
-            cudaFree(p_);
+            device_free(p_, pool_dev_);
         p_ = nullptr;
         n_ = 0;
     }
-    T* release() { T* p = p_; p_ = nullptr; n_ = 0; return p; }
     T* get() const { return p_; }
     size_t size() const { return n_; }
 
   private:
     T* p_ = nullptr;
     size_t n_ = 0;
+    int pool_dev_ = -1;
 };
 
 // Plain view of a built matrix passed to kernels by value.
