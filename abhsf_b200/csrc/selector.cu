@@ -7,7 +7,7 @@
 // and scores restricted choices by their regret, the storage above that
 // minimum in percent (block_statistics/consistency.cpp:140-174).  The MLP
 // predicts the minimum-storage size from one pass of features instead of five
-// histograms; block_size_storage (builder.cu) gives the exhaustive answer it
+// histograms; block_size_storage (block_stats.cu) gives the exhaustive answer it
 // is trained on and scored against.
 //
 // Model layout (ABHSF_MLP_PARAMS floats): W1[F][H] b1[H] W2[H][H] b2[H]

@@ -313,8 +313,9 @@ def block_histograms_all(rows, cols, m: int, n: int, stream=None) -> dict[str, d
         r, s = 2 << (p // 8), 2 << (p % 8)
         h = hist[off:off + r * s + 1]
         nz = np.nonzero(h)[0]
-        out[f"{r}x{s}"] = {int(z): int(h[z]) for z in nz}
-        assert sum(out[f"{r}x{s}"].values()) == blocks[p]
+        count = h[nz]
+        assert int(count.sum()) == blocks[p]
+        out[f"{r}x{s}"] = dict(zip(nz.tolist(), count.tolist()))
         off += r * s + 1
     return out
 
