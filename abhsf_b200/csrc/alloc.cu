@@ -7,8 +7,9 @@
 // of the library's own, one per device.  Larger ones stay with cudaMalloc,
 // which maps a gigabyte in 0.4 ms where a pool that has to grow takes 6.5.
 //
-// The pool keeps at most kPoolKept bytes that nobody uses (CUDA gives back what
-// is above that at the next synchronisation) and all of it is given back when an
+// The pool keeps at most kPoolKept bytes that nobody uses: its release threshold
+// (CUDA gives back what the pool holds above it at the next synchronisation) is
+// moved along with the bytes in use.  All that is unused is given back when an
 // allocation fails.  Allocations and frees go through a stream of the library's;
 // a block is handed out after that stream has been waited for and goes back
 // after the device has been waited for, as cudaFree does, so it may be used on
@@ -21,25 +22,31 @@ namespace abhsf {
 
 namespace {
 
-constexpr size_t kPoolBlock = size_t(32) << 20;
-constexpr uint64_t kPoolKept = uint64_t(256) << 20;
+constexpr size_t kPoolBlock = size_t(1) << 30;
+constexpr uint64_t kPoolKept = uint64_t(2) << 30;
 constexpr int kMaxDevices = 64;
 
 struct device_pool {
     bool tried = false;
     cudaMemPool_t pool = nullptr;
     cudaStream_t st = nullptr;
+    uint64_t used = 0;  // bytes of the blocks in use
 };
 
 std::mutex g_pool_mutex;
 device_pool g_pools[kMaxDevices];  // the pools live as long as the process
 
-// The current device's pool (null where it has none).
-device_pool pool_of(int dev)
+// `more` bytes come into use (or go out of it).
+void use_bytes(device_pool& p, int64_t more)
 {
-    if (dev < 0 || dev >= kMaxDevices)
-        return {};
-    std::lock_guard<std::mutex> lock(g_pool_mutex);
+    p.used += (uint64_t)more;
+    uint64_t threshold = p.used + kPoolKept;
+    cudaMemPoolSetAttribute(p.pool, cudaMemPoolAttrReleaseThreshold, &threshold);
+}
+
+// The current device's pool (null where it has none).  Under g_pool_mutex.
+device_pool& pool_of(int dev)
+{
     device_pool& p = g_pools[dev];
     if (!p.tried) {
         p.tried = true;
@@ -48,15 +55,14 @@ device_pool pool_of(int dev)
         props.allocType = cudaMemAllocationTypePinned;
         props.location.type = cudaMemLocationTypeDevice;
         props.location.id = dev;
-        uint64_t kept = kPoolKept;
         cudaMemPool_t pool = nullptr;
         cudaStream_t st = nullptr;
         if (cudaDeviceGetAttribute(&supported, cudaDevAttrMemoryPoolsSupported, dev) == cudaSuccess && supported &&
             cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) == cudaSuccess &&
-            cudaMemPoolCreate(&pool, &props) == cudaSuccess &&
-            cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &kept) == cudaSuccess) {
+            cudaMemPoolCreate(&pool, &props) == cudaSuccess) {
             p.pool = pool;
             p.st = st;
+            use_bytes(p, 0);
         } else {
             cudaGetLastError();  // no pool: cudaMalloc serves
         }
@@ -66,19 +72,24 @@ device_pool pool_of(int dev)
 
 }  // namespace
 
-void* device_alloc(size_t bytes, int& pool_dev)
+void* device_alloc(size_t bytes, device_block& block)
 {
-    pool_dev = -1;
+    block = {};
     int dev = 0;
     ABHSF_CUDA(cudaGetDevice(&dev));
-    const device_pool p = pool_of(dev);
     void* ptr = nullptr;
+    std::lock_guard<std::mutex> lock(g_pool_mutex);
+    device_pool none;
+    device_pool& p = dev >= 0 && dev < kMaxDevices ? pool_of(dev) : none;
     if (p.pool && bytes <= kPoolBlock) {
+        use_bytes(p, (int64_t)bytes);
         if (cudaMallocFromPoolAsync(&ptr, bytes, p.pool, p.st) == cudaSuccess &&
             cudaStreamSynchronize(p.st) == cudaSuccess) {
-            pool_dev = dev;
+            block.dev = dev;
+            block.bytes = bytes;
             return ptr;
         }
+        use_bytes(p, -(int64_t)bytes);
         cudaGetLastError();
     }
     cudaError_t e = cudaMalloc(&ptr, bytes);
@@ -91,19 +102,24 @@ void* device_alloc(size_t bytes, int& pool_dev)
     return ptr;
 }
 
-void device_free(void* ptr, int pool_dev) noexcept
+void device_free(void* ptr, const device_block& block) noexcept
 {
-    if (pool_dev < 0) {
+    if (block.dev < 0) {
         cudaFree(ptr);
         return;
     }
-    int dev = pool_dev;
+    int dev = block.dev;
     cudaGetDevice(&dev);
-    if (dev != pool_dev)
-        cudaSetDevice(pool_dev);
+    if (dev != block.dev)
+        cudaSetDevice(block.dev);
     cudaDeviceSynchronize();
-    cudaFreeAsync(ptr, g_pools[pool_dev].st);
-    if (dev != pool_dev)
+    {
+        std::lock_guard<std::mutex> lock(g_pool_mutex);
+        device_pool& p = g_pools[block.dev];
+        cudaFreeAsync(ptr, p.st);
+        use_bytes(p, -(int64_t)block.bytes);
+    }
+    if (dev != block.dev)
         cudaSetDevice(dev);
 }
 

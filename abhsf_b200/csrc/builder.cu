@@ -10,9 +10,12 @@
 // adds whose result does not depend on their order.
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_scan.cuh>
+#include <cub/device/device_select.cuh>
+#include <thrust/iterator/counting_iterator.h>
 
 #include <algorithm>
 #include <map>
+#include <memory>
 #include <mutex>
 #include <vector>
 
@@ -32,65 +35,74 @@ inline unsigned grid_for(int64_t n)
 
 #define GRID_STRIDE(i, n) for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < (n); i += (int64_t)gridDim.x * blockDim.x)
 
-enum : int { kErrRange = 1, kErrDuplicate = 2, kErrCsrTooLong = 4, kErrHistOverflow = 8 };
+enum : int { kErrRange = 1, kErrDuplicate = 2, kErrCsrTooLong = 4, kErrHistOverflow = 8, kUnordered = 16 };
 
 // key = ((I * N + J) << 2 lg) | (lrow << lg) | lcol: tiles in (block row,
-// block column) order, elements of a tile in row-major order.
-__global__ void k_make_keys(const int64_t* __restrict__ rows, const int64_t* __restrict__ cols,
-                            const double* __restrict__ vals, int64_t nnz, int64_t m, int64_t n, int lg,
-                            uint64_t N, uint64_t* __restrict__ keys, double* __restrict__ vout,
+// block column) order, elements of a tile in row-major order; and the
+// element's place in the input.  kUnordered: the input is not in row-major
+// order.
+__global__ void k_make_keys(const int64_t* __restrict__ rows, const int64_t* __restrict__ cols, int64_t nnz, int64_t m,
+                            int64_t n, int lg, uint64_t N, uint64_t* __restrict__ keys, uint32_t* __restrict__ place,
                             int* __restrict__ err)
 {
     const uint64_t lmask = (uint64_t(1) << lg) - 1;
+    int e = 0;
     GRID_STRIDE(i, nnz)
     {
         const int64_t r = rows[i], c = cols[i];
+        if (i > 0) {
+            const int64_t pr = rows[i - 1];
+            if (pr > r || (pr == r && cols[i - 1] > c))
+                e |= kUnordered;
+        }
+        place[i] = (uint32_t)i;
         if (r < 0 || r >= m || c < 0 || c >= n) {
-            atomicOr(err, kErrRange);
+            e |= kErrRange;
             keys[i] = 0;
-            vout[i] = 0.0;
             continue;
         }
         const uint64_t I = uint64_t(r) >> lg, J = uint64_t(c) >> lg;
         keys[i] = ((I * N + J) << (2 * lg)) | ((uint64_t(r) & lmask) << lg) | (uint64_t(c) & lmask);
-        vout[i] = vals ? vals[i] : 1.0;
     }
+    e = __reduce_or_sync(0xffffffffu, e);
+    // (one lane, and only for a bit that is not set yet: every warp may have the same news)
+    if ((threadIdx.x & 31) == 0 && (*(volatile int*)err & e) != e)
+        atomicOr(err, e);
 }
 
-// head[i] = 1 where a new block starts (key >> shift changes); flags
-// duplicate (row, col) pairs when check_dup.
-__global__ void k_heads(const uint64_t* __restrict__ keys, int64_t nnz, int shift, int check_dup,
-                        int64_t* __restrict__ head, int* __restrict__ err)
+// Element i starts a tile (keys sorted); flags duplicate (row, col) pairs.
+struct new_tile {
+    const uint64_t* keys;
+    int shift;
+    int* err;
+    __device__ bool operator()(int64_t i) const
+    {
+        if (i == 0)
+            return true;
+        const uint64_t p = keys[i - 1], k = keys[i];
+        if (p == k)
+            atomicOr(err, kErrDuplicate);
+        return (p >> shift) != (k >> shift);
+    }
+};
+
+// head[i] = 1 where a new block starts (the sorted key changes).
+__global__ void k_heads(const uint64_t* __restrict__ keys, int64_t nnz, int64_t* __restrict__ head)
+{
+    GRID_STRIDE(i, nnz)
+    head[i] = i == 0 || keys[i - 1] != keys[i] ? 1 : 0;
+}
+
+// After an inclusive scan of the head flags, run_of[i] is 1 + the run of i.
+__global__ void k_run_starts(const int64_t* __restrict__ run_of, int64_t nnz, int64_t* __restrict__ start)
 {
     GRID_STRIDE(i, nnz)
     {
-        const uint64_t k = keys[i];
-        int64_t h = 1;
-        if (i > 0) {
-            const uint64_t p = keys[i - 1];
-            if (check_dup && p == k)
-                atomicOr(err, kErrDuplicate);
-            h = ((p >> shift) != (k >> shift)) ? 1 : 0;
-        }
-        head[i] = h;
-    }
-}
-
-// After an inclusive scan of the head flags, tile_of[i] is 1 + the tile of i.
-__global__ void k_tile_starts(const uint64_t* __restrict__ keys, const int64_t* __restrict__ tile_of,
-                              int64_t nnz, int shift, int64_t* __restrict__ tile_start,
-                              uint64_t* __restrict__ tile_key)
-{
-    GRID_STRIDE(i, nnz)
-    {
-        const int64_t t = tile_of[i] - 1;
-        if (i == 0 || tile_of[i - 1] != tile_of[i]) {
-            tile_start[t] = i;
-            if (tile_key)
-                tile_key[t] = keys[i] >> shift;
-        }
+        const int64_t t = run_of[i] - 1;
+        if (i == 0 || run_of[i - 1] != run_of[i])
+            start[t] = i;
         if (i == nnz - 1)
-            tile_start[t + 1] = nnz;
+            start[t + 1] = nnz;
     }
 }
 
@@ -100,8 +112,9 @@ struct scheme_params {
     int is_binary, allow_csr, forced;
 };
 
-__global__ void k_tile_meta(int64_t T, const int64_t* __restrict__ tile_start, const uint64_t* __restrict__ tile_key,
-                            uint64_t N, scheme_params sp, int64_t* __restrict__ tile_row,
+__global__ void k_tile_meta(int64_t T, int64_t nnz, const int64_t* __restrict__ tile_start,
+                            const uint64_t* __restrict__ keys, int shift, uint64_t N, scheme_params sp,
+                            int64_t* __restrict__ tile_row,
                             uint32_t* __restrict__ tile_col, uint32_t* __restrict__ tile_nnz,
                             uint8_t* __restrict__ tile_scheme, int64_t* __restrict__ stored,
                             int64_t* __restrict__ pay, int* __restrict__ err)
@@ -113,8 +126,8 @@ __global__ void k_tile_meta(int64_t T, const int64_t* __restrict__ tile_start, c
             pay[T] = 0;
             continue;
         }
-        const int64_t z = tile_start[t + 1] - tile_start[t];
-        const uint64_t tk = tile_key[t];
+        const int64_t s0 = tile_start[t], z = (t + 1 < T ? tile_start[t + 1] : nnz) - s0;
+        const uint64_t tk = keys[s0] >> shift;
         int sch = sp.forced;
         if (sch < 0)
             sch = abhsf_select_scheme(sp.s, sp.s, (uint64_t)z, sp.bits, sp.is_binary, sp.allow_csr, nullptr);
@@ -156,47 +169,123 @@ __device__ __forceinline__ uint16_t f64_to_bf16_bits(double v)
     return (uint16_t)(u >> 16);
 }
 
-__global__ void k_scatter(const uint64_t* __restrict__ keys, const double* __restrict__ vals,
-                          const int64_t* __restrict__ tile_of, int64_t nnz, int lg,
-                          const int64_t* __restrict__ tile_start, const uint8_t* __restrict__ tile_scheme,
-                          const int64_t* __restrict__ tile_val_off, const int64_t* __restrict__ tile_idx_off,
-                          int value_type, uint8_t* __restrict__ payload, void* __restrict__ values)
+// Every element to its tile's payload and values.  A CTA takes kScatter
+// consecutive sorted elements: the first one's tile by a search (32 probes a
+// step), the others' by counting the tile starts among them.  The value comes
+// from the element's place in the input.  A bitmap word's bits are put together
+// in the warp first: its elements are neighbours.
+constexpr int kScatter = 2048;
+__global__ void __launch_bounds__(kThreads) k_scatter(const uint64_t* __restrict__ keys,
+                                                      const uint32_t* __restrict__ place,
+                                                      const double* __restrict__ vals, int64_t nnz, int64_t T, int lg,
+                                                      const int64_t* __restrict__ tile_start,
+                                                      const uint8_t* __restrict__ tile_scheme,
+                                                      const int64_t* __restrict__ tile_val_off,
+                                                      const int64_t* __restrict__ tile_idx_off, int value_type,
+                                                      uint8_t* __restrict__ payload, void* __restrict__ values)
 {
+    constexpr int PER = kScatter / kThreads;
+    __shared__ uint64_t sk[kScatter + 2];  // the key before the chunk, the chunk's, the key after it
+    __shared__ uint16_t rank[kScatter];    // tile starts up to and with the element
+    __shared__ int wsum[kThreads / 32];
+    __shared__ int64_t first;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, shift = 2 * lg;
     const int64_t s = int64_t(1) << lg;
-    const uint64_t lmask = (uint64_t(1) << (2 * lg)) - 1;
-    GRID_STRIDE(i, nnz)
-    {
-        const int64_t t = tile_of[i] - 1;
-        const int64_t p = i - tile_start[t];
-        const uint64_t local = keys[i] & lmask;
-        const uint32_t lr = (uint32_t)(local >> lg), lc = (uint32_t)(local & (s - 1));
-        const int sch = tile_scheme[t];
-        const int64_t vpos = tile_val_off[t] + (sch == ABHSF_SCHEME_DENSE ? (int64_t)local : p);
-        const double v = vals[i];
-        if (value_type == ABHSF_VALUE_F64)
-            static_cast<double*>(values)[vpos] = v;
-        else if (value_type == ABHSF_VALUE_F32)
-            static_cast<float*>(values)[vpos] = __double2float_rn(v);
-        else
-            static_cast<uint16_t*>(values)[vpos] = f64_to_bf16_bits(v);
-        uint8_t* pay = payload + tile_idx_off[t];
-        if (sch == ABHSF_SCHEME_COO) {
-            reinterpret_cast<uint16_t*>(pay)[p] = (uint16_t)((lr << lg) | lc);
-        } else if (sch == ABHSF_SCHEME_CSR) {
-            pay[2 * s + p] = (uint8_t)lc;
-            // The last element of each row writes row_end for its row and the
-            // empty rows that follow it (rows before the first element stay 0).
-            const int64_t tend = tile_start[t + 1];
-            uint32_t next_lr = (uint32_t)s;
-            if (i + 1 < tend)
-                next_lr = (uint32_t)((keys[i + 1] & lmask) >> lg);
-            if (next_lr != lr) {
-                uint16_t* row_end = reinterpret_cast<uint16_t*>(pay);
-                for (uint32_t r = lr; r < next_lr; ++r)
-                    row_end[r] = (uint16_t)(p + 1);
+    const uint64_t lmask = (uint64_t(1) << shift) - 1;
+    for (int64_t base = blockIdx.x * (int64_t)kScatter; base < nnz; base += (int64_t)gridDim.x * kScatter) {
+        const int n = (int)min((int64_t)kScatter, nnz - base);
+        __syncthreads();
+        for (int e = tid; e < n + 2; e += kThreads) {
+            const int64_t i = base + e - 1;
+            sk[e] = i >= 0 && i < nnz ? keys[i] : ~uint64_t(0);
+        }
+        if (warp == 0) {  // the last tile that starts at or before base
+            int64_t lo = 0, hi = T;  // tile_start[lo] <= base, tile_start[hi] > base (tile_start[T] = nnz)
+            while (hi - lo > 1) {
+                const int64_t step = (hi - lo + 31) / 32, at = lo + step * (lane + 1);
+                const bool le = at < hi && tile_start[at] <= base;
+                const int k = __popc(__ballot_sync(0xffffffffu, le));  // starts ascend: the first k lanes
+                const int64_t nlo = lo + step * k;
+                hi = min(hi, nlo + step);
+                lo = nlo;
             }
-        } else if (sch == ABHSF_SCHEME_BITMAP) {
-            atomicOr(reinterpret_cast<unsigned long long*>(pay) + (local >> 6), 1ull << (local & 63));
+            if (lane == 0)
+                first = lo;
+        }
+        __syncthreads();
+        int starts[PER], sum = 0;  // thread: PER consecutive elements
+#pragma unroll
+        for (int j = 0; j < PER; ++j) {
+            const int e = tid * PER + j;
+            // the first element's tile is `first`, whether it starts there or not
+            sum += e > 0 && e < n && (sk[e] >> shift) != (sk[e + 1] >> shift);
+            starts[j] = sum;
+        }
+        int inc = sum;
+#pragma unroll
+        for (int d = 1; d < 32; d *= 2) {
+            const int v = __shfl_up_sync(0xffffffffu, inc, d);
+            if (lane >= d)
+                inc += v;
+        }
+        if (lane == 31)
+            wsum[warp] = inc;
+        __syncthreads();
+        int before = inc - sum;
+        for (int w = 0; w < warp; ++w)
+            before += wsum[w];
+#pragma unroll
+        for (int j = 0; j < PER; ++j)
+            rank[tid * PER + j] = (uint16_t)(before + starts[j]);
+        __syncthreads();
+        for (int e0 = 0; e0 < n; e0 += kThreads) {
+            const int e = e0 + tid;
+            const bool have = e < n;
+            const int64_t i = base + e;
+            const uint64_t key = sk[min(e, n - 1) + 1], local = key & lmask;
+            const int64_t t = first + rank[min(e, n - 1)];
+            const int64_t ts = tile_start[t], p = i - ts;
+            const int sch = tile_scheme[t];
+            uint8_t* pay = payload + tile_idx_off[t];
+            const uint32_t lr = (uint32_t)(local >> lg), lc = (uint32_t)(local & (s - 1));
+            if (have) {
+                const int64_t vpos = tile_val_off[t] + (sch == ABHSF_SCHEME_DENSE ? (int64_t)local : p);
+                const double v = vals ? vals[place[i]] : 1.0;
+                if (value_type == ABHSF_VALUE_F64)
+                    static_cast<double*>(values)[vpos] = v;
+                else if (value_type == ABHSF_VALUE_F32)
+                    static_cast<float*>(values)[vpos] = __double2float_rn(v);
+                else
+                    static_cast<uint16_t*>(values)[vpos] = f64_to_bf16_bits(v);
+                if (sch == ABHSF_SCHEME_COO) {
+                    reinterpret_cast<uint16_t*>(pay)[p] = (uint16_t)((lr << lg) | lc);
+                } else if (sch == ABHSF_SCHEME_CSR) {
+                    pay[2 * s + p] = (uint8_t)lc;
+                    // The last element of each row writes row_end for its row and the
+                    // empty rows that follow it (rows before the first element stay 0).
+                    const uint64_t nk = sk[e + 2];
+                    const bool last = i + 1 >= nnz || (nk >> shift) != (key >> shift);
+                    const uint32_t next_lr = last ? (uint32_t)s : (uint32_t)((nk & lmask) >> lg);
+                    uint16_t* row_end = reinterpret_cast<uint16_t*>(pay);
+                    for (uint32_t r = lr; r < next_lr; ++r)
+                        row_end[r] = (uint16_t)(p + 1);
+                }
+            }
+            const unsigned bm = __ballot_sync(0xffffffffu, have && sch == ABHSF_SCHEME_BITMAP);
+            if (have && sch == ABHSF_SCHEME_BITMAP) {
+                const unsigned same = __match_any_sync(bm, key >> 6);  // one word of one tile
+                uint64_t bits = uint64_t(1) << (local & 63);
+                const int top = 31 - __clz(same);
+                // the lanes of a word are neighbours: an inclusive OR towards its last lane
+#pragma unroll
+                for (int d = 1; d < 32; d *= 2) {
+                    const uint64_t o = __shfl_up_sync(bm, bits, d);
+                    if (lane >= d && ((same >> (lane - d)) & 1u))
+                        bits |= o;
+                }
+                if (lane == top)
+                    atomicOr(reinterpret_cast<unsigned long long*>(pay) + (local >> 6), (unsigned long long)bits);
+            }
         }
     }
 }
@@ -255,6 +344,29 @@ __global__ void k_len_hist_shared(int64_t B, const int64_t* __restrict__ start, 
             atomicAdd(hist + i, (unsigned long long)sh[i]);
 }
 
+// Histogram of the tiles' nonzeros over many counters: tiles of few in shared
+// memory first.
+__global__ void k_nnz_hist(int64_t T, const uint32_t* __restrict__ nnz, unsigned long long* __restrict__ hist)
+{
+    constexpr int N = 4096;
+    __shared__ unsigned int sh[N];
+    for (int i = threadIdx.x; i < N; i += blockDim.x)
+        sh[i] = 0;
+    __syncthreads();
+    GRID_STRIDE(t, T)
+    {
+        const uint32_t z = nnz[t];
+        if (z < N)
+            atomicAdd(&sh[z], 1u);
+        else
+            atomicAdd(hist + z, 1ull);
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < N; i += blockDim.x)
+        if (sh[i])
+            atomicAdd(hist + i, (unsigned long long)sh[i]);
+}
+
 void check_launch(const char* what) { ABHSF_CUDA(cudaGetLastError()); (void)what; }
 
 template <typename T>
@@ -294,41 +406,22 @@ struct coo_inputs {
     }
 };
 
-// Segments sorted keys into runs of equal (key >> shift); returns the run
-// count and fills start[0..runs] (start[runs] = nnz) and optionally run keys.
-int64_t segment_runs(const uint64_t* keys, int64_t nnz, int shift, bool check_dup, cudaStream_t st,
-                     dbuf<int64_t>& tile_of, dbuf<int64_t>& start, dbuf<uint64_t>* run_key, int* err)
+// Segments sorted keys into runs of equal keys; returns the run count and fills
+// start[0..runs] (start[runs] = nnz).
+int64_t segment_runs(const uint64_t* keys, int64_t nnz, cudaStream_t st, dbuf<int64_t>& start)
 {
-    dbuf<int64_t> head(nnz);
-    tile_of.alloc(nnz);
-    k_heads<<<grid_for(nnz), kThreads, 0, st>>>(keys, nnz, shift, check_dup ? 1 : 0, head.get(), err);
+    dbuf<int64_t> head(nnz), run_of(nnz);
+    k_heads<<<grid_for(nnz), kThreads, 0, st>>>(keys, nnz, head.get());
     check_launch("k_heads");
     size_t tmp_bytes = 0;
-    ABHSF_CUDA(cub::DeviceScan::InclusiveSum(nullptr, tmp_bytes, head.get(), tile_of.get(), nnz, st));
+    ABHSF_CUDA(cub::DeviceScan::InclusiveSum(nullptr, tmp_bytes, head.get(), run_of.get(), nnz, st));
     dbuf<uint8_t> tmp(tmp_bytes);
-    ABHSF_CUDA(cub::DeviceScan::InclusiveSum(tmp.get(), tmp_bytes, head.get(), tile_of.get(), nnz, st));
-    const int64_t runs = read_scalar(tile_of.get() + nnz - 1, st);
+    ABHSF_CUDA(cub::DeviceScan::InclusiveSum(tmp.get(), tmp_bytes, head.get(), run_of.get(), nnz, st));
+    const int64_t runs = read_scalar(run_of.get() + nnz - 1, st);
     start.alloc(runs + 1);
-    if (run_key)
-        run_key->alloc(runs);
-    k_tile_starts<<<grid_for(nnz), kThreads, 0, st>>>(keys, tile_of.get(), nnz, shift, start.get(),
-                                                       run_key ? run_key->get() : nullptr);
-    check_launch("k_tile_starts");
+    k_run_starts<<<grid_for(nnz), kThreads, 0, st>>>(run_of.get(), nnz, start.get());
+    check_launch("k_run_starts");
     return runs;
-}
-
-void sort_pairs(dbuf<uint64_t>& keys, dbuf<double>& vals, int64_t nnz, int end_bit, cudaStream_t st)
-{
-    dbuf<uint64_t> keys_out(nnz);
-    dbuf<double> vals_out(nnz);
-    size_t tmp_bytes = 0;
-    ABHSF_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, keys.get(), keys_out.get(), vals.get(),
-                                               vals_out.get(), nnz, 0, end_bit, st));
-    dbuf<uint8_t> tmp(tmp_bytes);
-    ABHSF_CUDA(cub::DeviceRadixSort::SortPairs(tmp.get(), tmp_bytes, keys.get(), keys_out.get(), vals.get(),
-                                               vals_out.get(), nnz, 0, end_bit, st));
-    keys = std::move(keys_out);
-    vals = std::move(vals_out);
 }
 
 void exclusive_scan(int64_t* in, int64_t* out, int64_t count, cudaStream_t st)
@@ -416,26 +509,40 @@ void mmf_line_from_hist(int64_t m, int64_t n, int64_t nnz, int type, int64_t r, 
 
 namespace {
 
-void finish_stats(abhsf_matrix& a, uint64_t dense_bits, cudaStream_t st)
+// The scheme follows from a tile's nonzeros (or is the forced one), so the
+// histogram of the tiles' nonzeros gives every total.
+void finish_stats(abhsf_matrix& a, const scheme_params& sp, const int64_t* tile_start, cudaStream_t st)
 {
-    std::vector<uint32_t> nz(a.T);
-    std::vector<uint8_t> sch(a.T);
+    const int64_t hl = (int64_t)a.s * a.s + 1;
+    std::vector<uint64_t> h(hl, 0);
     if (a.T) {
-        ABHSF_CUDA(cudaMemcpyAsync(nz.data(), a.tile_nnz.get(), a.T * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-        ABHSF_CUDA(cudaMemcpyAsync(sch.data(), a.tile_scheme.get(), a.T, cudaMemcpyDeviceToHost, st));
+        dbuf<unsigned long long> dh(hl);
+        dbuf<int> err(1);
+        ABHSF_CUDA(cudaMemsetAsync(dh.get(), 0, hl * sizeof(unsigned long long), st));
+        if (hl <= 8192)
+            k_len_hist_shared<<<std::min(grid_for(a.T), 148u * 4), kThreads, hl * sizeof(unsigned int), st>>>(
+                a.T, tile_start, a.nnz, dh.get(), (int)hl, err.get());
+        else
+            k_nnz_hist<<<std::min(grid_for(a.T), 148u * 4), kThreads, 0, st>>>(a.T, a.tile_nnz.get(), dh.get());
+        check_launch("k_len_hist_shared");
+        ABHSF_CUDA(cudaMemcpyAsync(h.data(), dh.get(), hl * sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
+        ABHSF_CUDA(cudaStreamSynchronize(st));
     }
-    ABHSF_CUDA(cudaStreamSynchronize(st));
     abhsf_stats& s = a.stats;
     s = abhsf_stats{};
     s.m = a.m; s.n = a.n; s.nnz = a.nnz;
     s.block_size = a.s; s.value_type = a.value_type;
     s.block_rows = a.M; s.block_cols = a.N; s.tiles = a.T;
     std::map<uint64_t, uint64_t> hist;
-    for (int64_t t = 0; t < a.T; ++t) {
-        s.tiles_per_scheme[sch[t]]++;
-        s.nnz_per_scheme[sch[t]] += nz[t];
-        hist[nz[t]]++;
-    }
+    for (int64_t z = 1; z < hl; ++z)
+        if (h[z]) {
+            const int sch = sp.forced >= 0 ? sp.forced
+                                           : abhsf_select_scheme(sp.s, sp.s, (uint64_t)z, sp.bits, sp.is_binary,
+                                                                 sp.allow_csr, nullptr);
+            s.tiles_per_scheme[sch] += h[z];
+            s.nnz_per_scheme[sch] += z * h[z];
+            hist.emplace_hint(hist.end(), z, h[z]);
+        }
     s.stored_values = a.n_values;
     s.payload_bytes = a.payload_bytes;
     s.format_bytes = (a.M + 1) * 8 + a.T * (4 + 4 + 1) + (a.T + 1) * 16 + a.payload_bytes +
@@ -444,7 +551,7 @@ void finish_stats(abhsf_matrix& a, uint64_t dense_bits, cudaStream_t st)
     // mmf line at this block size whose "double" column has the dense-cost
     // width; binary matrices carry no value bits (mmf.cpp:45-46).
     uint64_t o1[8], o2[8];
-    const uint64_t bits1 = (a.matrix_type == ABHSF_MATRIX_BINARY) ? 0 : dense_bits / 2;
+    const uint64_t bits1 = (a.matrix_type == ABHSF_MATRIX_BINARY) ? 0 : sp.bits / 2;
     mmf_line_from_hist(a.m, a.n, a.nnz, a.matrix_type, a.s, a.s, hist, bits1, o1, o2);
     std::copy(o2, o2 + 8, s.msmf_bits);
 }
@@ -494,26 +601,53 @@ void build_matrix(const int64_t* rows, const int64_t* cols, const double* vals, 
     a.M = M; a.N = N;
     ABHSF_CUDA(cudaGetDevice(&a.device));
 
-    dbuf<int> err(1);
-    ABHSF_CUDA(cudaMemsetAsync(err.get(), 0, sizeof(int), st));
-    dbuf<int64_t> tile_of, tile_start, tile_row, stored, pay;
-    dbuf<uint64_t> keys, tile_key;
-    dbuf<double> svals;
-    int64_t T = 0;
+    if (nnz > int64_t(UINT32_MAX))  // (the inputs and the sort's buffers would not fit a GPU)
+        fail(ABHSF_ERROR_OUT_OF_MEMORY, "more than 2^32 elements");
+
+    // totals the host reads, together: error bits, tiles, stored values, payload bytes
+    dbuf<int64_t> totals(4);
+    ABHSF_CUDA(cudaMemsetAsync(totals.get(), 0, 4 * sizeof(int64_t), st));
+    int* err = reinterpret_cast<int*>(totals.get());
+    int64_t tot[4] = {0, 0, 0, 0};
+    auto read_totals = [&] {
+        ABHSF_CUDA(cudaMemcpyAsync(tot, totals.get(), sizeof(tot), cudaMemcpyDeviceToHost, st));
+        ABHSF_CUDA(cudaStreamSynchronize(st));
+        raise_err((int)tot[0]);
+    };
+    dbuf<int64_t> tile_row, stored, pay;
+    dbuf<uint64_t> keys_in, keys;
+    dbuf<uint32_t> place_in, place;
+    int64_t* tile_start = nullptr;
+    std::unique_ptr<coo_inputs> in;
+    const int shift = 2 * lg;
     if (nnz > 0) {
-        coo_inputs in(rows, cols, binary ? nullptr : vals, nnz, o.inputs_on_device != 0, st);
+        in = std::make_unique<coo_inputs>(rows, cols, binary ? nullptr : vals, nnz, o.inputs_on_device != 0, st);
+        keys_in.alloc(nnz);
+        place_in.alloc(nnz);
         keys.alloc(nnz);
-        svals.alloc(nnz);
-        k_make_keys<<<grid_for(nnz), kThreads, 0, st>>>(in.rows, in.cols, in.vals, nnz, m, n, lg, (uint64_t)N,
-                                                         keys.get(), svals.get(), err.get());
+        place.alloc(nnz);
+        k_make_keys<<<grid_for(nnz), kThreads, 0, st>>>(in->rows, in->cols, nnz, m, n, lg, (uint64_t)N, keys_in.get(),
+                                                         place_in.get(), err);
         check_launch("k_make_keys");
-        raise_err(read_scalar(err.get(), st));
+        read_totals();
+        // Elements given row by row, columns ascending (CSR order, most files):
+        // those of a tile are in its order already, and a stable sort by tile
+        // leaves them so -- 4 passes instead of 6 for a 4M x 4M matrix.
+        const int begin_bit = (tot[0] & kUnordered) ? 0 : std::min(shift, key_bits - 1);
+        size_t b1 = 0, b2 = 0;
+        const thrust::counting_iterator<int64_t> all(0);
+        const new_tile head{keys.get(), shift, err};
+        ABHSF_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, b1, keys_in.get(), keys.get(), place_in.get(), place.get(),
+                                                   nnz, begin_bit, key_bits, st));
+        tile_start = reinterpret_cast<int64_t*>(keys_in.get());  // the unsorted keys' memory, once they are sorted
+        ABHSF_CUDA(cub::DeviceSelect::If(nullptr, b2, all, tile_start, totals.get() + 1, nnz, head, st));
+        dbuf<uint8_t> tmp(std::max(b1, b2));
+        ABHSF_CUDA(cub::DeviceRadixSort::SortPairs(tmp.get(), b1, keys_in.get(), keys.get(), place_in.get(),
+                                                   place.get(), nnz, begin_bit, key_bits, st));
+        ABHSF_CUDA(cub::DeviceSelect::If(tmp.get(), b2, all, tile_start, totals.get() + 1, nnz, head, st));
+        read_totals();
     }
-    if (nnz > 0) {
-        sort_pairs(keys, svals, nnz, key_bits, st);
-        T = segment_runs(keys.get(), nnz, 2 * lg, true, st, tile_of, tile_start, &tile_key, err.get());
-        raise_err(read_scalar(err.get(), st));
-    }
+    const int64_t T = tot[1];
     a.T = T;
     a.brow_ptr.alloc(M + 1);
     a.tile_col.alloc(T);
@@ -525,32 +659,45 @@ void build_matrix(const int64_t* rows, const int64_t* cols, const double* vals, 
     stored.alloc(T + 1);
     pay.alloc(T + 1);
     scheme_params sp{s, dense_bits, binary ? 1 : 0, o.allow_csr ? 1 : 0, o.forced_scheme};
-    k_tile_meta<<<grid_for(T + 1), kThreads, 0, st>>>(T, tile_start.get(), tile_key.get(), (uint64_t)N, sp,
+    k_tile_meta<<<grid_for(T + 1), kThreads, 0, st>>>(T, nnz, tile_start, keys.get(), shift, (uint64_t)N, sp,
                                                        tile_row.get(), a.tile_col.get(), a.tile_nnz.get(),
-                                                       a.tile_scheme.get(), stored.get(), pay.get(), err.get());
+                                                       a.tile_scheme.get(), stored.get(), pay.get(), err);
     check_launch("k_tile_meta");
     exclusive_scan(stored.get(), a.tile_val_off.get(), T + 1, st);
     exclusive_scan(pay.get(), a.tile_idx_off.get(), T + 1, st);
     k_brow_ptr<<<grid_for(M + 1), kThreads, 0, st>>>(M, T, tile_row.get(), a.brow_ptr.get());
     check_launch("k_brow_ptr");
-    raise_err(read_scalar(err.get(), st));
-    a.n_values = read_scalar(a.tile_val_off.get() + T, st);
-    a.payload_bytes = read_scalar(a.tile_idx_off.get() + T, st);
+    ABHSF_CUDA(cudaMemcpyAsync(totals.get() + 2, a.tile_val_off.get() + T, sizeof(int64_t), cudaMemcpyDeviceToDevice,
+                               st));
+    ABHSF_CUDA(cudaMemcpyAsync(totals.get() + 3, a.tile_idx_off.get() + T, sizeof(int64_t), cudaMemcpyDeviceToDevice,
+                               st));
+    read_totals();
+    a.n_values = tot[2];
+    a.payload_bytes = tot[3];
     a.payload.alloc(a.payload_bytes);
     // 16 bytes of padding: pipelined kernels copy 16-byte-aligned supersets of value ranges
-    a.values.alloc(a.n_values * value_size(a.value_type) + 16);
+    const size_t vs = value_size(a.value_type);
+    a.values.alloc(a.n_values * vs + 16);
     ABHSF_CUDA(cudaMemsetAsync(a.payload.get(), 0, a.payload.size(), st));
-    ABHSF_CUDA(cudaMemsetAsync(a.values.get(), 0, a.values.size(), st));
+    if (a.n_values == nnz)  // no dense tile: every value is written
+        ABHSF_CUDA(cudaMemsetAsync(a.values.get() + a.n_values * vs, 0, 16, st));
+    else
+        ABHSF_CUDA(cudaMemsetAsync(a.values.get(), 0, a.values.size(), st));
     if (nnz > 0) {
-        k_scatter<<<grid_for(nnz), kThreads, 0, st>>>(keys.get(), svals.get(), tile_of.get(), nnz, lg,
-                                                       tile_start.get(), a.tile_scheme.get(), a.tile_val_off.get(),
-                                                       a.tile_idx_off.get(), a.value_type, a.payload.get(),
-                                                       a.values.get());
+        const unsigned g = (unsigned)std::min<int64_t>((nnz + kScatter - 1) / kScatter, 148 * 8);
+        k_scatter<<<g, kThreads, 0, st>>>(keys.get(), place.get(), in->vals, nnz, T, lg, tile_start,
+                                          a.tile_scheme.get(), a.tile_val_off.get(), a.tile_idx_off.get(),
+                                          a.value_type, a.payload.get(), a.values.get());
         check_launch("k_scatter");
     }
     a.dev_status.alloc(1);
     ABHSF_CUDA(cudaMemsetAsync(a.dev_status.get(), 0, sizeof(int), st));
-    finish_stats(a, dense_bits, st);
+    finish_stats(a, sp, tile_start, st);
+    in.reset();  // the sort's memory is not needed any more
+    keys_in.reset();
+    keys.reset();
+    place_in.reset();
+    place.reset();
     prepare_tree(a, st);
     prepare_ring(a, st);
 }
@@ -589,8 +736,8 @@ void block_histogram(const int64_t* rows, const int64_t* cols, int64_t nnz, int6
         ABHSF_CUDA(cub::DeviceRadixSort::SortKeys(tmp.get(), tmp_bytes, keys.get(), keys_out.get(), nnz, 0, end_bit,
                                                   st));
     }
-    dbuf<int64_t> run_of, start;
-    const int64_t B = segment_runs(keys_out.get(), nnz, 0, false, st, run_of, start, nullptr, err.get());
+    dbuf<int64_t> start;
+    const int64_t B = segment_runs(keys_out.get(), nnz, st, start);
     dbuf<unsigned long long> dh(hist_len);
     ABHSF_CUDA(cudaMemsetAsync(dh.get(), 0, hist_len * sizeof(unsigned long long), st));
     // few counters: added up in shared memory first (most blocks hold one of a
@@ -707,12 +854,12 @@ void block_histogram_noalloc(const int64_t* rows, const int64_t* cols, int64_t n
     check_launch("k_block_keys");
     raise_err(read_scalar(err, st));
     ABHSF_CUDA(cub::DeviceRadixSort::SortKeys(sort_tmp, sort_bytes, keys, keys_out, nnz, 0, end_bit, st));
-    k_heads<<<grid_for(nnz), kThreads, 0, st>>>(keys_out, nnz, 0, 0, head, err);
+    k_heads<<<grid_for(nnz), kThreads, 0, st>>>(keys_out, nnz, head);
     check_launch("k_heads");
     ABHSF_CUDA(cub::DeviceScan::InclusiveSum(scan_tmp, scan_bytes, head, run_of, nnz, st));
     const int64_t B = read_scalar(run_of + nnz - 1, st);
-    k_tile_starts<<<grid_for(nnz), kThreads, 0, st>>>(keys_out, run_of, nnz, 0, start, nullptr);
-    check_launch("k_tile_starts");
+    k_run_starts<<<grid_for(nnz), kThreads, 0, st>>>(run_of, nnz, start);
+    check_launch("k_run_starts");
     k_len_hist<<<grid_for(B), kThreads, 0, st>>>(B, start, dh, hl, err);
     check_launch("k_len_hist");
     ABHSF_CUDA(cudaMemcpyAsync(hist, dh, hl * sizeof(uint64_t), cudaMemcpyDeviceToHost, st));

@@ -69,9 +69,13 @@ inline std::atomic<int64_t>& dbuf_allocations()
 }
 
 // Device memory (alloc.cu): usable on any stream at once, given back after the
-// device has been waited for.  pool_dev: what device_free needs with it.
-void* device_alloc(size_t bytes, int& pool_dev);
-void device_free(void* ptr, int pool_dev) noexcept;
+// device has been waited for.
+struct device_block {
+    int dev = -1;      // the device whose pool it came from (-1: cudaMalloc)
+    size_t bytes = 0;
+};
+void* device_alloc(size_t bytes, device_block& block);
+void device_free(void* ptr, const device_block& block) noexcept;
 
 // Owning device allocation.
 template <typename T>
@@ -82,12 +86,12 @@ class dbuf {
     ~dbuf() { reset(); }
     dbuf(const dbuf&) = delete;
     dbuf& operator=(const dbuf&) = delete;
-    dbuf(dbuf&& o) noexcept : p_(o.p_), n_(o.n_), pool_dev_(o.pool_dev_) { o.p_ = nullptr; o.n_ = 0; }
+    dbuf(dbuf&& o) noexcept : p_(o.p_), n_(o.n_), block_(o.block_) { o.p_ = nullptr; o.n_ = 0; }
     dbuf& operator=(dbuf&& o) noexcept
     {
         if (this != &o) {
             reset();
-            p_ = o.p_; n_ = o.n_; pool_dev_ = o.pool_dev_;
+            p_ = o.p_; n_ = o.n_; block_ = o.block_;
             o.p_ = nullptr; o.n_ = 0;
         }
         return *this;
@@ -97,14 +101,14 @@ class dbuf {
         reset();
         if (count == 0)
             count = 1;
-        p_ = static_cast<T*>(device_alloc(count * sizeof(T), pool_dev_));
+        p_ = static_cast<T*>(device_alloc(count * sizeof(T), block_));
         dbuf_allocations().fetch_add(1, std::memory_order_relaxed);
         n_ = count;
     }
     void reset()
     {
         if (p_)
-            device_free(p_, pool_dev_);
+            device_free(p_, block_);
         p_ = nullptr;
         n_ = 0;
     }
@@ -114,7 +118,7 @@ class dbuf {
   private:
     T* p_ = nullptr;
     size_t n_ = 0;
-    int pool_dev_ = -1;
+    device_block block_;
 };
 
 // Plain view of a built matrix passed to kernels by value.

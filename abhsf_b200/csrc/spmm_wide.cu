@@ -272,7 +272,9 @@ __global__ void k_tile_bytes_max(int64_t T, const int64_t* __restrict__ idx_off,
     unsigned long long most = 0;
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < T; t += (int64_t)gridDim.x * blockDim.x)
         most = max(most, (unsigned long long)((idx_off[t + 1] - idx_off[t]) + 8 * (val_off[t + 1] - val_off[t])));
-    atomicMax(out, most);
+    const unsigned int w = __reduce_max_sync(0xffffffffu, (unsigned int)most);  // a tile's bytes fit 32 bits
+    if ((threadIdx.x & 31) == 0 && w)
+        atomicMax(out, (unsigned long long)w);
 }
 
 template <int S, int K>

@@ -39,6 +39,7 @@
 #include <vector>
 
 #include <cub/cub.cuh>
+#include <thrust/iterator/counting_iterator.h>
 
 #include "chain_sum.cuh"
 #include "common.cuh"
@@ -670,35 +671,69 @@ __device__ __forceinline__ int64_t brow_of_tile(const int64_t* brow_ptr, int64_t
     return lo;
 }
 
+// A warp's lanes over the z elements of one tile, in any order: f(e, row,
+// column) for element e of the tile, its row and column in the tile.
+template <typename F>
+__device__ __forceinline__ void for_elements(const tiles_view& A, int64_t t, int64_t z, int s, int lg, int lane, F&& f)
+{
+    const uint8_t* pay = A.payload + A.tile_idx_off[t];
+    const uint16_t* w16 = reinterpret_cast<const uint16_t*>(pay);
+    const int sch = A.tile_scheme[t];
+    if (sch == ABHSF_SCHEME_CSR) {
+        for (int64_t e = lane; e < z; e += 32) {
+            int lo = 0, hi = s - 1;  // the first row whose end is beyond e
+            while (lo < hi) {
+                const int mid = (lo + hi) / 2;
+                if (w16[mid] > e)
+                    hi = mid;
+                else
+                    lo = mid + 1;
+            }
+            f(e, lo, (int)pay[2 * s + e]);
+        }
+    } else if (sch == ABHSF_SCHEME_BITMAP) {
+        const uint64_t* bm = reinterpret_cast<const uint64_t*>(pay);
+        const int words = s * s / 64;
+        int64_t done = 0;
+        for (int w0 = 0; w0 < words; w0 += 32) {
+            const int wi = w0 + lane;
+            uint64_t bits = wi < words ? bm[wi] : 0;
+            const int cnt = __popcll(bits);
+            int inc = cnt;
+#pragma unroll
+            for (int d = 1; d < 32; d *= 2) {
+                const int v = __shfl_up_sync(0xffffffffu, inc, d);
+                if (lane >= d)
+                    inc += v;
+            }
+            int64_t e = done + inc - cnt;
+            for (; bits; bits &= bits - 1, ++e) {
+                const int bit = wi * 64 + __ffsll((long long)bits) - 1;
+                f(e, bit >> lg, bit & (s - 1));
+            }
+            done += __shfl_sync(0xffffffffu, inc, 31);
+        }
+    } else {
+        for (int64_t e = lane; e < z; e += 32)
+            f(e, w16[e] >> lg, w16[e] & (s - 1));
+    }
+}
+
 // Elements per row of the slice block rows (sidx[I] >= 0): cnt[sidx * s + lrow].
+// A tile a warp (a thread a tile took 0.7 ms to expand 1M elements in tiles of
+// 256, whose elements it visited one after another).
 __global__ void k_dc_row_counts(int64_t T, tiles_view A, int s, int lg, const int32_t* __restrict__ sidx,
                                 unsigned int* __restrict__ cnt)
 {
-    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < T; t += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t I = brow_of_tile(A.brow_ptr, A.M, t);
-        const int k = sidx[I];
+    const int lane = threadIdx.x & 31;
+    const int64_t warps = (int64_t)gridDim.x * (blockDim.x / 32);
+    for (int64_t t = blockIdx.x * (int64_t)(blockDim.x / 32) + threadIdx.x / 32; t < T; t += warps) {
+        const int k = sidx[brow_of_tile(A.brow_ptr, A.M, t)];
         if (k < 0)
             continue;
         unsigned int* c = cnt + (int64_t)k * s;
-        const uint8_t* pay = A.payload + A.tile_idx_off[t];
         const int64_t z = A.tile_val_off[t + 1] - A.tile_val_off[t];
-        if (A.tile_scheme[t] == ABHSF_SCHEME_CSR) {
-            const uint16_t* re = reinterpret_cast<const uint16_t*>(pay);
-            for (int r = 0; r < s; ++r) {
-                const unsigned int d = re[r] - (r ? re[r - 1] : 0);
-                if (d)
-                    atomicAdd(c + r, d);
-            }
-        } else if (A.tile_scheme[t] == ABHSF_SCHEME_BITMAP) {
-            const uint64_t* bm = reinterpret_cast<const uint64_t*>(pay);
-            for (int i = 0; i < s * s / 64; ++i)
-                for (uint64_t b = bm[i]; b; b &= b - 1)
-                    atomicAdd(c + ((i * 64 + __ffsll((long long)b) - 1) >> lg), 1u);
-        } else {
-            const uint16_t* key = reinterpret_cast<const uint16_t*>(pay);
-            for (int64_t e = 0; e < z; ++e)
-                atomicAdd(c + (key[e] >> lg), 1u);
-        }
+        for_elements(A, t, z, s, lg, lane, [&](int64_t, int lr, int) { atomicAdd(c + lr, 1u); });
     }
 }
 
@@ -709,48 +744,118 @@ __global__ void k_dc_expand(int64_t T, tiles_view A, int s, int lg, const int32_
                             const int64_t* __restrict__ ebase, uint32_t* __restrict__ key, uint32_t* __restrict__ pos,
                             uint32_t* __restrict__ colv, int64_t* __restrict__ vidx)
 {
-    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < T; t += (int64_t)gridDim.x * blockDim.x) {
+    const int lane = threadIdx.x & 31;
+    const int64_t warps = (int64_t)gridDim.x * (blockDim.x / 32);
+    for (int64_t t = blockIdx.x * (int64_t)(blockDim.x / 32) + threadIdx.x / 32; t < T; t += warps) {
         const int64_t I = brow_of_tile(A.brow_ptr, A.M, t);
         const int k = sidx[I];
         if (k < 0)
             continue;
         const int64_t v0 = A.tile_val_off[t], z = A.tile_val_off[t + 1] - v0;
         const int64_t e0 = ebase[k] + (v0 - A.tile_val_off[A.brow_ptr[I]]);
-        const uint8_t* pay = A.payload + A.tile_idx_off[t];
         const uint64_t c0 = (uint64_t)A.tile_col[t] * (uint64_t)s;
-        const uint16_t* w16 = reinterpret_cast<const uint16_t*>(pay);
-        const uint64_t* bm = reinterpret_cast<const uint64_t*>(pay);
-        const int sch = A.tile_scheme[t];
-        int r = 0;          // CSR: the element's row
-        int wi = 0;         // bitmap: the word holding the next set bit
-        uint64_t bits = 0;  // bitmap: that word's bits not yet taken
-        if (sch == ABHSF_SCHEME_BITMAP)
-            bits = bm[0];
-        for (int64_t e = 0; e < z; ++e) {
-            int lr, lc;
-            if (sch == ABHSF_SCHEME_CSR) {
-                while (w16[r] <= e)
-                    ++r;
-                lr = r;
-                lc = pay[2 * s + e];
-            } else if (sch == ABHSF_SCHEME_BITMAP) {
-                while (bits == 0)
-                    bits = bm[++wi];
-                const int bit = wi * 64 + __ffsll((long long)bits) - 1;
-                bits &= bits - 1;
-                lr = bit >> lg;
-                lc = bit & (s - 1);
-            } else {
-                lr = w16[e] >> lg;
-                lc = w16[e] & (s - 1);
-            }
+        for_elements(A, t, z, s, lg, lane, [&](int64_t e, int lr, int lc) {
             const int64_t q = e0 + e;
             key[q] = (uint32_t)((int64_t)k * s + lr);
             pos[q] = (uint32_t)q;
             colv[q] = (uint32_t)(c0 + (uint64_t)lc);
             vidx[q] = v0 + e;
-        }
+        });
     }
+}
+
+// The sliced rows (1 .. kChainMin elements), and the chains, among the ns * s
+// rows.
+struct is_sliced {
+    const unsigned int* cnt;
+    __device__ bool operator()(uint32_t q) const { return cnt[q] >= 1u && cnt[q] <= (unsigned)kChainMin; }
+};
+struct is_chain {
+    const unsigned int* cnt;
+    __device__ bool operator()(uint32_t q) const { return cnt[q] > (unsigned)kChainMin; }
+};
+
+// Index of the segment (seg[0 .. n]: block-row boundaries) block row I lies in.
+__device__ __forceinline__ int segment_of(const int64_t* seg, int n, int64_t I)
+{
+    int lo = 0, hi = n;
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) / 2;
+        if (seg[mid] <= I)
+            lo = mid;
+        else
+            hi = mid;
+    }
+    return lo;
+}
+
+// Sort keys of the sliced rows: segment, then length, longest first.
+__global__ void k_dc_row_keys(int64_t nS, const uint32_t* __restrict__ q, const unsigned int* __restrict__ cnt,
+                              const uint32_t* __restrict__ sel, const int64_t* __restrict__ seg, int nseg, int lg,
+                              uint32_t* __restrict__ key)
+{
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nS; i += (int64_t)gridDim.x * blockDim.x)
+        key[i] = (uint32_t)segment_of(seg, nseg, sel[q[i] >> lg]) << kLenBits | ((unsigned)kChainMin - cnt[q[i]]);
+}
+
+// begin[g]: the first sorted row of segment g (g = 0 .. nseg).
+__global__ void k_dc_segment_begin(int64_t nS, const uint32_t* __restrict__ key, int nseg, int64_t* __restrict__ begin)
+{
+    for (int g = blockIdx.x * blockDim.x + threadIdx.x; g <= nseg; g += gridDim.x * blockDim.x) {
+        int64_t lo = 0, hi = nS;
+        while (lo < hi) {
+            const int64_t mid = (lo + hi) / 2;
+            if ((int64_t)(key[mid] >> kLenBits) < g)
+                lo = mid + 1;
+            else
+                hi = mid;
+        }
+        begin[g] = lo;
+    }
+}
+
+// Steps of every slice: the length of its first row.  first[g]: the first
+// slice of segment g.
+__global__ void k_dc_steps(int64_t nS, const uint32_t* __restrict__ key, const int64_t* __restrict__ begin,
+                           const int64_t* __restrict__ first, uint32_t* __restrict__ steps)
+{
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nS; i += (int64_t)gridDim.x * blockDim.x) {
+        const int g = (int)(key[i] >> kLenBits);
+        const int64_t at = i - begin[g];
+        if (at % 32 == 0)
+            steps[first[g] + at / 32] = (uint32_t)kChainMin - (key[i] & kLenMask);
+    }
+}
+
+// Lane record and first slot of every sliced row.
+__global__ void k_dc_lanes(int64_t nS, const uint32_t* __restrict__ key, const uint32_t* __restrict__ q,
+                           const uint32_t* __restrict__ sel, const int64_t* __restrict__ seg,
+                           const int64_t* __restrict__ begin, const int64_t* __restrict__ first,
+                           const int64_t* __restrict__ base, int lg, uint32_t* __restrict__ lane,
+                           int64_t* __restrict__ slot0)
+{
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nS; i += (int64_t)gridDim.x * blockDim.x) {
+        const int g = (int)(key[i] >> kLenBits);
+        const int64_t at = i - begin[g], j = first[g] + at / 32;
+        const uint32_t len = (uint32_t)kChainMin - (key[i] & kLenMask), r = q[i];
+        const int64_t off = (((int64_t)sel[r >> lg] - seg[g]) << lg) + (r & ((1u << lg) - 1u));
+        lane[32 * j + at % 32] = (uint32_t)off << kLenBits | (len - 1u);
+        slot0[r] = base[j] + at % 32;
+    }
+}
+
+__global__ void k_dc_gather(int64_t n, const uint32_t* __restrict__ q, const unsigned int* __restrict__ cnt,
+                            unsigned int* __restrict__ out)
+{
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+        out[i] = cnt[q[i]];
+}
+
+__global__ void k_dc_chain_slots(int64_t n, const uint32_t* __restrict__ q, const int64_t* __restrict__ slot,
+                                 int64_t* __restrict__ slot0)
+{
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+        slot0[q[i]] = slot[i];
 }
 
 // Words and values at their slots, from the elements sorted row by row (each
@@ -760,14 +865,14 @@ template <typename V>
 __global__ void k_dc_emit(int64_t E, const uint32_t* __restrict__ key, const uint32_t* __restrict__ pos,
                           const uint32_t* __restrict__ colv, const int64_t* __restrict__ vidx,
                           const int64_t* __restrict__ rstart, const int64_t* __restrict__ slot0,
-                          const uint8_t* __restrict__ chain, const V* __restrict__ values,
+                          const unsigned int* __restrict__ cnt, const V* __restrict__ values,
                           uint32_t* __restrict__ words, V* __restrict__ vals)
 {
     for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < E; q += (int64_t)gridDim.x * blockDim.x) {
         const uint32_t kr = key[q];
         const int64_t rank = q - rstart[kr];
         const uint32_t c = colv[pos[q]];
-        const bool ch = chain[kr] != 0;
+        const bool ch = cnt[kr] > (unsigned)kChainMin;
         const int64_t slot = slot0[kr] + (ch ? rank : 32 * rank);
         words[slot] = (ch || rank == 0) ? c : c - colv[pos[q - 1]];
         vals[slot] = values[vidx[pos[q]]];
@@ -933,11 +1038,14 @@ void prepare_stream(abhsf_matrix& a, float avg, cudaStream_t st)
     ABHSF_CUDA(cudaMemcpyAsync(rows.data(), a.tree_rows.get(), nr * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
     ABHSF_CUDA(cudaStreamSynchronize(st));
     // slice block rows in ascending block-row order
-    std::vector<std::pair<uint32_t, int64_t>> sel;  // (block row, tree position)
+    std::vector<int64_t> tree_at(a.M, -1);
     for (int64_t k = 0; k < nr; ++k)
         if (okh[k])
-            sel.push_back({rows[k], k});
-    std::sort(sel.begin(), sel.end());
+            tree_at[rows[k]] = k;
+    std::vector<std::pair<uint32_t, int64_t>> sel;  // (block row, tree position)
+    for (int64_t I = 0; I < a.M; ++I)
+        if (tree_at[I] >= 0)
+            sel.push_back({(uint32_t)I, tree_at[I]});
     const int64_t ns = (int64_t)sel.size();
     int64_t E = 0;
     for (auto& p : sel)
@@ -954,89 +1062,154 @@ void prepare_stream(abhsf_matrix& a, float avg, cudaStream_t st)
     dbuf<unsigned int> cnt(ns * s);
     ABHSF_CUDA(cudaMemcpyAsync(sidx.get(), sidx_h.data(), a.M * sizeof(int32_t), cudaMemcpyHostToDevice, st));
     ABHSF_CUDA(cudaMemsetAsync(cnt.get(), 0, ns * s * sizeof(unsigned int), st));
-    k_dc_row_counts<<<grid_of(a.T), 256, 0, st>>>(a.T, a.view(), s, lg, sidx.get(), cnt.get());
+    k_dc_row_counts<<<grid_of(8 * a.T), 256, 0, st>>>(a.T, a.view(), s, lg, sidx.get(), cnt.get());
     ABHSF_CUDA(cudaGetLastError());
-    std::vector<unsigned int> ch(ns * s);
-    ABHSF_CUDA(cudaMemcpyAsync(ch.data(), cnt.get(), ns * s * sizeof(unsigned int), cudaMemcpyDeviceToHost, st));
-    ABHSF_CUDA(cudaStreamSynchronize(st));
-    // chains: per block row, its rows longer than kChainMin, longest first
-    // (then ascending row).  Sliced rows: per segment (slice_segments), the
-    // other non-empty rows of its block rows by length, longest first, then
-    // ascending row, in groups of 32 -- rows of one length class share a
-    // slice whatever their block row, so that its lanes run out together.
-    std::vector<int64_t> rstart(ns * s + 1, 0), slot0(ns * s, 0);
-    std::vector<uint8_t> chain(ns * s, 0);
-    for (int64_t q = 0; q < ns * s; ++q)
-        rstart[q + 1] = rstart[q] + ch[q];
-    std::vector<uint32_t> lane_rec;
-    auto& SL = a.dc_host;
-    int64_t slots = 0;
-    std::vector<int> order(s);
-    std::vector<int64_t> rest;  // sliced rows of a segment: k s + r
+    // Sliced rows: per segment (slice_segments), the rows of up to kChainMin
+    // elements by length, longest first, then ascending row, in groups of 32 --
+    // rows of one length class share a slice whatever their block row, so that
+    // its lanes run out together.  Longer rows are chains, per block row, longest
+    // first, then ascending row; a segment's chains come before its slices.
+    // The rows are ordered on the device (871k rows of the tiled mixture took 8
+    // ms on the host); the host adds up the slots, one step a slice.
+    const int64_t R = ns * s;
     const std::vector<int64_t> seg = slice_segments(a.M, s);
-    int64_t k = 0;
-    for (size_t g = 0; g + 1 < seg.size(); ++g) {
-        const int64_t b0 = seg[g], b1 = seg[g + 1];
-        rest.clear();
-        for (; k < ns && (int64_t)sel[k].first < b1; ++k) {
-            const unsigned int* c = ch.data() + k * s;
-            int live = 0;
-            for (int r = 0; r < s; ++r)
-                if (c[r])
-                    order[live++] = r;
-            std::stable_sort(order.begin(), order.begin() + live, [&](int p, int q) { return c[p] > c[q]; });
-            int i = 0;
-            for (; i < live && c[order[i]] > (unsigned int)kChainMin; ++i) {
-                abhsf_matrix::dc_slice_host h;
-                h.base = slots;
-                h.meta = order[i];
-                h.brow = sel[k].first;
-                h.steps = c[order[i]];
-                h.lanes = 1;
-                h.chain = true;
-                slot0[k * s + order[i]] = slots;
-                chain[k * s + order[i]] = 1;
-                slots += c[order[i]];
-                SL.push_back(h);
-            }
-            std::sort(order.begin() + i, order.begin() + live);
-            for (; i < live; ++i)
-                rest.push_back(k * s + order[i]);
+    const int nseg = (int)seg.size() - 1;
+    std::vector<uint32_t> selrow_h(ns);
+    for (int64_t k = 0; k < ns; ++k)
+        selrow_h[k] = sel[k].first;
+    dbuf<uint32_t> selrow(ns), sq(R), sq2(R), cq(E / kChainMin + 1), skey(R), skey2(R);
+    dbuf<int64_t> seg_d(nseg + 1), begin_d(nseg + 1), first_d(nseg + 1), found(2), rstart(R + 1), slot0(R);
+    ABHSF_CUDA(cudaMemcpyAsync(selrow.get(), selrow_h.data(), ns * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
+    ABHSF_CUDA(cudaMemcpyAsync(seg_d.get(), seg.data(), (nseg + 1) * sizeof(int64_t), cudaMemcpyHostToDevice, st));
+    std::vector<int64_t> begin(nseg + 1, 0), first(nseg + 1, 0);
+    std::vector<uint32_t> chain_q;
+    std::vector<unsigned int> chain_len;
+    int64_t nS = 0;
+    {
+        const thrust::counting_iterator<uint32_t> all(0);
+        size_t b1 = 0, b2 = 0, b3 = 0, b4 = 0;
+        int kb = kLenBits;
+        while ((int64_t(1) << (kb - kLenBits)) < nseg)
+            ++kb;
+        ABHSF_CUDA(cub::DeviceSelect::If(nullptr, b1, all, sq.get(), found.get(), R, is_sliced{cnt.get()}, st));
+        ABHSF_CUDA(cub::DeviceSelect::If(nullptr, b2, all, cq.get(), found.get() + 1, R, is_chain{cnt.get()}, st));
+        ABHSF_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, b3, skey.get(), skey2.get(), sq.get(), sq2.get(), R, 0, kb,
+                                                   st));
+        ABHSF_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, b4, cnt.get(), rstart.get(), R, st));
+        dbuf<uint8_t> tmp(std::max(std::max(b1, b2), std::max(b3, b4)));
+        ABHSF_CUDA(cub::DeviceSelect::If(tmp.get(), b1, all, sq.get(), found.get(), R, is_sliced{cnt.get()}, st));
+        ABHSF_CUDA(cub::DeviceSelect::If(tmp.get(), b2, all, cq.get(), found.get() + 1, R, is_chain{cnt.get()}, st));
+        ABHSF_CUDA(cub::DeviceScan::ExclusiveSum(tmp.get(), b4, cnt.get(), rstart.get(), R, st));
+        int64_t n2[2] = {0, 0};
+        ABHSF_CUDA(cudaMemcpyAsync(n2, found.get(), sizeof(n2), cudaMemcpyDeviceToHost, st));
+        ABHSF_CUDA(cudaStreamSynchronize(st));
+        nS = n2[0];
+        if (nS) {
+            k_dc_row_keys<<<grid_of(nS), 256, 0, st>>>(nS, sq.get(), cnt.get(), selrow.get(), seg_d.get(), nseg, lg,
+                                                       skey.get());
+            ABHSF_CUDA(cudaGetLastError());
+            ABHSF_CUDA(cub::DeviceRadixSort::SortPairs(tmp.get(), b3, skey.get(), skey2.get(), sq.get(), sq2.get(), nS,
+                                                       0, kb, st));
+            k_dc_segment_begin<<<1, 256, 0, st>>>(nS, skey2.get(), nseg, begin_d.get());
+            ABHSF_CUDA(cudaGetLastError());
+            ABHSF_CUDA(cudaMemcpyAsync(begin.data(), begin_d.get(), (nseg + 1) * sizeof(int64_t),
+                                       cudaMemcpyDeviceToHost, st));
         }
-        std::stable_sort(rest.begin(), rest.end(), [&](int64_t p, int64_t q) { return ch[p] > ch[q]; });
-        for (size_t i = 0; i < rest.size(); i += 32) {
-            const int n32 = (int)std::min<size_t>(32, rest.size() - i);
+        if (n2[1]) {
+            chain_q.resize(n2[1]);
+            ABHSF_CUDA(cudaMemcpyAsync(chain_q.data(), cq.get(), n2[1] * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+            dbuf<unsigned int> cl(n2[1]);
+            k_dc_gather<<<grid_of(n2[1]), 256, 0, st>>>(n2[1], cq.get(), cnt.get(), cl.get());
+            ABHSF_CUDA(cudaGetLastError());
+            chain_len.resize(n2[1]);
+            ABHSF_CUDA(cudaMemcpyAsync(chain_len.data(), cl.get(), n2[1] * sizeof(unsigned int),
+                                       cudaMemcpyDeviceToHost, st));
+            ABHSF_CUDA(cudaStreamSynchronize(st));
+        }
+        ABHSF_CUDA(cudaStreamSynchronize(st));
+    }
+    int64_t nslices = 0;
+    for (int g = 0; g < nseg; ++g) {
+        first[g] = nslices;
+        nslices += (begin[g + 1] - begin[g] + 31) / 32;
+    }
+    first[nseg] = nslices;
+    std::vector<uint32_t> steps(nslices);
+    if (nS) {
+        dbuf<uint32_t> steps_d(nslices);
+        ABHSF_CUDA(cudaMemcpyAsync(first_d.get(), first.data(), (nseg + 1) * sizeof(int64_t), cudaMemcpyHostToDevice,
+                                   st));
+        k_dc_steps<<<grid_of(nS), 256, 0, st>>>(nS, skey2.get(), begin_d.get(), first_d.get(), steps_d.get());
+        ABHSF_CUDA(cudaGetLastError());
+        ABHSF_CUDA(cudaMemcpyAsync(steps.data(), steps_d.get(), nslices * sizeof(uint32_t), cudaMemcpyDeviceToHost,
+                                   st));
+        ABHSF_CUDA(cudaStreamSynchronize(st));
+    }
+    std::vector<size_t> corder(chain_q.size());  // chains by block row, then length (longest first), then row
+    for (size_t i = 0; i < corder.size(); ++i)
+        corder[i] = i;
+    std::stable_sort(corder.begin(), corder.end(), [&](size_t x, size_t y) {
+        const uint32_t kx = chain_q[x] >> lg, ky = chain_q[y] >> lg;
+        return kx != ky ? kx < ky : chain_len[x] > chain_len[y];
+    });
+    auto& SL = a.dc_host;
+    SL.reserve(nslices + chain_q.size());
+    std::vector<int64_t> base(nslices), chain_slot(chain_q.size());
+    int64_t slots = 0;
+    size_t c = 0;
+    for (int g = 0; g < nseg; ++g) {
+        for (; c < corder.size(); ++c) {
+            const uint32_t q = chain_q[corder[c]];
+            if ((int64_t)selrow_h[q >> lg] >= seg[g + 1])
+                break;
             abhsf_matrix::dc_slice_host h;
             h.base = slots;
-            h.meta = (int64_t)lane_rec.size();
-            h.brow = (uint32_t)b0;
-            h.steps = ch[rest[i]];
-            h.lanes = n32;
+            h.meta = q & (uint32_t)(s - 1);
+            h.brow = selrow_h[q >> lg];
+            h.steps = chain_len[corder[c]];
+            h.lanes = 1;
+            h.chain = true;
+            chain_slot[corder[c]] = slots;
+            slots += h.steps;
+            SL.push_back(h);
+        }
+        for (int64_t j = first[g]; j < first[g + 1]; ++j) {
+            abhsf_matrix::dc_slice_host h;
+            h.base = slots;
+            h.meta = 32 * j;
+            h.brow = (uint32_t)seg[g];
+            h.steps = steps[j];
+            h.lanes = (uint32_t)std::min<int64_t>(32, begin[g + 1] - begin[g] - 32 * (j - first[g]));
             h.chain = false;
-            for (int l = 0; l < 32; ++l) {
-                if (l < n32) {
-                    const int64_t q = rest[i + l];
-                    const int64_t off = (int64_t)sel[q / s].first * s + q % s - b0 * s;
-                    lane_rec.push_back((uint32_t)off << kLenBits | (ch[q] - 1u));
-                    slot0[q] = slots + l;
-                } else {
-                    lane_rec.push_back(0u);
-                }
-            }
+            base[j] = slots;
             slots += 32 * (int64_t)h.steps;
             SL.push_back(h);
         }
     }
+    a.dc_lane.alloc(std::max<int64_t>(32 * nslices, 1));
+    if (nS) {
+        dbuf<int64_t> base_d(nslices);
+        ABHSF_CUDA(cudaMemcpyAsync(base_d.get(), base.data(), nslices * sizeof(int64_t), cudaMemcpyHostToDevice, st));
+        ABHSF_CUDA(cudaMemsetAsync(a.dc_lane.get(), 0, 32 * nslices * sizeof(uint32_t), st));
+        k_dc_lanes<<<grid_of(nS), 256, 0, st>>>(nS, skey2.get(), sq2.get(), selrow.get(), seg_d.get(), begin_d.get(),
+                                                first_d.get(), base_d.get(), lg, a.dc_lane.get(), slot0.get());
+        ABHSF_CUDA(cudaGetLastError());
+        ABHSF_CUDA(cudaStreamSynchronize(st));
+    }
+    if (!chain_q.empty()) {
+        dbuf<int64_t> slot_d(chain_q.size());
+        ABHSF_CUDA(cudaMemcpyAsync(slot_d.get(), chain_slot.data(), chain_q.size() * sizeof(int64_t),
+                                   cudaMemcpyHostToDevice, st));
+        k_dc_chain_slots<<<grid_of(chain_q.size()), 256, 0, st>>>((int64_t)chain_q.size(), cq.get(), slot_d.get(),
+                                                                  slot0.get());
+        ABHSF_CUDA(cudaGetLastError());
+        ABHSF_CUDA(cudaStreamSynchronize(st));
+    }
     // the elements row by row: sort by (block row, row), stable in format order
     dbuf<uint32_t> key(E), pos(E), key2(E), pos2(E), colv(E);
-    dbuf<int64_t> vidx(E), ebase_d(ns + 1), rstart_d(ns * s + 1), slot0_d(ns * s);
-    dbuf<uint8_t> chain_d(ns * s);
+    dbuf<int64_t> vidx(E), ebase_d(ns + 1);
     ABHSF_CUDA(cudaMemcpyAsync(ebase_d.get(), ebase.data(), (ns + 1) * sizeof(int64_t), cudaMemcpyHostToDevice, st));
-    ABHSF_CUDA(cudaMemcpyAsync(rstart_d.get(), rstart.data(), (ns * s + 1) * sizeof(int64_t), cudaMemcpyHostToDevice,
-                               st));
-    ABHSF_CUDA(cudaMemcpyAsync(slot0_d.get(), slot0.data(), ns * s * sizeof(int64_t), cudaMemcpyHostToDevice, st));
-    ABHSF_CUDA(cudaMemcpyAsync(chain_d.get(), chain.data(), ns * s, cudaMemcpyHostToDevice, st));
-    k_dc_expand<<<grid_of(a.T), 256, 0, st>>>(a.T, a.view(), s, lg, sidx.get(), ebase_d.get(), key.get(), pos.get(),
+    k_dc_expand<<<grid_of(8 * a.T), 256, 0, st>>>(a.T, a.view(), s, lg, sidx.get(), ebase_d.get(), key.get(), pos.get(),
                                               colv.get(), vidx.get());
     ABHSF_CUDA(cudaGetLastError());
     int bits = 1;
@@ -1054,16 +1227,12 @@ void prepare_stream(abhsf_matrix& a, float avg, cudaStream_t st)
     const size_t vs = value_size(a.value_type);
     a.dc_words.alloc(slots);
     a.dc_vals.alloc(slots * vs);
-    a.dc_lane.alloc(std::max<size_t>(lane_rec.size(), 1));
     ABHSF_CUDA(cudaMemsetAsync(a.dc_words.get(), 0, slots * sizeof(uint32_t), st));
     ABHSF_CUDA(cudaMemsetAsync(a.dc_vals.get(), 0, slots * vs, st));
-    if (!lane_rec.empty())
-        ABHSF_CUDA(cudaMemcpyAsync(a.dc_lane.get(), lane_rec.data(), lane_rec.size() * sizeof(uint32_t),
-                                   cudaMemcpyHostToDevice, st));
     auto emit = [&](auto tag) {
         using V = decltype(tag);
-        k_dc_emit<V><<<grid_of(E), 256, 0, st>>>(E, key2.get(), pos2.get(), colv.get(), vidx.get(), rstart_d.get(),
-                                                  slot0_d.get(), chain_d.get(),
+        k_dc_emit<V><<<grid_of(E), 256, 0, st>>>(E, key2.get(), pos2.get(), colv.get(), vidx.get(), rstart.get(),
+                                                  slot0.get(), cnt.get(),
                                                   reinterpret_cast<const V*>(a.values.get()), a.dc_words.get(),
                                                   reinterpret_cast<V*>(a.dc_vals.get()));
     };
@@ -1080,15 +1249,12 @@ void prepare_stream(abhsf_matrix& a, float avg, cudaStream_t st)
         a.dc_tree_flag[sel[k].second] = 1;
         moved += fh[sel[k].second];
     }
-    int64_t live_lanes = 0;
-    for (const auto& h : SL)
-        live_lanes += h.chain ? 0 : h.lanes;
     a.stats.spmv_bytes = a.stats.format_bytes - moved + E * (int64_t)(sizeof(uint32_t) + vs) +
-                         (int64_t)SL.size() * (int64_t)sizeof(dc_slice) + live_lanes * (int64_t)sizeof(uint32_t);
+                         (int64_t)SL.size() * (int64_t)sizeof(dc_slice) + nS * (int64_t)sizeof(uint32_t);  // a lane record a sliced row
     a.dc_elements = E;
     a.dc_rows = ns;
     a.dc_slots = slots;
-    a.dc_lane_records = (int64_t)lane_rec.size();
+    a.dc_lane_records = 32 * nslices;
     deal_slices({&a}, a.dc_sched, a.dc_wbeg, a.dc_warps, st, 0, INT64_MAX, kDealSliced);
     deal_slices({&a}, a.dc_csched, a.dc_cwbeg, a.dc_cwarps, st, 0, INT64_MAX, kDealChains);
     if (a.dc_cwarps)
