@@ -5,12 +5,20 @@
 //
 // The reference has no solver; its SpMV is the kernel such a solver calls
 // (spmv/bottlenecks/spmv.cpp:58-64).  Both solvers here keep every scalar
-// (alpha, beta, r.r) on the device: a CG iteration is one SpMV and five small
+// (alpha, beta, r.r) on the device: a CG iteration is one SpMV and three vector
 // kernels, and chunks of iterations are captured once into a CUDA graph and
-// replayed, with one host read of the state per chunk.  Dot products are
-// summed in FP64 over a fixed grid (deterministic).  Once the recurrence
-// residual meets the tolerance, the state's `done` flag turns the rest of the
-// chunk's updates into no-ops.
+// replayed.  A dot product is summed in FP64 over a fixed grid (deterministic);
+// the kernel that needs the result adds up the grid's partial sums itself, every
+// CTA the same way, instead of waiting for a kernel of one CTA.  Each kernel is
+// launched while the one before it ends (programmatic dependent launch) and
+// waits for it on the device.  Once the recurrence residual meets the tolerance,
+// the state's `done` flag turns the rest of the chunk into no-ops; where the
+// SpMV heeds the flag too, a chunk is queued before the state after the one
+// before it has been read.
+// Bound by memory for large systems (the vector kernels move eight vectors an
+// iteration: dot 2, residual 3, direction 5, less one the SpMV need not read,
+// where a kernel each for x and r, and for p, moved eleven) and by the launches
+// for small ones.
 #include <cmath>
 #include <vector>
 
@@ -24,16 +32,28 @@ constexpr int kRedBlocks = 592;  // 4 x 148 SMs
 constexpr int kRedThreads = 256;
 constexpr int kChunk = 8;  // CG iterations per captured graph
 
+// rr and done: entry i for iterations whose number in the chunk is i modulo 2.
+// A kernel reads this iteration's entry and writes the next one's.
 struct cg_state {
-    double rr;     // r . r of the current residual
+    double rr[2];  // r . r of the residual the iteration starts from
     double alpha;  // step of this iteration
-    double beta;   // p update of this iteration
     double tol2;   // stop when r . r <= tol2
-    int done;      // tolerance met, or iteration limit reached
+    int done[2];   // tolerance met, or iteration limit reached, before the iteration
     int iters;     // iterations performed
     int max_iters;
-    int active;  // this iteration updates x, r and p (done was not set before it)
+    int active;  // this iteration updates x, r and p (not a breakdown)
 };
+static_assert(kChunk % 2 == 0, "a chunk ends at entry 0 again");
+
+// Waits for the kernel before, then lets the next one be launched (launches with
+// the programmatic-serialization attribute).  What the kernel before wrote is
+// read by plain loads: the read-only path (const __restrict__, __ldg) promises
+// nothing about data written during the kernel's life, which begins before the
+// wait.
+__device__ __forceinline__ void wait_and_next()
+{
+    asm volatile("griddepcontrol.wait;\ngriddepcontrol.launch_dependents;" ::: "memory");
+}
 
 __device__ __forceinline__ double block_sum(double v)
 {
@@ -76,9 +96,12 @@ constexpr int64_t kStride = (int64_t)kRedBlocks * kRedThreads;
 // partial[blockIdx.x] = sum over this block's grid-stride share of a[i] b[i]
 // (with VEC, packs of 16 bytes, then the tail past the last whole pack)
 template <typename T, bool VEC>
-__global__ void __launch_bounds__(kRedThreads) k_dot(int64_t n, const T* __restrict__ a, const T* __restrict__ b,
-                                                     double* __restrict__ partial)
+__global__ void __launch_bounds__(kRedThreads) k_dot(int64_t n, const T* a, const T* b, double* partial,
+                                                     const int* done)
 {
+    wait_and_next();
+    if (done && *done)
+        return;
     constexpr int N = pack<T>::N;
     const int64_t tid = blockIdx.x * (int64_t)kRedThreads + threadIdx.x;
     const int64_t nv = VEC ? n / N : 0;
@@ -96,7 +119,7 @@ __global__ void __launch_bounds__(kRedThreads) k_dot(int64_t n, const T* __restr
         partial[blockIdx.x] = s;
 }
 
-__device__ __forceinline__ double sum_partials(const double* __restrict__ partial)
+__device__ __forceinline__ double sum_partials(const double* partial)
 {
     double s = 0.0;
     for (int i = threadIdx.x; i < kRedBlocks; i += kRedThreads)
@@ -110,13 +133,13 @@ __global__ void __launch_bounds__(kRedThreads) k_cg_init(const double* __restric
 {
     const double rr = sum_partials(partial);
     if (threadIdx.x == 0) {
-        st->rr = rr;
-        st->alpha = st->beta = 0.0;
+        st->rr[0] = rr;
+        st->alpha = 0.0;
         st->tol2 = tol2;
         st->iters = 0;
         st->max_iters = max_iters;
         st->active = 0;
-        st->done = (rr <= tol2 || max_iters <= 0) ? 1 : 0;
+        st->done[0] = (rr <= tol2 || max_iters <= 0) ? 1 : 0;
     }
 }
 
@@ -128,58 +151,56 @@ __global__ void __launch_bounds__(kRedThreads) k_cg_resume(const double* __restr
     const double rr = sum_partials(partial);
     if (threadIdx.x == 0) {
         const double tol2 = factor2 * rr;
-        st->rr = rr;
+        st->rr[0] = rr;
         st->tol2 = tol2;
-        st->done = (rr <= tol2 || st->iters >= st->max_iters) ? 1 : 0;
+        st->done[0] = (rr <= tol2 || st->iters >= st->max_iters) ? 1 : 0;
     }
 }
 
-__global__ void __launch_bounds__(kRedThreads) k_cg_alpha(const double* __restrict__ partial, cg_state* st)
+// alpha = r.r / p.Ap from the partial sums; r -= alpha Ap; partial r . r.
+// ZERO: Ap = 0, ready for the next y += A p (else that SpMV starts from zero).
+template <typename T, bool VEC, bool ZERO>
+__global__ void __launch_bounds__(kRedThreads) k_cg_residual(int64_t n, T* r, T* ap, cg_state* st, int cur,
+                                                             const double* pap_part, double* partial)
 {
-    const double pap = sum_partials(partial);
+    wait_and_next();
+    if (st->done[cur])
+        return;
+    constexpr int N = pack<T>::N;
+    __shared__ double step;
+    const double pap = sum_partials(pap_part);
     if (threadIdx.x == 0) {
-        if (st->done || !(pap > 0.0)) {  // converged, or breakdown (p = 0 or A not positive definite on p)
-            st->alpha = 0.0;
-            st->done = 1;
-            st->active = 0;
-        } else {
-            st->alpha = st->rr / pap;
-            st->active = 1;
+        const bool go = pap > 0.0;  // else breakdown: p = 0 or A not positive definite on p
+        step = go ? st->rr[cur] / pap : 0.0;
+        if (blockIdx.x == 0) {
+            st->alpha = step;
+            st->active = go ? 1 : 0;
         }
     }
-}
-
-// x += alpha p; r -= alpha Ap; Ap = 0 (ready for the next y += A p); partial r . r
-template <typename T, bool VEC>
-__global__ void __launch_bounds__(kRedThreads) k_cg_update_xr(int64_t n, T* __restrict__ x, T* __restrict__ r,
-                                                              T* __restrict__ ap, const T* __restrict__ p,
-                                                              const cg_state* st, double* __restrict__ partial)
-{
-    constexpr int N = pack<T>::N;
-    const T alpha = (T)st->alpha;
+    __syncthreads();
+    const T alpha = (T)step;
     const int64_t tid = blockIdx.x * (int64_t)kRedThreads + threadIdx.x;
     const int64_t nv = VEC ? n / N : 0;
     double s = 0.0;
     for (int64_t i = tid; i < nv; i += kStride) {
-        pack<T> vr = ld_pack(r + i * N), vx = ld_pack(x + i * N);
-        const pack<T> va = ld_pack(ap + i * N), vp = ld_pack(p + i * N);
+        pack<T> vr = ld_pack(r + i * N);
+        const pack<T> va = ld_pack(ap + i * N);
         pack<T> zero;
 #pragma unroll
         for (int k = 0; k < N; ++k) {
             vr.v[k] = vr.v[k] - alpha * va.v[k];
-            vx.v[k] += alpha * vp.v[k];
             zero.v[k] = T(0);
             s += (double)vr.v[k] * (double)vr.v[k];
         }
-        st_pack(x + i * N, vx);
         st_pack(r + i * N, vr);
-        st_pack(ap + i * N, zero);
+        if (ZERO)
+            st_pack(ap + i * N, zero);
     }
     for (int64_t i = nv * N + tid; i < n; i += kStride) {
         const T ri = r[i] - alpha * ap[i];
-        x[i] += alpha * p[i];
         r[i] = ri;
-        ap[i] = T(0);
+        if (ZERO)
+            ap[i] = T(0);
         s += (double)ri * (double)ri;
     }
     s = block_sum(s);
@@ -187,39 +208,63 @@ __global__ void __launch_bounds__(kRedThreads) k_cg_update_xr(int64_t n, T* __re
         partial[blockIdx.x] = s;
 }
 
-__global__ void __launch_bounds__(kRedThreads) k_cg_beta(const double* __restrict__ partial, cg_state* st)
-{
-    const double rr_new = sum_partials(partial);
-    if (threadIdx.x == 0 && !st->done) {
-        st->beta = rr_new / st->rr;
-        st->rr = rr_new;
-        st->iters += 1;
-        if (rr_new <= st->tol2 || st->iters >= st->max_iters)
-            st->done = 1;
-    }
-}
-
-// p = r + beta p, also in the iteration that met the tolerance, so that a
-// recurrence resumed from a replaced residual continues from the right p
+// beta = new r.r / r.r from the partial sums; x += alpha p; p = r + beta p, also
+// in the iteration that met the tolerance, so that a recurrence resumed from a
+// replaced residual continues from the right p; the next iteration's state.
 template <typename T, bool VEC>
-__global__ void k_cg_update_p(int64_t n, T* __restrict__ p, const T* __restrict__ r, const cg_state* st)
+__global__ void __launch_bounds__(kRedThreads) k_cg_direction(int64_t n, T* x, T* p, const T* r, cg_state* st, int cur,
+                                                              const double* rr_part)
 {
-    if (!st->active)
+    wait_and_next();
+    const int nxt = cur ^ 1;
+    if (st->done[cur]) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            st->rr[nxt] = st->rr[cur];
+            st->done[nxt] = 1;
+        }
         return;
+    }
     constexpr int N = pack<T>::N;
-    const T beta = (T)st->beta;
-    const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, stride = (int64_t)gridDim.x * blockDim.x;
+    __shared__ double grow;
+    const bool active = st->active != 0;
+    const T alpha = (T)st->alpha;
+    const double rr_new = sum_partials(rr_part);
+    if (threadIdx.x == 0) {
+        const double rr = st->rr[cur];
+        grow = rr_new / rr;
+        if (blockIdx.x == 0) {
+            int done = 1;
+            if (active) {
+                const int iters = st->iters + 1;
+                st->iters = iters;
+                done = rr_new <= st->tol2 || iters >= st->max_iters ? 1 : 0;
+            }
+            st->rr[nxt] = active ? rr_new : rr;
+            st->done[nxt] = done;
+        }
+    }
+    __syncthreads();
+    const T beta = (T)grow;
+    const int64_t tid = blockIdx.x * (int64_t)kRedThreads + threadIdx.x;
     const int64_t nv = VEC ? n / N : 0;
-    for (int64_t i = tid; i < nv; i += stride) {
-        pack<T> vp = ld_pack(p + i * N);
+    for (int64_t i = tid; i < nv; i += kStride) {
+        pack<T> vx = ld_pack(x + i * N), vp = ld_pack(p + i * N);
         const pack<T> vr = ld_pack(r + i * N);
 #pragma unroll
-        for (int k = 0; k < N; ++k)
+        for (int k = 0; k < N; ++k) {
+            vx.v[k] += alpha * vp.v[k];
             vp.v[k] = vr.v[k] + beta * vp.v[k];
-        st_pack(p + i * N, vp);
+        }
+        st_pack(x + i * N, vx);
+        if (active)
+            st_pack(p + i * N, vp);
     }
-    for (int64_t i = nv * N + tid; i < n; i += stride)
-        p[i] = r[i] + beta * p[i];
+    for (int64_t i = nv * N + tid; i < n; i += kStride) {
+        const T pi = p[i];
+        x[i] += alpha * pi;
+        if (active)
+            p[i] = r[i] + beta * pi;
+    }
 }
 
 template <typename T>
@@ -268,13 +313,26 @@ void residual(const abhsf_matrix& a, const T* b, const T* x, T* r, T* xn, int64_
 
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
-template <typename T>
-void dot(const T* a, const T* b, int64_t n, double* partial, cudaStream_t st)
+// A vector kernel that waits on the device for the kernel before it in st.
+template <typename... P, typename... A>
+void launch_after(void (*kern)(P...), cudaStream_t st, A... args)
 {
-    if (aligned16(a) && aligned16(b))
-        k_dot<T, true><<<kRedBlocks, kRedThreads, 0, st>>>(n, a, b, partial);
-    else
-        k_dot<T, false><<<kRedBlocks, kRedThreads, 0, st>>>(n, a, b, partial);
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(kRedBlocks);
+    cfg.blockDim = dim3(kRedThreads);
+    cfg.stream = st;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    ABHSF_CUDA(cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...));
+}
+
+template <typename T>
+void dot(const T* a, const T* b, int64_t n, double* partial, cudaStream_t st, const int* done = nullptr)
+{
+    launch_after(aligned16(a) && aligned16(b) ? k_dot<T, true> : k_dot<T, false>, st, n, a, b, partial, done);
 }
 
 // p = r, Ap = 0 and the state from r . r: the start of a CG recurrence.
@@ -294,52 +352,91 @@ void cg_start(cg_work<T>& w, int64_t n, cg_state* st_d, double* partial, double 
 template <typename T>
 class cg_graph {
   public:
+    // partial: 2 kRedBlocks
     cg_graph(const abhsf_matrix& a, T* x, cg_work<T>& w, int64_t n, cg_state* st_d, double* partial, cudaStream_t cs)
+        : heeds_(spmv_sets_y(a))
     {
+        ABHSF_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&seen_), 2 * sizeof(cg_state), cudaHostAllocDefault));
         cudaGraph_t graph = nullptr;
-        const bool vec = aligned16(x) && aligned16(w.r.get()) && aligned16(w.ap.get()) && aligned16(w.p.get());
-        ABHSF_CUDA(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
-        for (int it = 0; it < kChunk; ++it) {
-            spmv_t(a, w.p.get(), w.ap.get(), cs);
-            dot<T>(w.p.get(), w.ap.get(), n, partial, cs);
-            k_cg_alpha<<<1, kRedThreads, 0, cs>>>(partial, st_d);
-            if (vec)
-                k_cg_update_xr<T, true>
-                    <<<kRedBlocks, kRedThreads, 0, cs>>>(n, x, w.r.get(), w.ap.get(), w.p.get(), st_d, partial);
-            else
-                k_cg_update_xr<T, false>
-                    <<<kRedBlocks, kRedThreads, 0, cs>>>(n, x, w.r.get(), w.ap.get(), w.p.get(), st_d, partial);
-            k_cg_beta<<<1, kRedThreads, 0, cs>>>(partial, st_d);
-            if (vec)
-                k_cg_update_p<T, true><<<elem_grid(n), 256, 0, cs>>>(n, w.p.get(), w.r.get(), st_d);
-            else
-                k_cg_update_p<T, false><<<elem_grid(n), 256, 0, cs>>>(n, w.p.get(), w.r.get(), st_d);
+        try {
+            for (cudaEvent_t& e : ev_)
+                ABHSF_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+            ABHSF_CUDA(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
+            try {
+                record(a, x, w, n, st_d, partial, cs);
+            } catch (...) {
+                if (cudaStreamEndCapture(cs, &graph) == cudaSuccess && graph)
+                    cudaGraphDestroy(graph);
+                throw;
+            }
+            const cudaError_t cap = cudaStreamEndCapture(cs, &graph);
+            if (cap != cudaSuccess || !graph)
+                fail(ABHSF_ERROR_CUDA, std::string("CG graph capture: ") + cudaGetErrorString(cap));
+            const cudaError_t ins = cudaGraphInstantiate(&exec_, graph, 0);
+            cudaGraphDestroy(graph);
+            if (ins != cudaSuccess)
+                fail(ABHSF_ERROR_CUDA, std::string("CG graph instantiation: ") + cudaGetErrorString(ins));
+        } catch (...) {
+            release();
+            throw;
         }
-        const cudaError_t cap = cudaStreamEndCapture(cs, &graph);
-        if (cap != cudaSuccess || !graph)
-            fail(ABHSF_ERROR_CUDA, std::string("CG graph capture: ") + cudaGetErrorString(cap));
-        const cudaError_t ins = cudaGraphInstantiate(&exec_, graph, 0);
-        cudaGraphDestroy(graph);
-        if (ins != cudaSuccess)
-            fail(ABHSF_ERROR_CUDA, std::string("CG graph instantiation: ") + cudaGetErrorString(ins));
     }
-    ~cg_graph() { cudaGraphExecDestroy(exec_); }
+    ~cg_graph() { release(); }
     cg_graph(const cg_graph&) = delete;
     cg_graph& operator=(const cg_graph&) = delete;
 
-    // replays chunks until the state says done; returns the iteration count
-    int run(cg_state* st_d, cg_state* st_h, cudaStream_t cs)
+    // Replays chunks until the state says done; returns the iteration count.
+    // Where a chunk after the last is a no-op throughout, it is queued before
+    // the state is read, so that the GPU does not wait for the host.
+    int run(const cg_state* st_d, cudaStream_t cs)
     {
-        for (;;) {
-            ABHSF_CUDA(cudaMemcpyAsync(st_h, st_d, sizeof(cg_state), cudaMemcpyDeviceToHost, cs));
-            ABHSF_CUDA(cudaStreamSynchronize(cs));
-            if (st_h->done)
-                return st_h->iters;
-            ABHSF_CUDA(cudaGraphLaunch(exec_, cs));
+        for (int k = 0;; ++k) {
+            if (heeds_ || k > 0)
+                ABHSF_CUDA(cudaGraphLaunch(exec_, cs));
+            ABHSF_CUDA(cudaMemcpyAsync(seen_ + (k & 1), st_d, sizeof(cg_state), cudaMemcpyDeviceToHost, cs));
+            ABHSF_CUDA(cudaEventRecord(ev_[k & 1], cs));
+            const int look = heeds_ ? k - 1 : k;  // the state to wait for
+            if (look < 0)
+                continue;
+            ABHSF_CUDA(cudaEventSynchronize(ev_[look & 1]));
+            if (seen_[look & 1].done[0])
+                return seen_[look & 1].iters;
         }
     }
 
   private:
+    void record(const abhsf_matrix& a, T* x, cg_work<T>& w, int64_t n, cg_state* st_d, double* partial, cudaStream_t cs)
+    {
+        T *r = w.r.get(), *p = w.p.get(), *ap = w.ap.get();
+        const bool vec = aligned16(x) && aligned16(r) && aligned16(ap) && aligned16(p);
+        double *pap = partial, *rr = partial + kRedBlocks;
+        for (int it = 0; it < kChunk; ++it) {
+            const int cur = it & 1;
+            if (heeds_)
+                spmv_set_y(a, p, ap, st_d->done + cur, cs);
+            else
+                spmv_t(a, p, ap, cs);
+            dot<T>(p, ap, n, pap, cs, st_d->done + cur);
+            launch_after(heeds_ ? (vec ? k_cg_residual<T, true, false> : k_cg_residual<T, false, false>)
+                                : (vec ? k_cg_residual<T, true, true> : k_cg_residual<T, false, true>),
+                         cs, n, r, ap, st_d, cur, pap, rr);
+            launch_after(vec ? k_cg_direction<T, true> : k_cg_direction<T, false>, cs, n, x, p, r, st_d, cur, rr);
+        }
+    }
+    void release()
+    {
+        if (exec_)
+            cudaGraphExecDestroy(exec_);
+        for (cudaEvent_t e : ev_)
+            if (e)
+                cudaEventDestroy(e);
+        if (seen_)
+            cudaFreeHost(seen_);
+    }
+
+    const bool heeds_;  // the SpMV sets y and heeds the done flag
+    cg_state* seen_ = nullptr;  // pinned: the state after the last two chunks
+    cudaEvent_t ev_[2] = {nullptr, nullptr};
     cudaGraphExec_t exec_ = nullptr;
 };
 
@@ -367,7 +464,7 @@ double norm2(const double* a, int64_t n, double* partial, cg_state* st_d, cg_sta
     k_cg_init<<<1, kRedThreads, 0, cs>>>(partial, st_d, 0.0, 0);
     ABHSF_CUDA(cudaMemcpyAsync(st_h, st_d, sizeof(cg_state), cudaMemcpyDeviceToHost, cs));
     ABHSF_CUDA(cudaStreamSynchronize(cs));
-    return st_h->rr;
+    return st_h->rr[0];
 }
 
 void check_square(const abhsf_matrix& a)
@@ -386,14 +483,14 @@ void cg_solve(const abhsf_matrix& a, const double* b, double* x, double rtol, in
     solve_stream ss(user);
     cudaStream_t cs = ss.cs;
     cg_work<double> w(n);
-    dbuf<double> xn(n), partial(kRedBlocks);
+    dbuf<double> xn(n), partial(2 * kRedBlocks);
     dbuf<cg_state> st_d(1);
     cg_state st_h{};
     const double bb = norm2(b, n, partial.get(), st_d.get(), &st_h, cs);
     residual<double>(a, b, x, w.r.get(), xn.get(), n, cs);
     cg_start<double>(w, n, st_d.get(), partial.get(), rtol * rtol * bb, max_iters, cs);
     cg_graph<double> g(a, x, w, n, st_d.get(), partial.get(), cs);
-    const int iters = g.run(st_d.get(), &st_h, cs);
+    const int iters = g.run(st_d.get(), cs);
     residual<double>(a, b, x, w.r.get(), xn.get(), n, cs);
     const double rr = norm2(w.r.get(), n, partial.get(), st_d.get(), &st_h, cs);
     info->iterations = iters;
@@ -412,7 +509,7 @@ void cg_solve_mixed(const abhsf_matrix& a64, const abhsf_matrix& a32, const doub
     const double f2 = update_factor * update_factor;
     solve_stream ss(user);
     cudaStream_t cs = ss.cs;
-    dbuf<double> r64(n), xn(n), partial(kRedBlocks);
+    dbuf<double> r64(n), xn(n), partial(2 * kRedBlocks);
     cg_work<float> w(n);
     dbuf<float> d(n);  // the f32 solution since the last update
     dbuf<cg_state> st_d(1), st64_d(1);
@@ -429,7 +526,7 @@ void cg_solve_mixed(const abhsf_matrix& a64, const abhsf_matrix& a32, const doub
         k_cg_resume<<<1, kRedThreads, 0, cs>>>(partial.get(), st_d.get(), f2);  // partials of r32 . r32
         cg_graph<float> g(a32, d.get(), w, n, st_d.get(), partial.get(), cs);
         for (;;) {
-            iters = g.run(st_d.get(), &st_h, cs);
+            iters = g.run(st_d.get(), cs);
             // reliable update: fold the f32 solution into x, replace r by b - A x in FP64
             k_fold<<<elem_grid(n), 256, 0, cs>>>(n, x, d.get());
             residual<double>(a64, b, x, r64.get(), xn.get(), n, cs);

@@ -142,6 +142,12 @@ void prepare_batch_stream(abhsf_batch& b, cudaStream_t st);
 void batch_stream_begin(const abhsf_batch& b, const double* const* xs, double* const* ys, cudaStream_t st);
 void batch_stream_end(const abhsf_batch& b, const double* const* xs, double* const* ys, cudaStream_t st);
 
+// y = A x (y need not be zeroed) through the slices and chains, or nothing at
+// all where *skip is set (device memory): for matrices whose every row they
+// serve (spmv_sets_y).  T = double for f64 matrices, float for f32 and bf16.
+bool spmv_sets_y(const abhsf_matrix& a);
+void spmv_set_y(const abhsf_matrix& a, const void* x, void* y, const int* skip, cudaStream_t st);
+
 // Conjugate gradients (cg.cu).
 void cg_solve(const abhsf_matrix& a, const double* b, double* x, double rtol, int max_iters, abhsf_cg_info* info,
               cudaStream_t st);

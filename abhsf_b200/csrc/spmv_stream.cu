@@ -137,10 +137,24 @@ struct dc_args {
     void* y;
     int64_t ldx, ldy;        // SpMM: x[i * ldx + column], y[i * ldy + column]
     int cols;                // SpMM: columns
+    int fresh;               // SpMV: y = A x (y starts from zero); 2: launched while the kernel before it ends
+    const int* skip;         // ... nothing is done where *skip is set
     const dc_mat* mats;      // a batch (B = true): matrix i's arrays, x and y
     const void* const* xs;
     void* const* ys;
 };
+
+// A fresh launch (spmv_set_y) waits for the kernel before it, then lets the next
+// one be launched; true where there is nothing to do.  (x, which the kernel
+// before wrote, is read by plain loads: the read-only path promises nothing
+// about data written during the kernel's life.)
+__device__ __forceinline__ bool begin_fresh(const dc_args& P)
+{
+    if (!P.fresh)
+        return false;
+    asm volatile("griddepcontrol.wait;\ngriddepcontrol.launch_dependents;" ::: "memory");
+    return P.skip && *reinterpret_cast<const volatile int*>(P.skip) != 0;
+}
 
 // Eight consecutive values from shared memory (16-byte aligned), in two or
 // four 16-byte loads.
@@ -202,7 +216,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerCta, kCtasPerSm) k_spmv_slices(d
     constexpr int U = VT == ABHSF_VALUE_F64 ? kUnroll : 2 * kUnroll;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int gw = blockIdx.x * kWarpsPerCta + warp;
-    if (gw >= P.warps)
+    if (begin_fresh(P) || gw >= P.warps)
         return;
     int64_t si = P.wbeg[gw];
     const int64_t s1 = P.wbeg[gw + 1];
@@ -229,7 +243,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerCta, kCtasPerSm) k_spmv_slices(d
         // one row per lane, element k of the lane's row at slot 32 k + lane
         const int len = lane < (int)sl.lanes ? (int)(rec & kLenMask) + 1 : 0;
         const int64_t row = (int64_t)sl.brow * S + (int64_t)(rec >> kLenBits);
-        T acc = len ? Y[row] : T(0);
+        T acc = len && !P.fresh ? Y[row] : T(0);
         uint32_t col = 0;
         // values stay in their stored type until their product: a widening
         // at the load would wait for the prefetch it belongs to
@@ -254,7 +268,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerCta, kCtasPerSm) k_spmv_slices(d
 #pragma unroll
             for (int u = 0; u < U; ++u) {
                 col += w[u];
-                x[u] = k0 + u < len ? __ldg(X + col) : T(0);
+                x[u] = k0 + u < len ? X[col] : T(0);
             }
 #pragma unroll
             for (int u = 0; u < U; ++u)
@@ -353,7 +367,7 @@ __global__ void __launch_bounds__(32 * kChainWarps, kChainCtasPerSm) k_spmv_chai
     extern __shared__ __align__(16) uint8_t chain_smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int gw = blockIdx.x * kChainWarps + warp;
-    if (gw >= P.warps)
+    if (begin_fresh(P) || gw >= P.warps)
         return;
     T* xb = reinterpret_cast<T*>(chain_smem + warp * chain_smem_warp<T, V>());
     V* vb = reinterpret_cast<V*>(xb + 2 * 32 * STX);
@@ -413,7 +427,7 @@ __global__ void __launch_bounds__(32 * kChainWarps, kChainCtasPerSm) k_spmv_chai
     };
     load_words();
     nxt = ahead;
-    T y_nxt = *nxt.y;
+    T y_nxt = P.fresh ? T(0) : *nxt.y;
     advance();
     copy(0);
     asm volatile("cp.async.commit_group;\n" ::: "memory");
@@ -435,7 +449,7 @@ __global__ void __launch_bounds__(32 * kChainWarps, kChainCtasPerSm) k_spmv_chai
         if (more) {
             nxt = ahead;
             if (nxt.b0 == 0)
-                y_nxt = *nxt.y;
+                y_nxt = P.fresh ? T(0) : *nxt.y;
             advance();
             copy(half ^ 1);
             if (ahead.si < s1)
@@ -1017,7 +1031,7 @@ void prepare_stream(abhsf_matrix& a, float avg, cudaStream_t st)
     a.dc_host.clear();
     a.dc_tree_flag.assign((size_t)a.tree_nrows, 0);
     a.dc_warps = a.dc_cwarps = 0;
-    a.dc_beside_ring = false;
+    a.dc_beside_ring = a.dc_every_row = false;
     a.dc_elements = a.dc_rows = a.dc_slots = a.dc_lane_records = 0;
     const int s = a.s, lg = a.lg;
     if (avg <= 0.f || a.tree_nrows == 0 || a.sum_order != ABHSF_SUM_REFERENCE || (uint64_t)a.n > (uint64_t(1) << 32))
@@ -1253,6 +1267,7 @@ void prepare_stream(abhsf_matrix& a, float avg, cudaStream_t st)
                          (int64_t)SL.size() * (int64_t)sizeof(dc_slice) + nS * (int64_t)sizeof(uint32_t);  // a lane record a sliced row
     a.dc_elements = E;
     a.dc_rows = ns;
+    a.dc_every_row = ns == a.tree_nrows && nS + (int64_t)chain_q.size() == a.m;
     a.dc_slots = slots;
     a.dc_lane_records = 32 * nslices;
     deal_slices({&a}, a.dc_sched, a.dc_wbeg, a.dc_warps, st, 0, INT64_MAX, kDealSliced);
@@ -1287,6 +1302,23 @@ void same_carveout(int smem = 0)
     done.fetch_or(bit, std::memory_order_relaxed);
 }
 
+// A fresh launch of sliced rows only is queued while the kernel before it ends
+// (it waits for it on the device); beside chains the events order it.
+void launch_maybe_after(void (*kern)(dc_args), unsigned grid, int threads, int smem, const dc_args& P, cudaStream_t st)
+{
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = (size_t)smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = P.fresh == 2 ? 1 : 0;
+    ABHSF_CUDA(cudaLaunchKernelEx(&cfg, kern, P));
+}
+
 template <int S, int VT, bool B>
 void launch_kind(bool chains, const dc_args& P, cudaStream_t st)
 {
@@ -1294,13 +1326,12 @@ void launch_kind(bool chains, const dc_args& P, cudaStream_t st)
         constexpr int smem = kChainWarps * chain_smem_warp<typename vt_of<VT>::T, typename vt_of<VT>::V>();
         same_carveout<k_spmv_chains<S, VT, B>>(smem);
         const unsigned grid = (unsigned)((P.warps + kChainWarps - 1) / kChainWarps);
-        k_spmv_chains<S, VT, B><<<grid, 32 * kChainWarps, smem, st>>>(P);
+        launch_maybe_after(k_spmv_chains<S, VT, B>, grid, 32 * kChainWarps, smem, P, st);
     } else {
         same_carveout<k_spmv_slices<S, VT, B>>();
         const unsigned grid = (unsigned)((P.warps + kWarpsPerCta - 1) / kWarpsPerCta);
-        k_spmv_slices<S, VT, B><<<grid, 32 * kWarpsPerCta, 0, st>>>(P);
+        launch_maybe_after(k_spmv_slices<S, VT, B>, grid, 32 * kWarpsPerCta, 0, P, st);
     }
-    ABHSF_CUDA(cudaGetLastError());
 }
 
 template <int VT, bool B>
@@ -1456,6 +1487,29 @@ void slices_end(const abhsf_matrix& a, const dc_plan& p, const void* x, int64_t 
     if (p.warps && !beside)
         launch_cols(a.s, a.value_type, false, args_of(a, p.sched, p.wbeg, p.warps, x, ldx, y, ldy, cols), st);
     if (p.cwarps || beside)
+        ABHSF_CUDA(cudaStreamWaitEvent(st, a.dc_join, 0));
+}
+
+bool spmv_sets_y(const abhsf_matrix& a) { return a.dc_every_row; }
+
+void spmv_set_y(const abhsf_matrix& a, const void* x, void* y, const int* skip, cudaStream_t st)
+{
+    std::lock_guard<std::mutex> lock(a.dc_mu);
+    auto args = [&](const dbuf<uint8_t>& sched, const dbuf<int64_t>& wbeg, int warps) {
+        dc_args P = args_of(a, sched.get(), wbeg.get(), warps, x, 1, y, 1, 1);
+        P.fresh = a.dc_cwarps ? 1 : 2;
+        P.skip = skip;
+        return P;
+    };
+    if (a.dc_cwarps) {
+        ABHSF_CUDA(cudaEventRecord(a.dc_fork, st));
+        ABHSF_CUDA(cudaStreamWaitEvent(a.dc_side, a.dc_fork, 0));
+        launch(a.s, a.value_type, false, true, args(a.dc_csched, a.dc_cwbeg, a.dc_cwarps), a.dc_side);
+        ABHSF_CUDA(cudaEventRecord(a.dc_join, a.dc_side));
+    }
+    if (a.dc_warps)
+        launch(a.s, a.value_type, false, false, args(a.dc_sched, a.dc_wbeg, a.dc_warps), st);
+    if (a.dc_cwarps)
         ABHSF_CUDA(cudaStreamWaitEvent(st, a.dc_join, 0));
 }
 
