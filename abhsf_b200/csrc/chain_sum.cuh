@@ -116,7 +116,10 @@ __device__ __forceinline__ bool sum_group(T& y, const T (&p)[L], int lane)
     using B = typename bits_of<T>::B;
     using I = typename B::I;
     constexpr unsigned full = 0xffffffffu;
-    constexpr int kAgain = 12;     // segments run again at most
+    // Segments run again at most.  Adding in turn takes as long as some 16
+    // of 32 segments run again, but 4 of 8 (R-MAT scale 18, 7 columns: 121 us
+    // with 2 or more of 8, 99 with 1).
+    constexpr int kAgain = STRIDE == 1 ? 12 : 1;
     constexpr int kFar = 1 << 20;  // spacings between a start and the end before it
     const int g = lane / STRIDE, h = lane % STRIDE;
     const unsigned mine = (full / ((1u << STRIDE) - 1u)) << h;  // the lanes of this chain

@@ -6,7 +6,6 @@
 #include <atomic>
 #include <cstdint>
 #include <cstdio>
-#include <mutex>
 #include <string>
 #include <utility>
 #include <vector>
@@ -200,7 +199,6 @@ struct abhsf_matrix {
     int ring_bulk = 0;   // x / y blocks as bulk copies (timed at build)
     bool ring_ready = false;  // the ring kernel and the slice kernel together serve this matrix
     bool dc_every_row = false;  // the slices and chains serve every row of the matrix
-    bool dc_beside_ring = false;  // the sliced rows run on dc_side beside the ring kernel (one CTA an SM)
     // delta-coded row slices of the hypersparse block rows (spmv_stream.cu)
     struct dc_slice_host {
         int64_t base = 0;   // first slot of its words and values
@@ -219,12 +217,9 @@ struct abhsf_matrix {
     abhsf::dbuf<uint32_t> seq_rows;      // the non-empty block rows outside the slices (where there are slices):
     int64_t seq_nrows = 0;               // the streaming kernel's (s = 16 / 128 / 256) and the wide SpMM's
     int64_t wide_cap = 0;                // wide SpMM (spmm_wide.cu): bytes of a tile's payload and values (0: none)
-    abhsf::dbuf<uint8_t> dc_csched;      // ... and its chains, launched on dc_side beside the others
+    abhsf::dbuf<uint8_t> dc_csched;      // ... and its chains, launched beside the others
     abhsf::dbuf<int64_t> dc_cwbeg;
     int dc_cwarps = 0;
-    cudaStream_t dc_side = nullptr;      // created with the first chain; forked from the caller's stream
-    cudaEvent_t dc_fork = nullptr, dc_join = nullptr;
-    mutable std::mutex dc_mu;            // one fork / join sequence at a time
     int64_t dc_elements = 0, dc_rows = 0, dc_slots = 0, dc_lane_records = 0;
     float dc_avg = 0.f;                  // largest mean elements per tile of a slice block row (0: none)
     abhsf::dbuf<int> dev_status;  // ABHSF_DEVSTAT_* bits set by kernels
@@ -254,12 +249,6 @@ struct abhsf_matrix {
     abhsf_matrix& operator=(const abhsf_matrix&) = delete;
     ~abhsf_matrix()
     {
-        if (dc_fork)
-            cudaEventDestroy(dc_fork);
-        if (dc_join)
-            cudaEventDestroy(dc_join);
-        if (dc_side)
-            cudaStreamDestroy(dc_side);
         for (cudaEvent_t e : host_events)
             cudaEventDestroy(e);
         if (host_in)
@@ -309,20 +298,8 @@ struct abhsf_batch {
     abhsf::dbuf<uint8_t> dc_csched;
     abhsf::dbuf<int64_t> dc_cwbeg;
     int dc_cwarps = 0;
-    cudaStream_t dc_side = nullptr;
-    cudaEvent_t dc_fork = nullptr, dc_join = nullptr;
-    mutable std::mutex dc_mu;
 
     abhsf_batch() = default;
     abhsf_batch(const abhsf_batch&) = delete;
     abhsf_batch& operator=(const abhsf_batch&) = delete;
-    ~abhsf_batch()
-    {
-        if (dc_fork)
-            cudaEventDestroy(dc_fork);
-        if (dc_join)
-            cudaEventDestroy(dc_join);
-        if (dc_side)
-            cudaStreamDestroy(dc_side);
-    }
 };

@@ -5,6 +5,7 @@
 #include <string>
 #include <memory>
 
+#include "beside.cuh"
 #include "common.cuh"
 
 namespace abhsf {
@@ -106,10 +107,10 @@ void batch_seq_spmv(const abhsf_batch& b, const double* const* xs, double* const
 // elements per tile on average), encodes them and deals the slices;
 // deal_slices deals the slices of one kind (deal_kind) of block rows
 // [brow_lo, brow_hi) of several matrices over one launch.  A launch plan
-// names the schedules; slices_begin forks the chains onto the side stream
-// (call it before the ring kernel, so that they run beside it) and
-// slices_end adds the sliced rows on st and joins the chains back (x[i * ldx],
-// y[i * ldy]).  The caller holds dc_mu across the pair.
+// names the schedules; slices_begin queues the chains (the longest bounds the
+// launch, so they take their place on the SMs first), slices_end the sliced rows
+// (x[i * ldx], y[i * ldy]); they and the kernel between them run side by side
+// (beside.cuh).
 void prepare_stream(abhsf_matrix& a, float avg, cudaStream_t st);
 // Parts of a matrix's block rows the host-memory SpMV (abhsf_spmv_host)
 // copies in, sums and copies out one after another: [M c / kHostChunks,
@@ -134,13 +135,13 @@ struct dc_plan {
 dc_plan plan_of(const abhsf_matrix& a);
 // cols > 1 (FP64 only): Y += A X over that many columns in one launch, each
 // column bitwise its SpMV.
-void slices_begin(const abhsf_matrix& a, const dc_plan& p, const void* x, int64_t ldx, void* y, int64_t ldy,
-                  cudaStream_t st, int cols = 1);
-void slices_end(const abhsf_matrix& a, const dc_plan& p, const void* x, int64_t ldx, void* y, int64_t ldy,
+void slices_begin(beside& bs, const abhsf_matrix& a, const dc_plan& p, const void* x, int64_t ldx, void* y,
+                  int64_t ldy, cudaStream_t st, int cols = 1);
+void slices_end(beside& bs, const abhsf_matrix& a, const dc_plan& p, const void* x, int64_t ldx, void* y, int64_t ldy,
                 cudaStream_t st, int cols = 1);
 void prepare_batch_stream(abhsf_batch& b, cudaStream_t st);
-void batch_stream_begin(const abhsf_batch& b, const double* const* xs, double* const* ys, cudaStream_t st);
-void batch_stream_end(const abhsf_batch& b, const double* const* xs, double* const* ys, cudaStream_t st);
+void batch_stream_begin(beside& bs, const abhsf_batch& b, const double* const* xs, double* const* ys, cudaStream_t st);
+void batch_stream_end(beside& bs, const abhsf_batch& b, const double* const* xs, double* const* ys, cudaStream_t st);
 
 // y = A x (y need not be zeroed) through the slices and chains, or nothing at
 // all where *skip is set (device memory): for matrices whose every row they
@@ -172,7 +173,7 @@ bool spmm_f64_wide(const abhsf_matrix& a, int k, const double* X, int64_t ldx, d
                    cudaStream_t st);
 // ... its block sizes 32 and 64 (spmv_ring.cu): kt = 16 or 32 columns of X and
 // Y over the block rows given, with the ring's per-scheme sums (a row a lane).
-void spmm_staged(const abhsf_matrix& a, int kt, const uint32_t* rows, int64_t nrows, const double* X, int64_t ldx,
+void spmm_staged(beside& bs, const abhsf_matrix& a, int kt, const uint32_t* rows, int64_t nrows, const double* X, int64_t ldx,
                  double* Y, int64_t ldy, cudaStream_t st);
 // Y += A X (k columns, row-major X and Y) through the same kernel, several
 // right-hand sides per pass; false when the matrix has no ring schedule.

@@ -204,6 +204,7 @@ __global__ void __launch_bounds__(kWideThreads, wide_min_ctas<S>()) k_spmm_wide(
     const tiles_view& A = P.A;
     uint16_t* marks = reinterpret_cast<uint16_t*>(wide_smem + 2 * P.stage_bytes);
     int64_t k = blockIdx.x;
+    beside_begin();
     if (k >= P.nrows)
         return;
     int64_t I = P.rows[k], t = A.brow_ptr[I], tend = A.brow_ptr[I + 1];
@@ -263,6 +264,7 @@ __global__ void __launch_bounds__(kWideThreads, wide_min_ctas<S>()) k_spmm_wide(
         tend = tne;
         cur ^= 1;
     }
+    beside_end();
 }
 
 // Largest payload + value bytes of one tile.
@@ -284,7 +286,7 @@ int wide_smem_bytes(const abhsf_matrix& a)
 }
 
 template <int S, int K>
-void launch_wide(const abhsf_matrix& a, const uint32_t* rows, int64_t nrows, const double* X, int64_t ldx, double* Y,
+void launch_wide(beside& bs, const abhsf_matrix& a, const uint32_t* rows, int64_t nrows, const double* X, int64_t ldx, double* Y,
                  int64_t ldy, cudaStream_t st)
 {
     const int smem = wide_smem_bytes<S, K>(a);
@@ -300,8 +302,7 @@ void launch_wide(const abhsf_matrix& a, const uint32_t* rows, int64_t nrows, con
         fail(ABHSF_ERROR_UNSUPPORTED, "wide SpMM: the stages do not fit shared memory");
     const unsigned grid = (unsigned)std::min<int64_t>(nrows, (int64_t)nsm * per_sm);
     wide_args P{a.view(), rows, nrows, X, Y, ldx, ldy, x_block_bytes<S, K>() + (int)a.wide_cap};
-    kern<<<grid, kWideThreads, smem, st>>>(P);
-    ABHSF_CUDA(cudaGetLastError());
+    launch_beside(bs, kern, grid, kWideThreads, (size_t)smem, st, P);
 }
 
 }  // namespace
@@ -338,21 +339,21 @@ bool spmm_f64_wide(const abhsf_matrix& a, int k, const double* X, int64_t ldx, d
     const bool sliced = a.dc_rows > 0;
     const uint32_t* rows = sliced ? a.seq_rows.get() : a.tree_rows.get();
     const int64_t nrows = sliced ? a.seq_nrows : a.tree_nrows;
-    std::lock_guard<std::mutex> lock(a.dc_mu);
+    beside bs;
     const dc_plan p = plan_of(a);
     for (int j = 0; j < k;) {
         const int cols = k - j >= 32 ? 32 : 16;
         if (nrows > 0 && (a.s == 32 || a.s == 64))
-            spmm_staged(a, cols, rows, nrows, X + j, ldx, Y + j, ldy, st);
+            spmm_staged(bs, a, cols, rows, nrows, X + j, ldx, Y + j, ldy, st);
         else if (nrows > 0 && cols == 32)
-            launch_wide<16, 32>(a, rows, nrows, X + j, ldx, Y + j, ldy, st);
+            launch_wide<16, 32>(bs, a, rows, nrows, X + j, ldx, Y + j, ldy, st);
         else if (nrows > 0)
-            launch_wide<16, 16>(a, rows, nrows, X + j, ldx, Y + j, ldy, st);
+            launch_wide<16, 16>(bs, a, rows, nrows, X + j, ldx, Y + j, ldy, st);
         j += cols;
     }
     if (sliced) {
-        slices_begin(a, p, X, ldx, Y, ldy, st, k);
-        slices_end(a, p, X, ldx, Y, ldy, st, k);
+        slices_begin(bs, a, p, X, ldx, Y, ldy, st, k);
+        slices_end(bs, a, p, X, ldx, Y, ldy, st, k);
     }
     return true;
 }

@@ -902,6 +902,7 @@ __global__ void __launch_bounds__(staged_cfg<S, KT, KW, RPL>::NT) k_spmm_staged(
         q.tend = A.brow_ptr[q.I + 1];
         return true;
     };
+    beside_begin();
     if ((int64_t)blockIdx.x >= P.nrows)
         return;
     pos p0;
@@ -998,10 +999,11 @@ __global__ void __launch_bounds__(staged_cfg<S, KT, KW, RPL>::NT) k_spmm_staged(
         more1 = more2;
         cur ^= 1;
     }
+    beside_end();
 }
 
 template <int S, int KT, int KW, int RPL>
-void launch_staged(const abhsf_matrix& a, const uint32_t* rows, int64_t nrows, const double* X, int64_t ldx,
+void launch_staged(beside& bs, const abhsf_matrix& a, const uint32_t* rows, int64_t nrows, const double* X, int64_t ldx,
                    double* Y, int64_t ldy, cudaStream_t st)
 {
     constexpr int NT = staged_cfg<S, KT, KW, RPL>::NT, NW = staged_cfg<S, KT, KW, RPL>::NW;
@@ -1019,8 +1021,7 @@ void launch_staged(const abhsf_matrix& a, const uint32_t* rows, int64_t nrows, c
         fail(ABHSF_ERROR_UNSUPPORTED, "staged SpMM: the stages do not fit shared memory");
     const unsigned grid = (unsigned)std::min<int64_t>(nrows, (int64_t)nsm * per_sm);
     staged_args P{a.view(), rows, nrows, X, Y, ldx, ldy, stage_bytes};
-    kern<<<grid, NT, smem, st>>>(P);
-    ABHSF_CUDA(cudaGetLastError());
+    launch_beside(bs, kern, grid, NT, (size_t)smem, st, P);
 }
 
 // Warps 0 .. TM NC - 1 sum, NC per team; the last warp produces.
@@ -1039,6 +1040,7 @@ __global__ void __launch_bounds__(ring_threads<S, LY>(), kCtasPerSm) k_spmv_f64_
     const int n = (int)(P.wbeg[blockIdx.x + 1] - eb);
     const ring_desc* D = P.desc + eb;
     volatile int* abort = &sm.abort;
+    beside_begin();
     if (tid == 0) {
         for (int b = 0; b < kMaxQ; ++b) {
             mbar_init(&sm.full[b], 32 + 1);  // the producer lanes' cp.async arrivals + the expect_tx arrival
@@ -1216,6 +1218,7 @@ __global__ void __launch_bounds__(ring_threads<S, LY>(), kCtasPerSm) k_spmv_f64_
         }
         __syncthreads();
     }
+    beside_end();
 }
 
 // Bytes a block row moves through the ring, plus a fixed cost per tile and
@@ -1281,30 +1284,30 @@ __global__ void k_ring_max_pv(int64_t T, tiles_view A, int vsize, unsigned int* 
 // The kernel in consumer layout L (single right-hand side; passes of K > 1
 // right-hand sides use layout 0).
 template <int S, int K, int VT, bool B, int L>
-void launch_layout(unsigned grid, const ring_args& P, cudaStream_t st)
+void launch_layout(beside& bs, unsigned grid, const ring_args& P, cudaStream_t st)
 {
-    k_spmv_f64_ring<S, K, VT, B, L><<<grid, ring_threads<S, L>(), sizeof(ring_smem<S, K, VT>), st>>>(P);
+    launch_beside(bs, k_spmv_f64_ring<S, K, VT, B, L>, grid, ring_threads<S, L>(), sizeof(ring_smem<S, K, VT>), st, P);
 }
 
 template <int S, int K, int VT, bool B>
-void launch_any(int layout, unsigned grid, const ring_args& P, cudaStream_t st)
+void launch_any(beside& bs, int layout, unsigned grid, const ring_args& P, cudaStream_t st)
 {
     if constexpr (K == 1) {
         switch (layout) {
-        case 1: launch_layout<S, K, VT, B, 1>(grid, P, st); break;
-        case 2: launch_layout<S, K, VT, B, 2>(grid, P, st); break;
-        case 3: launch_layout<S, K, VT, B, 3>(grid, P, st); break;
-        default: launch_layout<S, K, VT, B, 0>(grid, P, st); break;
+        case 1: launch_layout<S, K, VT, B, 1>(bs, grid, P, st); break;
+        case 2: launch_layout<S, K, VT, B, 2>(bs, grid, P, st); break;
+        case 3: launch_layout<S, K, VT, B, 3>(bs, grid, P, st); break;
+        default: launch_layout<S, K, VT, B, 0>(bs, grid, P, st); break;
         }
     } else {
-        launch_layout<S, K, VT, B, 0>(grid, P, st);
+        launch_layout<S, K, VT, B, 0>(bs, grid, P, st);
     }
     ABHSF_CUDA(cudaGetLastError());
 }
 
 // One pass: K right-hand sides, X and Y starting at their first column.
 template <int S, int K, int VT>
-void launch_ring(const abhsf_matrix& a, const void* x, int64_t ldx, void* y, int64_t ldy, cudaStream_t st,
+void launch_ring(beside& bs, const abhsf_matrix& a, const void* x, int64_t ldx, void* y, int64_t ldy, cudaStream_t st,
                  bool tuning = false, const uint8_t* desc = nullptr, const int64_t* wbeg = nullptr, int ctas = 0)
 {
     static_assert(((sizeof(ring_smem<S, K, VT>) + 1023) / 1024 + 1) * 1024 * kCtasPerSm <= 233472,
@@ -1317,7 +1320,7 @@ void launch_ring(const abhsf_matrix& a, const void* x, int64_t ldx, void* y, int
     ring_args P{a.view(), reinterpret_cast<const ring_desc*>(desc), wbeg, x, y, ldx, ldy, nullptr, nullptr, nullptr,
                 a.dev_status.get(), a.ring_bulk, tuning ? -1 : g_drop_desc,
                 (g_spin_limit && !tuning) ? g_spin_limit : kWaitPolls};
-    launch_any<S, K, VT, false>(a.ring_layout, (unsigned)ctas, P, st);
+    launch_any<S, K, VT, false>(bs, a.ring_layout, (unsigned)ctas, P, st);
 }
 
 template <int S, int K, int VT, bool B = false, int L = 0>
@@ -1341,21 +1344,21 @@ bool ring_fits(const abhsf_matrix& a)
 
 // Y += A X over columns [0, k) in passes of the largest K that fits.
 template <int S>
-void spmm_ring(const abhsf_matrix& a, int k, const double* X, int64_t ldx, double* Y, int64_t ldy, cudaStream_t st)
+void spmm_ring(beside& bs, const abhsf_matrix& a, int k, const double* X, int64_t ldx, double* Y, int64_t ldy, cudaStream_t st)
 {
     for (int j = 0; j < k;) {
         const int left = k - j;
         if (left >= 8 && ring_fits<S, 8, ABHSF_VALUE_F64>(a)) {
-            launch_ring<S, 8, ABHSF_VALUE_F64>(a, X + j, ldx, Y + j, ldy, st);
+            launch_ring<S, 8, ABHSF_VALUE_F64>(bs, a, X + j, ldx, Y + j, ldy, st);
             j += 8;
         } else if (left >= 4 && ring_fits<S, 4, ABHSF_VALUE_F64>(a)) {
-            launch_ring<S, 4, ABHSF_VALUE_F64>(a, X + j, ldx, Y + j, ldy, st);
+            launch_ring<S, 4, ABHSF_VALUE_F64>(bs, a, X + j, ldx, Y + j, ldy, st);
             j += 4;
         } else if (left >= 2 && ring_fits<S, 2, ABHSF_VALUE_F64>(a)) {
-            launch_ring<S, 2, ABHSF_VALUE_F64>(a, X + j, ldx, Y + j, ldy, st);
+            launch_ring<S, 2, ABHSF_VALUE_F64>(bs, a, X + j, ldx, Y + j, ldy, st);
             j += 2;
         } else {
-            launch_ring<S, 1, ABHSF_VALUE_F64>(a, X + j, ldx, Y + j, ldy, st);
+            launch_ring<S, 1, ABHSF_VALUE_F64>(bs, a, X + j, ldx, Y + j, ldy, st);
             j += 1;
         }
     }
@@ -1479,7 +1482,8 @@ void tune_ring(abhsf_matrix& a, cudaStream_t st)
         [&](int tm, int bk) {
             a.ring_layout = tm;
             a.ring_bulk = bk;
-            launch_ring<S, 1, VT>(a, x.get(), 1, y.get(), 1, st, true);
+            beside bs;
+            launch_ring<S, 1, VT>(bs, a, x.get(), 1, y.get(), 1, st, true);
         },
         S, st, layout, bulk);
     a.ring_layout = layout;
@@ -1645,7 +1649,7 @@ void ring_set_up_all()
     ring_ctas_per_sm<S, 8, ABHSF_VALUE_F64>();
 }
 
-void batch_launch(const abhsf_batch& b, const double* const* xs, double* const* ys, cudaStream_t st, bool tuning)
+void batch_launch(beside& bs, const abhsf_batch& b, const double* const* xs, double* const* ys, cudaStream_t st, bool tuning)
 {
     ring_args P{};
     P.desc = reinterpret_cast<const ring_desc*>(b.desc.get());
@@ -1659,9 +1663,9 @@ void batch_launch(const abhsf_batch& b, const double* const* xs, double* const* 
     P.drop = -1;
     P.polls = (g_spin_limit && !tuning) ? g_spin_limit : kWaitPolls;
     if (b.s == 32)
-        launch_any<32, 1, ABHSF_VALUE_F64, true>(b.layout, (unsigned)b.ctas, P, st);
+        launch_any<32, 1, ABHSF_VALUE_F64, true>(bs, b.layout, (unsigned)b.ctas, P, st);
     else
-        launch_any<64, 1, ABHSF_VALUE_F64, true>(b.layout, (unsigned)b.ctas, P, st);
+        launch_any<64, 1, ABHSF_VALUE_F64, true>(bs, b.layout, (unsigned)b.ctas, P, st);
 }
 
 
@@ -1780,7 +1784,8 @@ void prepare_batch(abhsf_batch& b, cudaStream_t st)
                 [&](int tm, int bk) {
                     b.layout = tm;
                     b.bulk = bk;
-                    batch_launch(b, xs_d.get(), ys_d.get(), st, true);
+                    beside bs;
+                    batch_launch(bs, b, xs_d.get(), ys_d.get(), st, true);
                 },
                 b.s, st, layout, bulk);
         b.layout = layout;
@@ -1792,11 +1797,13 @@ void prepare_batch(abhsf_batch& b, cudaStream_t st)
 
 void batch_spmv(const abhsf_batch& b, const double* const* xs, double* const* ys, cudaStream_t st)
 {
-    std::lock_guard<std::mutex> lock(b.dc_mu);
-    batch_stream_begin(b, xs, ys, st);  // the chains, beside the rest
+    beside bs;
+// The ring first: a chain CTA's 73 KB would keep two of the ring's five CTAs
+    // from an SM (chains first 844 us, ring first 791, on the 256-matrix batch).
     if (b.ctas > 0)
-        batch_launch(b, xs, ys, st, false);
-    batch_stream_end(b, xs, ys, st);
+        batch_launch(bs, b, xs, ys, st, false);
+    batch_stream_begin(bs, b, xs, ys, st);
+    batch_stream_end(bs, b, xs, ys, st);
 }
 
 
@@ -1805,16 +1812,16 @@ bool spmv_f64_ring(const abhsf_matrix& a, const double* x, double* y, cudaStream
 {
     if (!a.ring_ready || a.value_type != ABHSF_VALUE_F64)
         return false;
-    std::lock_guard<std::mutex> lock(a.dc_mu);
+    beside bs;
     const dc_plan p = plan_of(a);
-    slices_begin(a, p, x, 1, y, 1, st);  // the chains, beside the rest
+    slices_begin(bs, a, p, x, 1, y, 1, st);  // the chains, beside the rest
     if (a.ring_warps) {
         if (a.s == 32)
-            launch_ring<32, 1, ABHSF_VALUE_F64>(a, x, 1, y, 1, st);
+            launch_ring<32, 1, ABHSF_VALUE_F64>(bs, a, x, 1, y, 1, st);
         else
-            launch_ring<64, 1, ABHSF_VALUE_F64>(a, x, 1, y, 1, st);
+            launch_ring<64, 1, ABHSF_VALUE_F64>(bs, a, x, 1, y, 1, st);
     }
-    slices_end(a, p, x, 1, y, 1, st);
+    slices_end(bs, a, p, x, 1, y, 1, st);
     return true;
 }
 
@@ -1826,23 +1833,23 @@ void spmv_f32_dispatch(const abhsf_matrix& a, const float* x, float* y, cudaStre
         spmv_f32_seq(a, x, y, st);  // block sizes 16, 128, 256 (slices beside it), or no ring schedule
         return;
     }
-    std::lock_guard<std::mutex> lock(a.dc_mu);
+    beside bs;
     const dc_plan p = plan_of(a);
-    slices_begin(a, p, x, 1, y, 1, st);
+    slices_begin(bs, a, p, x, 1, y, 1, st);
     if (a.ring_warps) {
         if (a.value_type == ABHSF_VALUE_F32) {
             if (a.s == 32)
-                launch_ring<32, 1, ABHSF_VALUE_F32>(a, x, 1, y, 1, st);
+                launch_ring<32, 1, ABHSF_VALUE_F32>(bs, a, x, 1, y, 1, st);
             else
-                launch_ring<64, 1, ABHSF_VALUE_F32>(a, x, 1, y, 1, st);
+                launch_ring<64, 1, ABHSF_VALUE_F32>(bs, a, x, 1, y, 1, st);
         } else {
             if (a.s == 32)
-                launch_ring<32, 1, ABHSF_VALUE_BF16>(a, x, 1, y, 1, st);
+                launch_ring<32, 1, ABHSF_VALUE_BF16>(bs, a, x, 1, y, 1, st);
             else
-                launch_ring<64, 1, ABHSF_VALUE_BF16>(a, x, 1, y, 1, st);
+                launch_ring<64, 1, ABHSF_VALUE_BF16>(bs, a, x, 1, y, 1, st);
         }
     }
-    slices_end(a, p, x, 1, y, 1, st);
+    slices_end(bs, a, p, x, 1, y, 1, st);
 }
 
 bool spmv_f64_ring_host(abhsf_matrix& a, const double* x, double* y, cudaStream_t st)
@@ -1888,8 +1895,8 @@ bool spmv_f64_ring_host(abhsf_matrix& a, const double* x, double* y, cudaStream_
         ABHSF_CUDA(cudaMemcpyAsync(ys + r0, y + r0, (r1 - r0) * sizeof(double), cudaMemcpyHostToDevice, a.host_in));
         ABHSF_CUDA(cudaEventRecord(ev[1 + c], a.host_in));
     }
-    std::lock_guard<std::mutex> lock(a.dc_mu);
     for (int c = 0; c < kChunks; ++c) {
+        beside bs;
         const auto& ch = a.host_chunks[c];
         ABHSF_CUDA(cudaStreamWaitEvent(st, ev[1 + c], 0));
         dc_plan p;
@@ -1899,14 +1906,14 @@ bool spmv_f64_ring_host(abhsf_matrix& a, const double* x, double* y, cudaStream_
         p.csched = ch.dc_csched.get();
         p.cwbeg = ch.dc_cwbeg.get();
         p.cwarps = ch.dc_cwarps;
-        slices_begin(a, p, xs, 1, ys, 1, st);
+        slices_begin(bs, a, p, xs, 1, ys, 1, st);
         if (ch.ctas > 0) {
             if (a.s == 32)
-                launch_ring<32, 1, ABHSF_VALUE_F64>(a, xs, 1, ys, 1, st, false, ch.desc.get(), ch.wbeg.get(), ch.ctas);
+                launch_ring<32, 1, ABHSF_VALUE_F64>(bs, a, xs, 1, ys, 1, st, false, ch.desc.get(), ch.wbeg.get(), ch.ctas);
             else
-                launch_ring<64, 1, ABHSF_VALUE_F64>(a, xs, 1, ys, 1, st, false, ch.desc.get(), ch.wbeg.get(), ch.ctas);
+                launch_ring<64, 1, ABHSF_VALUE_F64>(bs, a, xs, 1, ys, 1, st, false, ch.desc.get(), ch.wbeg.get(), ch.ctas);
         }
-        slices_end(a, p, xs, 1, ys, 1, st);
+        slices_end(bs, a, p, xs, 1, ys, 1, st);
         ABHSF_CUDA(cudaEventRecord(ev[1 + kChunks + c], st));
     }
     for (int c = 0; c < kChunks; ++c) {
@@ -1920,7 +1927,7 @@ bool spmv_f64_ring_host(abhsf_matrix& a, const double* x, double* y, cudaStream_
     return true;
 }
 
-void spmm_staged(const abhsf_matrix& a, int kt, const uint32_t* rows, int64_t nrows, const double* X, int64_t ldx,
+void spmm_staged(beside& bs, const abhsf_matrix& a, int kt, const uint32_t* rows, int64_t nrows, const double* X, int64_t ldx,
                  double* Y, int64_t ldy, cudaStream_t st)
 {
     // 16 columns: 4 a warp, so that a CTA keeps as many warps as at 32 (tiled
@@ -1928,11 +1935,11 @@ void spmm_staged(const abhsf_matrix& a, int kt, const uint32_t* rows, int64_t nr
     // lane (RPL = 2, each x row read once for the 64 rows) measured 1.31 ms
     // at 32 columns against 1.07 with one: fewer warps for the same stages.
     if (a.s == 32) {
-        kt == 32 ? launch_staged<32, 32, 8, 1>(a, rows, nrows, X, ldx, Y, ldy, st)
-                 : launch_staged<32, 16, 4, 1>(a, rows, nrows, X, ldx, Y, ldy, st);
+        kt == 32 ? launch_staged<32, 32, 8, 1>(bs, a, rows, nrows, X, ldx, Y, ldy, st)
+                 : launch_staged<32, 16, 4, 1>(bs, a, rows, nrows, X, ldx, Y, ldy, st);
     } else {
-        kt == 32 ? launch_staged<64, 32, 8, 1>(a, rows, nrows, X, ldx, Y, ldy, st)
-                 : launch_staged<64, 16, 4, 1>(a, rows, nrows, X, ldx, Y, ldy, st);
+        kt == 32 ? launch_staged<64, 32, 8, 1>(bs, a, rows, nrows, X, ldx, Y, ldy, st)
+                 : launch_staged<64, 16, 4, 1>(bs, a, rows, nrows, X, ldx, Y, ldy, st);
     }
 }
 
@@ -1941,16 +1948,16 @@ bool spmm_f64_ring(const abhsf_matrix& a, int k, const double* X, int64_t ldx, d
 {
     if (!a.ring_ready || a.value_type != ABHSF_VALUE_F64)
         return false;
-    std::lock_guard<std::mutex> lock(a.dc_mu);
+    beside bs;
     const dc_plan p = plan_of(a);
     if (a.ring_warps) {
         if (a.s == 32)
-            spmm_ring<32>(a, k, X, ldx, Y, ldy, st);
+            spmm_ring<32>(bs, a, k, X, ldx, Y, ldy, st);
         else
-            spmm_ring<64>(a, k, X, ldx, Y, ldy, st);
+            spmm_ring<64>(bs, a, k, X, ldx, Y, ldy, st);
     }
-    slices_begin(a, p, X, ldx, Y, ldy, st, k);  // the slice rows, every column in one launch
-    slices_end(a, p, X, ldx, Y, ldy, st, k);
+    slices_begin(bs, a, p, X, ldx, Y, ldy, st, k);  // the slice rows, every column in one launch
+    slices_end(bs, a, p, X, ldx, Y, ldy, st, k);
     return true;
 }
 

@@ -430,7 +430,7 @@ __device__ __forceinline__ void seq_block_row(const tiles_view& A, const void* x
 }
 
 template <int S, int VT, bool B = false>
-__global__ void __launch_bounds__(kWarps * 32, kMinCtasPerSm) k_spmv_seq(seq_args P)
+__global__ void __launch_bounds__(kWarps * 32, S == 16 && !B ? 8 : kMinCtasPerSm) k_spmv_seq(seq_args P)
 {
     using T = typename seq_t<VT>::T;
     __shared__ seq_smem<S, T> smem[kWarps];
@@ -438,6 +438,7 @@ __global__ void __launch_bounds__(kWarps * 32, kMinCtasPerSm) k_spmv_seq(seq_arg
     seq_smem<S, T>& sm = smem[threadIdx.x >> 5];
     const unsigned int nw = gridDim.x * kWarps;
     unsigned int k = blockIdx.x * kWarps + (threadIdx.x >> 5);
+    beside_begin();
     while ((int64_t)k < P.nrows) {
         unsigned int next = 0;
         if (lane == 0)
@@ -451,10 +452,13 @@ __global__ void __launch_bounds__(kWarps * 32, kMinCtasPerSm) k_spmv_seq(seq_arg
         }
         k = __shfl_sync(kFull, next, 0);
     }
+    beside_end();
 }
 
+// (the work counter is cleared by the caller before the product's first kernel:
+// nothing may come between its kernels)
 template <int S, int VT>
-void launch_seq(const abhsf_matrix& a, const uint32_t* rows, int64_t nrows, const void* x, void* y, cudaStream_t st)
+void launch_seq(beside& bs, const abhsf_matrix& a, const uint32_t* rows, int64_t nrows, const void* x, void* y, cudaStream_t st)
 {
     if (nrows == 0)
         return;
@@ -463,23 +467,21 @@ void launch_seq(const abhsf_matrix& a, const uint32_t* rows, int64_t nrows, cons
     ABHSF_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
     ABHSF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_spmv_seq<S, VT>, kWarps * 32, 0));
     seq_args P{a.view(), rows, nrows, a.tree_counter.get(), x, y, nullptr, nullptr, nullptr, nullptr};
-    ABHSF_CUDA(cudaMemsetAsync(a.tree_counter.get(), 0, sizeof(unsigned int), st));
     const int64_t ctas = (nrows + kWarps - 1) / kWarps;
     const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(ctas, (int64_t)nsm * std::max(per_sm, 1)));
-    k_spmv_seq<S, VT><<<grid, kWarps * 32, 0, st>>>(P);
-    ABHSF_CUDA(cudaGetLastError());
+    launch_beside(bs, k_spmv_seq<S, VT, false>, grid, kWarps * 32, 0, st, P);
 }
 
 template <int VT>
-void launch_seq_vt(const abhsf_matrix& a, const uint32_t* rows, int64_t nrows, const void* x, void* y,
+void launch_seq_vt(beside& bs, const abhsf_matrix& a, const uint32_t* rows, int64_t nrows, const void* x, void* y,
                    cudaStream_t st)
 {
     switch (a.s) {
-    case 16: launch_seq<16, VT>(a, rows, nrows, x, y, st); break;
-    case 32: launch_seq<32, VT>(a, rows, nrows, x, y, st); break;
-    case 64: launch_seq<64, VT>(a, rows, nrows, x, y, st); break;
-    case 128: launch_seq<128, VT>(a, rows, nrows, x, y, st); break;
-    case 256: launch_seq<256, VT>(a, rows, nrows, x, y, st); break;
+    case 16: launch_seq<16, VT>(bs, a, rows, nrows, x, y, st); break;
+    case 32: launch_seq<32, VT>(bs, a, rows, nrows, x, y, st); break;
+    case 64: launch_seq<64, VT>(bs, a, rows, nrows, x, y, st); break;
+    case 128: launch_seq<128, VT>(bs, a, rows, nrows, x, y, st); break;
+    case 256: launch_seq<256, VT>(bs, a, rows, nrows, x, y, st); break;
     default: fail(ABHSF_ERROR_UNSUPPORTED, "block size without an SpMV kernel");
     }
 }
@@ -491,25 +493,25 @@ void seq_any(const abhsf_matrix& a, const void* x, void* y, cudaStream_t st)
     if (a.M == 0 || a.T == 0)
         return;
     const bool slices = a.dc_rows > 0 && a.sum_order == ABHSF_SUM_REFERENCE && a.s != 32 && a.s != 64;
-    std::unique_lock<std::mutex> lock(a.dc_mu, std::defer_lock);
+    beside bs;
     dc_plan p;
     const uint32_t* rows = a.tree_rows.get();
     int64_t nrows = a.tree_nrows;
+    ABHSF_CUDA(cudaMemsetAsync(a.tree_counter.get(), 0, sizeof(unsigned int), st));
     if (slices) {
-        lock.lock();
         p = plan_of(a);
-        slices_begin(a, p, x, 1, y, 1, st);
+        slices_begin(bs, a, p, x, 1, y, 1, st);
         rows = a.seq_rows.get();
         nrows = a.seq_nrows;
     }
     if (a.value_type == ABHSF_VALUE_F64)
-        launch_seq_vt<ABHSF_VALUE_F64>(a, rows, nrows, x, y, st);
+        launch_seq_vt<ABHSF_VALUE_F64>(bs, a, rows, nrows, x, y, st);
     else if (a.value_type == ABHSF_VALUE_F32)
-        launch_seq_vt<ABHSF_VALUE_F32>(a, rows, nrows, x, y, st);
+        launch_seq_vt<ABHSF_VALUE_F32>(bs, a, rows, nrows, x, y, st);
     else
-        launch_seq_vt<ABHSF_VALUE_BF16>(a, rows, nrows, x, y, st);
+        launch_seq_vt<ABHSF_VALUE_BF16>(bs, a, rows, nrows, x, y, st);
     if (slices)
-        slices_end(a, p, x, 1, y, 1, st);
+        slices_end(bs, a, p, x, 1, y, 1, st);
 }
 
 }  // namespace
@@ -568,7 +570,7 @@ void prepare_batch_seq(abhsf_batch& b, cudaStream_t st)
 namespace {
 
 template <int S>
-void launch_batch_seq(const abhsf_batch& b, const double* const* xs, double* const* ys, cudaStream_t st)
+void launch_batch_seq(beside& bs, const abhsf_batch& b, const double* const* xs, double* const* ys, cudaStream_t st)
 {
     int dev = 0, nsm = 0, per_sm = 0;
     ABHSF_CUDA(cudaGetDevice(&dev));
@@ -582,28 +584,28 @@ void launch_batch_seq(const abhsf_batch& b, const double* const* xs, double* con
     P.items = b.seq_items.get();
     P.xs = reinterpret_cast<const void* const*>(xs);
     P.ys = reinterpret_cast<void* const*>(ys);
-    ABHSF_CUDA(cudaMemsetAsync(b.seq_counter.get(), 0, sizeof(unsigned int), st));
     const int64_t ctas = (b.seq_nitems + kWarps - 1) / kWarps;
     const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(ctas, (int64_t)nsm * std::max(per_sm, 1)));
-    kern<<<grid, kWarps * 32, 0, st>>>(P);
-    ABHSF_CUDA(cudaGetLastError());
+    launch_beside(bs, kern, grid, kWarps * 32, 0, st, P);
 }
 
 }  // namespace
 
 void batch_seq_spmv(const abhsf_batch& b, const double* const* xs, double* const* ys, cudaStream_t st)
 {
-    std::lock_guard<std::mutex> lock(b.dc_mu);
-    batch_stream_begin(b, xs, ys, st);  // the chains, beside the rest
+    beside bs;
+    if (b.seq_nitems > 0)
+        ABHSF_CUDA(cudaMemsetAsync(b.seq_counter.get(), 0, sizeof(unsigned int), st));
+    batch_stream_begin(bs, b, xs, ys, st);  // the chains, beside the rest
     if (b.seq_nitems > 0) {
         switch (b.s) {
-        case 16: launch_batch_seq<16>(b, xs, ys, st); break;
-        case 128: launch_batch_seq<128>(b, xs, ys, st); break;
-        case 256: launch_batch_seq<256>(b, xs, ys, st); break;
+        case 16: launch_batch_seq<16>(bs, b, xs, ys, st); break;
+        case 128: launch_batch_seq<128>(bs, b, xs, ys, st); break;
+        case 256: launch_batch_seq<256>(bs, b, xs, ys, st); break;
         default: fail(ABHSF_ERROR_UNSUPPORTED, "the batched streaming kernel serves block sizes 16, 128, 256");
         }
     }
-    batch_stream_end(b, xs, ys, st);
+    batch_stream_end(bs, b, xs, ys, st);
 }
 
 void spmv_f32_seq(const abhsf_matrix& a, const float* x, float* y, cudaStream_t st)

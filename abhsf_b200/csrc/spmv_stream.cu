@@ -26,15 +26,14 @@
 // running sum of the deltas, x gathered through L2 -- and adds each product
 // onto its row's sum in column order, starting from y: the order of the
 // reference CSR's spmv_naive (spmv/bottlenecks/spmv.cpp:58-64), so y is
-// bitwise the same.  A chain (its own kernel, on a side stream forked from
-// the caller's so that it runs beside the others): 512 products at a time,
+// bitwise the same.  A chain (its own kernel, queued first and run beside the
+// others): 512 products at a time,
 // a segment a lane, added in order to the bit by the rule of chain_sum.cuh.
 // Slices and chains are dealt to warps at preparation time, longest first.  No waits: nothing here can stall on
 // another warp.
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
-#include <mutex>
 #include <queue>
 #include <vector>
 
@@ -59,6 +58,7 @@ constexpr int kSliceGridPerSm = 3;  // sliced-row CTAs per SM beside chains
 constexpr int kChainGroup = 512;  // chain: elements a warp sums at a time, 16 a lane
 constexpr int kChainTurn = 4;     // chain: a last group of so few segments of 16 is added in turn
 constexpr int kMmCols = 4;        // columns a warp of the SpMM kernels serves
+constexpr int kMmWarps = 2, kMmCtas = 10;  // sliced-row SpMM: warps a CTA (small ones fit beside the chains), CTAs an SM
 constexpr int kMmAhead = 2;       // steps a lane of the sliced-row SpMM loads at a time
 constexpr uint32_t kChain = 1u;   // dc_slice::geo: a one-row chain
 constexpr int kMidShift = 20;     // dc_slice::geo: matrix index of a batch
@@ -137,22 +137,24 @@ struct dc_args {
     void* y;
     int64_t ldx, ldy;        // SpMM: x[i * ldx + column], y[i * ldy + column]
     int cols;                // SpMM: columns
-    int fresh;               // SpMV: y = A x (y starts from zero); 2: launched while the kernel before it ends
-    const int* skip;         // ... nothing is done where *skip is set
+    int fresh;               // SpMV: y = A x (y starts from zero)
+    int wait;                // waits for the kernel before it at its start
+    const int* skip;         // nothing is done where *skip is set
     const dc_mat* mats;      // a batch (B = true): matrix i's arrays, x and y
     const void* const* xs;
     void* const* ys;
 };
 
-// A fresh launch (spmv_set_y) waits for the kernel before it, then lets the next
-// one be launched; true where there is nothing to do.  (x, which the kernel
-// before wrote, is read by plain loads: the read-only path promises nothing
+// The start of an SpMV kernel: lets the next kernel start -- after the kernel
+// before is complete, for the first kernel of a product that was queued while
+// that one ran (spmv_set_y).  True where there is nothing to do.  (x, which that
+// kernel wrote, is read by plain loads: the read-only path promises nothing
 // about data written during the kernel's life.)
-__device__ __forceinline__ bool begin_fresh(const dc_args& P)
+__device__ __forceinline__ bool begin(const dc_args& P)
 {
-    if (!P.fresh)
-        return false;
-    asm volatile("griddepcontrol.wait;\ngriddepcontrol.launch_dependents;" ::: "memory");
+    if (P.wait)
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+    beside_begin();
     return P.skip && *reinterpret_cast<const volatile int*>(P.skip) != 0;
 }
 
@@ -216,12 +218,15 @@ __global__ void __launch_bounds__(32 * kWarpsPerCta, kCtasPerSm) k_spmv_slices(d
     constexpr int U = VT == ABHSF_VALUE_F64 ? kUnroll : 2 * kUnroll;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int gw = blockIdx.x * kWarpsPerCta + warp;
-    if (begin_fresh(P) || gw >= P.warps)
+    const bool nothing = begin(P);
+    if (gw >= P.warps)
         return;
     int64_t si = P.wbeg[gw];
     const int64_t s1 = P.wbeg[gw + 1];
-    if (si >= s1)
+    if (nothing || si >= s1) {
+        beside_end();
         return;
+    }
     auto mat = [&](const dc_slice& q) -> const dc_mat& { return B ? P.mats[q.geo >> kMidShift] : P.A; };
     auto record = [&](const dc_slice& q) -> uint32_t {
         return lane < (int)q.lanes ? mat(q).lane[q.meta + lane] : 0u;
@@ -286,6 +291,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerCta, kCtasPerSm) k_spmv_slices(d
         nx = nn;
         rec = rec_n;
     }
+    beside_end();
 }
 
 // Asynchronous 4- or 8-byte copy of one element to shared memory.
@@ -353,7 +359,7 @@ __device__ __forceinline__ void chain_at(const dc_args& P, const dc_slice& sl, c
 // Bound by latency: one warp issues 408 instructions a group, 4.8 cycles each
 // (a lone row of 98,304 ones 0.49 -> 0.20 ms, of N(0,1) products 0.49 -> 0.37,
 // against additions in turn).  R-MAT scale 22 (chains and sliced rows
-// together) 0.574 -> 0.368 ms, the 256-matrix batch 0.861 -> 0.787 ms.  Two
+// together) 0.574 -> 0.357 ms, the 256-matrix batch 0.861 -> 0.790 ms.  Two
 // CTAs an SM, or the sliced rows two, were slower on the batch (0.87 ms).
 template <int S, int VT, bool B>
 __global__ void __launch_bounds__(32 * kChainWarps, kChainCtasPerSm) k_spmv_chains(dc_args P)
@@ -367,15 +373,18 @@ __global__ void __launch_bounds__(32 * kChainWarps, kChainCtasPerSm) k_spmv_chai
     extern __shared__ __align__(16) uint8_t chain_smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int gw = blockIdx.x * kChainWarps + warp;
-    if (begin_fresh(P) || gw >= P.warps)
+    const bool nothing = begin(P);
+    if (gw >= P.warps)
         return;
     T* xb = reinterpret_cast<T*>(chain_smem + warp * chain_smem_warp<T, V>());
     V* vb = reinterpret_cast<V*>(xb + 2 * 32 * STX);
     const int64_t s1 = P.wbeg[gw + 1];
     chain_pos<T, V> cur{}, nxt{}, ahead;  // summed; copied; its words loaded
     ahead.si = P.wbeg[gw];
-    if (ahead.si >= s1)
+    if (nothing || ahead.si >= s1) {
+        beside_end();
         return;
+    }
     chain_at<S, B>(P, P.slices[ahead.si], ahead);
     dc_slice after = ahead.si + 1 < s1 ? P.slices[ahead.si + 1] : P.slices[ahead.si];
     uint32_t w[L];
@@ -490,6 +499,7 @@ __global__ void __launch_bounds__(32 * kChainWarps, kChainCtasPerSm) k_spmv_chai
         half ^= 1;
     }
     asm volatile("cp.async.wait_all;\n" ::: "memory");
+    beside_end();
 }
 
 // Y += A X over k > 1 columns (FP64), kMmCols = 4 of them a warp (blockIdx.x
@@ -504,14 +514,15 @@ __global__ void __launch_bounds__(32 * kChainWarps, kChainCtasPerSm) k_spmv_chai
 // Bound by the latency of the gathers (eight a lane in flight); one launch
 // whatever k is.  R-MAT scale 18, 7 columns: passes of 4, 2 and 1 columns, each
 // with up to four gathers a lane in flight and column and value by shuffles,
-// took 415 us of kernel time, this 77 us (with the chains: 1,305 -> 113 us).
+// took 415 us of kernel time, this 78 us (with the chains: 1,305 -> 98 us).
 template <int S>
-__global__ void __launch_bounds__(32 * kWarpsPerCta, 2) k_spmm_slices(dc_args P)
+__global__ void __launch_bounds__(32 * kMmWarps, kMmCtas) k_spmm_slices(dc_args P)
 {
     constexpr int R = kMmCols, U = kMmAhead;  // rows a lane (32 rows x 4 columns over 32 lanes); steps a round
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane / kMmCols, h = blockIdx.x * kMmCols + lane % kMmCols;
-    const int gw = blockIdx.y * kWarpsPerCta + warp;
+    const int gw = blockIdx.y * kMmWarps + warp;
+    beside_begin();
     if (gw >= P.warps || h >= P.cols)
         return;
     const double* X = static_cast<const double*>(P.x) + h;
@@ -570,6 +581,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerCta, 2) k_spmm_slices(dc_args P)
             if (len[i])
                 *y[i] = acc[i];
     }
+    beside_end();
 }
 
 // Y += A X over k > 1 columns, the chains: one row and kMmCols = 4 columns a
@@ -580,7 +592,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerCta, 2) k_spmm_slices(dc_args P)
 // that the 16 gathers of X a lane has in flight are one sector each for the
 // quad.  Where sum_group gives up, the segments are added one after another.
 // R-MAT scale 18, 7 columns: three passes with eight gathers in flight a warp
-// step took 1,236 us of kernel time, this 92 us.
+// step took 1,236 us of kernel time, this 88 us.
 template <int S>
 __global__ void __launch_bounds__(32 * kChainWarps, kChainCtasPerSm) k_spmm_chains(dc_args P)
 {
@@ -589,6 +601,7 @@ __global__ void __launch_bounds__(32 * kChainWarps, kChainCtasPerSm) k_spmm_chai
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane / kMmCols, q = lane % kMmCols, h = blockIdx.x * kMmCols + q;
     const int gw = blockIdx.y * kChainWarps + warp;
+    beside_begin();
     if (gw >= P.warps)
         return;
     const bool live = h < P.cols;  // the last columns' warps may hold fewer than four
@@ -643,6 +656,7 @@ __global__ void __launch_bounds__(32 * kChainWarps, kChainCtasPerSm) k_spmm_chai
         if (g == 0 && live)
             *y = run;
     }
+    beside_end();
 }
 
 // --------------------------------------------------------------- preparation
@@ -909,22 +923,6 @@ int stream_grid_warps(int64_t items, bool chains, bool beside_chains, bool besid
     return (int)std::max<int64_t>(1, std::min<int64_t>(full, items));
 }
 
-// The side stream and the fork / join events of a handle with chains.
-void make_side(cudaStream_t& side, cudaEvent_t& fork, cudaEvent_t& join)
-{
-    if (!side) {
-        // the highest priority: the chains' CTAs are placed before the others
-        // when both wait for SMs (the longest chain bounds the launch)
-        int least = 0, greatest = 0;
-        ABHSF_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
-        ABHSF_CUDA(cudaStreamCreateWithPriority(&side, cudaStreamNonBlocking, greatest));
-    }
-    if (!fork)
-        ABHSF_CUDA(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
-    if (!join)
-        ABHSF_CUDA(cudaEventCreateWithFlags(&join, cudaEventDisableTiming));
-}
-
 // Time a slice takes, for the deal: a sliced one walks its longest row, a
 // chain takes about 2,400 cycles a group while its sum is near zero (where
 // groups are added in turn more often) and 1,700 later, and its first loads.
@@ -1031,7 +1029,7 @@ void prepare_stream(abhsf_matrix& a, float avg, cudaStream_t st)
     a.dc_host.clear();
     a.dc_tree_flag.assign((size_t)a.tree_nrows, 0);
     a.dc_warps = a.dc_cwarps = 0;
-    a.dc_beside_ring = a.dc_every_row = false;
+    a.dc_every_row = false;
     a.dc_elements = a.dc_rows = a.dc_slots = a.dc_lane_records = 0;
     const int s = a.s, lg = a.lg;
     if (avg <= 0.f || a.tree_nrows == 0 || a.sum_order != ABHSF_SUM_REFERENCE || (uint64_t)a.n > (uint64_t(1) << 32))
@@ -1272,8 +1270,6 @@ void prepare_stream(abhsf_matrix& a, float avg, cudaStream_t st)
     a.dc_lane_records = 32 * nslices;
     deal_slices({&a}, a.dc_sched, a.dc_wbeg, a.dc_warps, st, 0, INT64_MAX, kDealSliced);
     deal_slices({&a}, a.dc_csched, a.dc_cwbeg, a.dc_cwarps, st, 0, INT64_MAX, kDealChains);
-    if (a.dc_cwarps)
-        make_side(a.dc_side, a.dc_fork, a.dc_join);
 }
 
 namespace {
@@ -1302,61 +1298,44 @@ void same_carveout(int smem = 0)
     done.fetch_or(bit, std::memory_order_relaxed);
 }
 
-// A fresh launch of sliced rows only is queued while the kernel before it ends
-// (it waits for it on the device); beside chains the events order it.
-void launch_maybe_after(void (*kern)(dc_args), unsigned grid, int threads, int smem, const dc_args& P, cudaStream_t st)
-{
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3((unsigned)threads);
-    cfg.dynamicSmemBytes = (size_t)smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = P.fresh == 2 ? 1 : 0;
-    ABHSF_CUDA(cudaLaunchKernelEx(&cfg, kern, P));
-}
-
 template <int S, int VT, bool B>
-void launch_kind(bool chains, const dc_args& P, cudaStream_t st)
+void launch_kind(beside& bs, bool chains, const dc_args& P, cudaStream_t st)
 {
     if (chains) {
         constexpr int smem = kChainWarps * chain_smem_warp<typename vt_of<VT>::T, typename vt_of<VT>::V>();
         same_carveout<k_spmv_chains<S, VT, B>>(smem);
         const unsigned grid = (unsigned)((P.warps + kChainWarps - 1) / kChainWarps);
-        launch_maybe_after(k_spmv_chains<S, VT, B>, grid, 32 * kChainWarps, smem, P, st);
+        launch_beside(bs, k_spmv_chains<S, VT, B>, grid, 32 * kChainWarps, smem, st, P);
     } else {
         same_carveout<k_spmv_slices<S, VT, B>>();
         const unsigned grid = (unsigned)((P.warps + kWarpsPerCta - 1) / kWarpsPerCta);
-        launch_maybe_after(k_spmv_slices<S, VT, B>, grid, 32 * kWarpsPerCta, 0, P, st);
+        launch_beside(bs, k_spmv_slices<S, VT, B>, grid, 32 * kWarpsPerCta, 0, st, P);
     }
 }
 
 template <int VT, bool B>
-void launch_vt(int s, bool chains, const dc_args& P, cudaStream_t st)
+void launch_vt(beside& bs, int s, bool chains, const dc_args& P, cudaStream_t st)
 {
     switch (s) {
-    case 16: launch_kind<16, VT, B>(chains, P, st); break;
-    case 32: launch_kind<32, VT, B>(chains, P, st); break;
-    case 64: launch_kind<64, VT, B>(chains, P, st); break;
-    case 128: launch_kind<128, VT, B>(chains, P, st); break;
-    default: launch_kind<256, VT, B>(chains, P, st); break;
+    case 16: launch_kind<16, VT, B>(bs, chains, P, st); break;
+    case 32: launch_kind<32, VT, B>(bs, chains, P, st); break;
+    case 64: launch_kind<64, VT, B>(bs, chains, P, st); break;
+    case 128: launch_kind<128, VT, B>(bs, chains, P, st); break;
+    default: launch_kind<256, VT, B>(bs, chains, P, st); break;
     }
 }
 
-void launch(int s, int vt, bool batch, bool chains, const dc_args& P, cudaStream_t st)
+void launch(beside& bs, int s, int vt, bool batch, bool chains, const dc_args& P, cudaStream_t st)
 {
     if (P.warps == 0)
         return;
     if (vt == ABHSF_VALUE_F64)
-        batch ? launch_vt<ABHSF_VALUE_F64, true>(s, chains, P, st) : launch_vt<ABHSF_VALUE_F64, false>(s, chains, P, st);
+        batch ? launch_vt<ABHSF_VALUE_F64, true>(bs, s, chains, P, st) : launch_vt<ABHSF_VALUE_F64, false>(bs, s, chains, P, st);
     else if (vt == ABHSF_VALUE_F32)
-        batch ? launch_vt<ABHSF_VALUE_F32, true>(s, chains, P, st) : launch_vt<ABHSF_VALUE_F32, false>(s, chains, P, st);
+        batch ? launch_vt<ABHSF_VALUE_F32, true>(bs, s, chains, P, st) : launch_vt<ABHSF_VALUE_F32, false>(bs, s, chains, P, st);
     else
-        batch ? launch_vt<ABHSF_VALUE_BF16, true>(s, chains, P, st)
-              : launch_vt<ABHSF_VALUE_BF16, false>(s, chains, P, st);
+        batch ? launch_vt<ABHSF_VALUE_BF16, true>(bs, s, chains, P, st)
+              : launch_vt<ABHSF_VALUE_BF16, false>(bs, s, chains, P, st);
 }
 
 dc_mat mat_of(const abhsf_matrix& a) { return dc_mat{a.dc_words.get(), a.dc_vals.get(), a.dc_lane.get(), a.m}; }
@@ -1395,50 +1374,33 @@ dc_args batch_args(const abhsf_batch& b, const uint8_t* sched, const int64_t* wb
 // Column groups first in the grid: the groups of one slice run side by side
 // and share its words and values in L2.
 template <int S>
-void launch_mm(bool chains, const dc_args& P, cudaStream_t st)
+void launch_mm(beside& bs, bool chains, const dc_args& P, cudaStream_t st)
 {
     same_carveout<k_spmm_chains<S>>();
     same_carveout<k_spmm_slices<S>>();
     const unsigned groups = (unsigned)((P.cols + kMmCols - 1) / kMmCols);
-    const int per = chains ? kChainWarps : kWarpsPerCta;
+    const int per = chains ? kChainWarps : kMmWarps;
     const dim3 grid(groups, (unsigned)((P.warps + per - 1) / per));
-    if (chains)
-        k_spmm_chains<S><<<grid, 32 * kChainWarps, 0, st>>>(P);
-    else
-        k_spmm_slices<S><<<grid, 32 * kWarpsPerCta, 0, st>>>(P);
-    ABHSF_CUDA(cudaGetLastError());
+    launch_beside(bs, chains ? k_spmm_chains<S> : k_spmm_slices<S>, grid, 32u * per, 0, st, P);
 }
 
 // P.cols columns: the SpMV kernels for one, the SpMM ones (FP64) for more and
 // for one that is a column of a wider X or Y.
-void launch_cols(int s, int vt, bool chains, const dc_args& P, cudaStream_t st)
+void launch_cols(beside& bs, int s, int vt, bool chains, const dc_args& P, cudaStream_t st)
 {
     if (P.warps == 0)
         return;
     if (P.cols == 1 && P.ldx == 1 && P.ldy == 1) {
-        launch(s, vt, false, chains, P, st);
+        launch(bs, s, vt, false, chains, P, st);
         return;
     }
     switch (s) {
-    case 16: launch_mm<16>(chains, P, st); break;
-    case 32: launch_mm<32>(chains, P, st); break;
-    case 64: launch_mm<64>(chains, P, st); break;
-    case 128: launch_mm<128>(chains, P, st); break;
-    default: launch_mm<256>(chains, P, st); break;
+    case 16: launch_mm<16>(bs, chains, P, st); break;
+    case 32: launch_mm<32>(bs, chains, P, st); break;
+    case 64: launch_mm<64>(bs, chains, P, st); break;
+    case 128: launch_mm<128>(bs, chains, P, st); break;
+    default: launch_mm<256>(bs, chains, P, st); break;
     }
-}
-
-// Chains on the side stream, after everything queued on st so far.
-void fork_chains(cudaStream_t st, cudaStream_t side, cudaEvent_t fork, cudaEvent_t join, int s, int vt, bool batch,
-                 const dc_args& P)
-{
-    ABHSF_CUDA(cudaEventRecord(fork, st));
-    ABHSF_CUDA(cudaStreamWaitEvent(side, fork, 0));
-    if (batch)
-        launch(s, vt, batch, true, P, side);
-    else
-        launch_cols(s, vt, true, P, side);
-    ABHSF_CUDA(cudaEventRecord(join, side));
 }
 
 }  // namespace
@@ -1455,73 +1417,48 @@ dc_plan plan_of(const abhsf_matrix& a)
     return p;
 }
 
-// Whether this launch runs the sliced rows on the side stream, beside the ring
-// kernel queued on st after slices_begin (single right-hand sides only).
-inline bool sliced_beside(const abhsf_matrix& a, const dc_plan& p, int cols)
+void slices_begin(beside& bs, const abhsf_matrix& a, const dc_plan& p, const void* x, int64_t ldx, void* y,
+                  int64_t ldy, cudaStream_t st, int cols)
 {
-    return a.dc_beside_ring && cols == 1 && p.warps > 0 && p.sched == a.dc_sched.get();
-}
-
-void slices_begin(const abhsf_matrix& a, const dc_plan& p, const void* x, int64_t ldx, void* y, int64_t ldy,
-                  cudaStream_t st, int cols)
-{
-    const bool beside = sliced_beside(a, p, cols);
-    if (p.cwarps == 0 && !beside)
-        return;
-    if (!a.dc_side)
-        fail(ABHSF_ERROR_CUDA, "matrix has chains but no side stream");
-    ABHSF_CUDA(cudaEventRecord(a.dc_fork, st));
-    ABHSF_CUDA(cudaStreamWaitEvent(a.dc_side, a.dc_fork, 0));
-    if (beside)  // first, so that its CTAs take their place before the ring's fill the SMs
-        launch(a.s, a.value_type, false, false, args_of(a, p.sched, p.wbeg, p.warps, x, ldx, y, ldy, 1), a.dc_side);
     if (p.cwarps)
-        launch_cols(a.s, a.value_type, true, args_of(a, p.csched, p.cwbeg, p.cwarps, x, ldx, y, ldy, cols),
-                    a.dc_side);
-    ABHSF_CUDA(cudaEventRecord(a.dc_join, a.dc_side));
+        launch_cols(bs, a.s, a.value_type, true, args_of(a, p.csched, p.cwbeg, p.cwarps, x, ldx, y, ldy, cols), st);
 }
 
-void slices_end(const abhsf_matrix& a, const dc_plan& p, const void* x, int64_t ldx, void* y, int64_t ldy,
+void slices_end(beside& bs, const abhsf_matrix& a, const dc_plan& p, const void* x, int64_t ldx, void* y, int64_t ldy,
                 cudaStream_t st, int cols)
 {
-    const bool beside = sliced_beside(a, p, cols);
-    if (p.warps && !beside)
-        launch_cols(a.s, a.value_type, false, args_of(a, p.sched, p.wbeg, p.warps, x, ldx, y, ldy, cols), st);
-    if (p.cwarps || beside)
-        ABHSF_CUDA(cudaStreamWaitEvent(st, a.dc_join, 0));
+    if (p.warps)
+        launch_cols(bs, a.s, a.value_type, false, args_of(a, p.sched, p.wbeg, p.warps, x, ldx, y, ldy, cols), st);
 }
 
 bool spmv_sets_y(const abhsf_matrix& a) { return a.dc_every_row; }
 
 void spmv_set_y(const abhsf_matrix& a, const void* x, void* y, const int* skip, cudaStream_t st)
 {
-    std::lock_guard<std::mutex> lock(a.dc_mu);
-    auto args = [&](const dbuf<uint8_t>& sched, const dbuf<int64_t>& wbeg, int warps) {
+    beside bs;
+    bs.any = true;  // its first kernel is queued while the kernel before runs, and waits for it at its start
+    auto args = [&](const dbuf<uint8_t>& sched, const dbuf<int64_t>& wbeg, int warps, bool wait) {
         dc_args P = args_of(a, sched.get(), wbeg.get(), warps, x, 1, y, 1, 1);
-        P.fresh = a.dc_cwarps ? 1 : 2;
+        P.fresh = 1;
+        P.wait = wait;
         P.skip = skip;
         return P;
     };
-    if (a.dc_cwarps) {
-        ABHSF_CUDA(cudaEventRecord(a.dc_fork, st));
-        ABHSF_CUDA(cudaStreamWaitEvent(a.dc_side, a.dc_fork, 0));
-        launch(a.s, a.value_type, false, true, args(a.dc_csched, a.dc_cwbeg, a.dc_cwarps), a.dc_side);
-        ABHSF_CUDA(cudaEventRecord(a.dc_join, a.dc_side));
-    }
-    if (a.dc_warps)
-        launch(a.s, a.value_type, false, false, args(a.dc_sched, a.dc_wbeg, a.dc_warps), st);
     if (a.dc_cwarps)
-        ABHSF_CUDA(cudaStreamWaitEvent(st, a.dc_join, 0));
+        launch(bs, a.s, a.value_type, false, true, args(a.dc_csched, a.dc_cwbeg, a.dc_cwarps, true), st);
+    if (a.dc_warps)
+        launch(bs, a.s, a.value_type, false, false, args(a.dc_sched, a.dc_wbeg, a.dc_warps, a.dc_cwarps == 0), st);
 }
 
 // The ring kernel serves some block rows: the sliced rows go beside it, dealt
-// over one CTA an SM.
+// over one CTA an SM, for which the ring leaves registers and warps (they need no
+// shared memory).  The ring is queued first: behind the sliced rows it began 5 us
+// later (tiled mixture 104.4 against 109.2 us, f32 73.2 against 76.9).
 void slices_beside_ring(abhsf_matrix& a, cudaStream_t st)
 {
     if (a.dc_warps == 0)
         return;
     deal_slices({&a}, a.dc_sched, a.dc_wbeg, a.dc_warps, st, 0, INT64_MAX, kDealSliced, true);
-    make_side(a.dc_side, a.dc_fork, a.dc_join);
-    a.dc_beside_ring = true;
 }
 
 // The slices of every matrix of a batch in one launch (and its chains in one more).
@@ -1540,24 +1477,20 @@ void prepare_batch_stream(abhsf_batch& b, cudaStream_t st)
     ABHSF_CUDA(cudaMemcpyAsync(b.dc_table.get(), t.data(), t.size() * sizeof(dc_mat), cudaMemcpyHostToDevice, st));
     deal_slices(b.mats, b.dc_sched, b.dc_wbeg, b.dc_warps, st, 0, INT64_MAX, kDealSliced);
     deal_slices(b.mats, b.dc_csched, b.dc_cwbeg, b.dc_cwarps, st, 0, INT64_MAX, kDealChains);
-    if (b.dc_cwarps)
-        make_side(b.dc_side, b.dc_fork, b.dc_join);
 }
 
-void batch_stream_begin(const abhsf_batch& b, const double* const* xs, double* const* ys, cudaStream_t st)
+void batch_stream_begin(beside& bs, const abhsf_batch& b, const double* const* xs, double* const* ys, cudaStream_t st)
 {
     if (b.dc_cwarps)
-        fork_chains(st, b.dc_side, b.dc_fork, b.dc_join, b.s, ABHSF_VALUE_F64, true,
-                    batch_args(b, b.dc_csched.get(), b.dc_cwbeg.get(), b.dc_cwarps, xs, ys));
+        launch(bs, b.s, ABHSF_VALUE_F64, true, true,
+               batch_args(b, b.dc_csched.get(), b.dc_cwbeg.get(), b.dc_cwarps, xs, ys), st);
 }
 
-void batch_stream_end(const abhsf_batch& b, const double* const* xs, double* const* ys, cudaStream_t st)
+void batch_stream_end(beside& bs, const abhsf_batch& b, const double* const* xs, double* const* ys, cudaStream_t st)
 {
     if (b.dc_warps)
-        launch(b.s, ABHSF_VALUE_F64, true, false, batch_args(b, b.dc_sched.get(), b.dc_wbeg.get(), b.dc_warps, xs, ys),
-               st);
-    if (b.dc_cwarps)
-        ABHSF_CUDA(cudaStreamWaitEvent(st, b.dc_join, 0));
+        launch(bs, b.s, ABHSF_VALUE_F64, true, false,
+               batch_args(b, b.dc_sched.get(), b.dc_wbeg.get(), b.dc_warps, xs, ys), st);
 }
 
 }  // namespace abhsf
