@@ -164,10 +164,18 @@ __global__ void __launch_bounds__(kRedThreads) k_cg_residual(int64_t n, T* r, T*
                                                              const double* pap_part, double* partial)
 {
     wait_and_next();
-    if (st->done[cur])
-        return;
     constexpr int N = pack<T>::N;
     __shared__ double step;
+    const int64_t tid = blockIdx.x * (int64_t)kRedThreads + threadIdx.x;
+    const int64_t nv = VEC ? n / N : 0;
+    // the first packs are on their way while the partial sums are added up
+    pack<T> nr{}, na{};
+    if (tid < nv) {
+        nr = ld_pack(r + tid * N);
+        na = ld_pack(ap + tid * N);
+    }
+    if (st->done[cur])
+        return;
     const double pap = sum_partials(pap_part);
     if (threadIdx.x == 0) {
         const bool go = pap > 0.0;  // else breakdown: p = 0 or A not positive definite on p
@@ -179,12 +187,14 @@ __global__ void __launch_bounds__(kRedThreads) k_cg_residual(int64_t n, T* r, T*
     }
     __syncthreads();
     const T alpha = (T)step;
-    const int64_t tid = blockIdx.x * (int64_t)kRedThreads + threadIdx.x;
-    const int64_t nv = VEC ? n / N : 0;
     double s = 0.0;
     for (int64_t i = tid; i < nv; i += kStride) {
-        pack<T> vr = ld_pack(r + i * N);
-        const pack<T> va = ld_pack(ap + i * N);
+        pack<T> vr = nr;
+        const pack<T> va = na;
+        if (i + kStride < nv) {
+            nr = ld_pack(r + (i + kStride) * N);
+            na = ld_pack(ap + (i + kStride) * N);
+        }
         pack<T> zero;
 #pragma unroll
         for (int k = 0; k < N; ++k) {
@@ -216,7 +226,16 @@ __global__ void __launch_bounds__(kRedThreads) k_cg_direction(int64_t n, T* x, T
                                                               const double* rr_part)
 {
     wait_and_next();
+    constexpr int N = pack<T>::N;
     const int nxt = cur ^ 1;
+    const int64_t tid = blockIdx.x * (int64_t)kRedThreads + threadIdx.x;
+    const int64_t nv = VEC ? n / N : 0;
+    pack<T> nx{}, np{}, nr{};  // the next pack of each vector
+    if (tid < nv) {
+        nx = ld_pack(x + tid * N);
+        np = ld_pack(p + tid * N);
+        nr = ld_pack(r + tid * N);
+    }
     if (st->done[cur]) {
         if (blockIdx.x == 0 && threadIdx.x == 0) {
             st->rr[nxt] = st->rr[cur];
@@ -224,7 +243,6 @@ __global__ void __launch_bounds__(kRedThreads) k_cg_direction(int64_t n, T* x, T
         }
         return;
     }
-    constexpr int N = pack<T>::N;
     __shared__ double grow;
     const bool active = st->active != 0;
     const T alpha = (T)st->alpha;
@@ -245,11 +263,15 @@ __global__ void __launch_bounds__(kRedThreads) k_cg_direction(int64_t n, T* x, T
     }
     __syncthreads();
     const T beta = (T)grow;
-    const int64_t tid = blockIdx.x * (int64_t)kRedThreads + threadIdx.x;
-    const int64_t nv = VEC ? n / N : 0;
     for (int64_t i = tid; i < nv; i += kStride) {
-        pack<T> vx = ld_pack(x + i * N), vp = ld_pack(p + i * N);
-        const pack<T> vr = ld_pack(r + i * N);
+        pack<T> vx = nx, vp = np;
+        const pack<T> vr = nr;
+        const int64_t j = i + kStride;
+        if (j < nv) {
+            nx = ld_pack(x + j * N);
+            np = ld_pack(p + j * N);
+            nr = ld_pack(r + j * N);
+        }
 #pragma unroll
         for (int k = 0; k < N; ++k) {
             vx.v[k] += alpha * vp.v[k];
