@@ -193,6 +193,11 @@ struct abhsf_matrix {
     // reference-order SpMV, s = 32 / 64: every CTA's tile descriptors and their ranges
     abhsf::dbuf<uint8_t> ring_desc;
     abhsf::dbuf<int64_t> ring_wbeg;
+    // a small matrix: a schedule of every block row, the slices' among them, so
+    // that one launch serves an SpMV
+    abhsf::dbuf<uint8_t> solo_desc;
+    abhsf::dbuf<int64_t> solo_wbeg;
+    int solo_ctas = 0;
     int ring_max_pv = 0;  // largest payload + values bytes of one tile (picks the SpMM pass width)
     int ring_warps = 0;  // CTAs of the ring kernel; 0: the streaming kernel serves this matrix
     int ring_layout = 0;  // consumer layout of its single-right-hand-side launches (timed at build)
