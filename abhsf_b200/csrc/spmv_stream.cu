@@ -215,81 +215,82 @@ __global__ void __launch_bounds__(32 * kWarpsPerCta, kCtasPerSm) k_spmv_slices(d
     using T = typename vt_of<VT>::T;
     using V = typename vt_of<VT>::V;
     // f32 / bf16 values leave room in 64 registers for twice the steps in flight
-    constexpr int U = VT == ABHSF_VALUE_F64 ? kUnroll : 2 * kUnroll;
+    // (bf16 one fewer: 213 us against 241 on the 3D Laplacian 256^3, 227 with 4;
+    // rows of 21 or of power-law lengths the same)
+    constexpr int U = VT == ABHSF_VALUE_F64 ? kUnroll : VT == ABHSF_VALUE_BF16 ? 2 * kUnroll - 1 : 2 * kUnroll;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int gw = blockIdx.x * kWarpsPerCta + warp;
     const bool nothing = begin(P);
     if (gw >= P.warps)
         return;
     int64_t si = P.wbeg[gw];
-    const int64_t s1 = P.wbeg[gw + 1];
-    if (nothing || si >= s1) {
-        beside_end();
-        return;
-    }
-    auto mat = [&](const dc_slice& q) -> const dc_mat& { return B ? P.mats[q.geo >> kMidShift] : P.A; };
-    auto record = [&](const dc_slice& q) -> uint32_t {
-        return lane < (int)q.lanes ? mat(q).lane[q.meta + lane] : 0u;
-    };
-    dc_slice sl = P.slices[si];
-    dc_slice nx = si + 1 < s1 ? P.slices[si + 1] : sl;
-    uint32_t rec = record(sl);
+    const int64_t s1 = nothing ? si : P.wbeg[gw + 1];
+    // (one way out: with a second return here the loop took 4% longer in FP64)
+    if (si < s1) {
+        auto mat = [&](const dc_slice& q) -> const dc_mat& { return B ? P.mats[q.geo >> kMidShift] : P.A; };
+        auto record = [&](const dc_slice& q) -> uint32_t {
+            return lane < (int)q.lanes ? mat(q).lane[q.meta + lane] : 0u;
+        };
+        dc_slice sl = P.slices[si];
+        dc_slice nx = si + 1 < s1 ? P.slices[si + 1] : sl;
+        uint32_t rec = record(sl);
 #pragma unroll 1
-    for (; si < s1; ++si) {
-        const bool more = si + 1 < s1;
-        const dc_slice nn = si + 2 < s1 ? P.slices[si + 2] : nx;
-        const uint32_t rec_n = more ? record(nx) : 0u;
-        const int mid = (int)(sl.geo >> kMidShift);
-        const dc_mat& M = mat(sl);
-        const T* X = static_cast<const T*>(B ? P.xs[mid] : P.x);
-        T* Y = static_cast<T*>(B ? P.ys[mid] : P.y);
-        const uint32_t* W = M.words + sl.base + lane;
-        const V* Vv = static_cast<const V*>(M.vals) + sl.base + lane;
-        // one row per lane, element k of the lane's row at slot 32 k + lane
-        const int len = lane < (int)sl.lanes ? (int)(rec & kLenMask) + 1 : 0;
-        const int64_t row = (int64_t)sl.brow * S + (int64_t)(rec >> kLenBits);
-        T acc = len && !P.fresh ? Y[row] : T(0);
-        uint32_t col = 0;
-        // values stay in their stored type until their product: a widening
-        // at the load would wait for the prefetch it belongs to
-        uint32_t w[U];
-        V v[U];
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            w[u] = u < len ? ld_stream(W + 32 * u) : 0u;
-            v[u] = u < len ? ld_stream(Vv + 32 * u) : V(0);
-        }
-#pragma unroll 1
-        for (int k0 = 0; k0 < (int)sl.steps; k0 += U) {
-            uint32_t wn[U];
-            V vn[U];
-            T x[U];
-#pragma unroll
-            for (int u = 0; u < U; ++u) {  // the next step's words and values
-                const int k = k0 + U + u;
-                wn[u] = k < len ? ld_stream(W + 32 * k) : 0u;
-                vn[u] = k < len ? ld_stream(Vv + 32 * k) : V(0);
-            }
+        for (; si < s1; ++si) {
+            const bool more = si + 1 < s1;
+            const dc_slice nn = si + 2 < s1 ? P.slices[si + 2] : nx;
+            const uint32_t rec_n = more ? record(nx) : 0u;
+            const int mid = (int)(sl.geo >> kMidShift);
+            const dc_mat& M = mat(sl);
+            const T* X = static_cast<const T*>(B ? P.xs[mid] : P.x);
+            T* Y = static_cast<T*>(B ? P.ys[mid] : P.y);
+            const uint32_t* W = M.words + sl.base + lane;
+            const V* Vv = static_cast<const V*>(M.vals) + sl.base + lane;
+            // one row per lane, element k of the lane's row at slot 32 k + lane
+            const int len = lane < (int)sl.lanes ? (int)(rec & kLenMask) + 1 : 0;
+            const int64_t row = (int64_t)sl.brow * S + (int64_t)(rec >> kLenBits);
+            T acc = len && !P.fresh ? Y[row] : T(0);
+            uint32_t col = 0;
+            // values stay in their stored type until their product: a widening
+            // at the load would wait for the prefetch it belongs to
+            uint32_t w[U];
+            V v[U];
 #pragma unroll
             for (int u = 0; u < U; ++u) {
-                col += w[u];
-                x[u] = k0 + u < len ? X[col] : T(0);
+                w[u] = u < len ? ld_stream(W + 32 * u) : 0u;
+                v[u] = u < len ? ld_stream(Vv + 32 * u) : V(0);
             }
+#pragma unroll 1
+            for (int k0 = 0; k0 < (int)sl.steps; k0 += U) {
+                uint32_t wn[U];
+                V vn[U];
+                T x[U];
 #pragma unroll
-            for (int u = 0; u < U; ++u)
-                if (k0 + u < len)
-                    acc = dadd(acc, dmul(wide(v[u]), x[u]));
+                for (int u = 0; u < U; ++u) {  // the next step's words and values
+                    const int k = k0 + U + u;
+                    wn[u] = k < len ? ld_stream(W + 32 * k) : 0u;
+                    vn[u] = k < len ? ld_stream(Vv + 32 * k) : V(0);
+                }
 #pragma unroll
-            for (int u = 0; u < U; ++u) {
-                w[u] = wn[u];
-                v[u] = vn[u];
+                for (int u = 0; u < U; ++u) {
+                    col += w[u];
+                    x[u] = k0 + u < len ? X[col] : T(0);
+                }
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                    if (k0 + u < len)
+                        acc = dadd(acc, dmul(wide(v[u]), x[u]));
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    w[u] = wn[u];
+                    v[u] = vn[u];
+                }
             }
+            if (len)
+                Y[row] = acc;
+            sl = nx;
+            nx = nn;
+            rec = rec_n;
         }
-        if (len)
-            Y[row] = acc;
-        sl = nx;
-        nx = nn;
-        rec = rec_n;
     }
     beside_end();
 }

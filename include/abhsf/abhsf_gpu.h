@@ -280,9 +280,8 @@ ABHSF_API abhsf_status abhsf_batch_create(const abhsf_matrix* const* mats, int32
                                           abhsf_batch** out);
 
 /* y_i += A_i x_i for every matrix of the batch in one call: one launch of
- * each kernel the matrices need (the tile kernel, the row-slice kernel, and
- * the chain kernel on a side stream forked from `stream` and joined back;
- * abhsf_batch_kernels), in the reference's summation order (each y_i bitwise
+ * each kernel the matrices need (the tile kernel, the chain kernel and the
+ * row-slice kernel, side by side on `stream`; abhsf_batch_kernels), in the reference's summation order (each y_i bitwise
  * what abhsf_spmv gives).  xs and ys are DEVICE arrays of count device
  * pointers (x_i of n_i doubles, y_i of m_i), so the call can be captured in
  * a CUDA graph.  Calls on one batch must not overlap on the GPU. */
