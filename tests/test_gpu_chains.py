@@ -1,6 +1,6 @@
 """The chains (rows of more than 256 elements, summed by a whole warp): y must
 be bitwise the additions in turn, for sums that cross binades, end in ties,
-overflow or cancel, and at every length around the groups of 256 elements."""
+overflow or cancel, and at lengths around the groups of 512 elements (the SpMM: 128)."""
 import numpy as np
 import pytest
 
