@@ -53,8 +53,8 @@ void autotune(const int64_t* rows, const int64_t* cols, const double* vals, int6
         fail(ABHSF_ERROR_INVALID_VALUE, "rows and cols must be non-NULL");
     abhsf_build_opts o = o_in;
     // host inputs cross to the device once for all candidate builds
-    dbuf<int64_t> r_d, c_d;
-    dbuf<double> v_d;
+    scratch<int64_t> r_d(st), c_d(st);
+    scratch<double> v_d(st);
     if (!o.inputs_on_device && nnz > 0) {
         r_d.alloc(nnz);
         c_d.alloc(nnz);
@@ -71,7 +71,7 @@ void autotune(const int64_t* rows, const int64_t* cols, const double* vals, int6
     o.inputs_on_device = 1;
     const bool f64 = o.value_type == ABHSF_VALUE_F64;
     // x = 0, y = 0: the kernels' speed does not depend on the values
-    dbuf<uint8_t> x((size_t)n * 8 + 16), y((size_t)m * 8 + 16);
+    scratch<uint8_t> x((size_t)n * 8 + 16, st), y((size_t)m * 8 + 16, st);
     ABHSF_CUDA(cudaMemsetAsync(x.get(), 0, (size_t)n * 8 + 16, st));
     ABHSF_CUDA(cudaMemsetAsync(y.get(), 0, (size_t)m * 8 + 16, st));
     event_pair ev;

@@ -398,13 +398,13 @@ void histograms(const int64_t* rows, const int64_t* cols, int64_t nnz, int64_t m
     const int end_bit = shift + bit_length(NI * NJ - 1);
     // counters: the histograms, then the number of tiles of more than kFew
     // elements, the number of tiles, the error bits
-    dbuf<unsigned long long> dh(sz.total + 3);
+    scratch<unsigned long long> dh(sz.total + 3, st);
     unsigned long long* nmany = dh.get() + sz.total;
     int64_t* tiles = reinterpret_cast<int64_t*>(nmany + 1);
     int* err = reinterpret_cast<int*>(nmany + 2);
-    dbuf<uint64_t> keys(nnz), sorted(nnz);
-    dbuf<int64_t> many(nnz / (kFew + 1) + 1);
-    dbuf<int64_t> rows_d, cols_d;  // host inputs
+    scratch<uint64_t> keys(nnz, st), sorted(nnz, st);
+    scratch<int64_t> many(nnz / (kFew + 1) + 1, st);
+    scratch<int64_t> rows_d(st), cols_d(st);  // host inputs
     if (!on_device) {
         rows_d.alloc(nnz);
         cols_d.alloc(nnz);
@@ -424,7 +424,7 @@ void histograms(const int64_t* rows, const int64_t* cols, int64_t nnz, int64_t m
     ABHSF_CUDA(cub::DeviceRadixSort::SortKeys(nullptr, b1, keys.get(), sorted.get(), nnz, shift,
                                               std::max(end_bit, shift + 1), st));
     ABHSF_CUDA(cub::DeviceSelect::If(nullptr, b2, all, start, tiles, nnz, head, st));
-    dbuf<uint8_t> tmp(std::max(b1, b2));
+    scratch<uint8_t> tmp(std::max(b1, b2), st);
     ABHSF_CUDA(cub::DeviceRadixSort::SortKeys(tmp.get(), b1, keys.get(), sorted.get(), nnz, shift,
                                               std::max(end_bit, shift + 1), st));
     ABHSF_CUDA(cub::DeviceSelect::If(tmp.get(), b2, all, start, tiles, nnz, head, st));

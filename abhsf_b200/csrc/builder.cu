@@ -380,13 +380,14 @@ T read_scalar(const T* dptr, cudaStream_t st)
 
 // Copies host inputs to the device (or wraps device inputs).
 struct coo_inputs {
-    dbuf<int64_t> rows_d, cols_d;
-    dbuf<double> vals_d;
+    scratch<int64_t> rows_d, cols_d;
+    scratch<double> vals_d;
     const int64_t* rows = nullptr;
     const int64_t* cols = nullptr;
     const double* vals = nullptr;
 
     coo_inputs(const int64_t* r, const int64_t* c, const double* v, int64_t nnz, bool on_device, cudaStream_t st)
+        : rows_d(st), cols_d(st), vals_d(st)
     {
         if (on_device) {
             rows = r; cols = c; vals = v;
@@ -408,14 +409,14 @@ struct coo_inputs {
 
 // Segments sorted keys into runs of equal keys; returns the run count and fills
 // start[0..runs] (start[runs] = nnz).
-int64_t segment_runs(const uint64_t* keys, int64_t nnz, cudaStream_t st, dbuf<int64_t>& start)
+int64_t segment_runs(const uint64_t* keys, int64_t nnz, cudaStream_t st, scratch<int64_t>& start)
 {
-    dbuf<int64_t> head(nnz), run_of(nnz);
+    scratch<int64_t> head(nnz, st), run_of(nnz, st);
     k_heads<<<grid_for(nnz), kThreads, 0, st>>>(keys, nnz, head.get());
     check_launch("k_heads");
     size_t tmp_bytes = 0;
     ABHSF_CUDA(cub::DeviceScan::InclusiveSum(nullptr, tmp_bytes, head.get(), run_of.get(), nnz, st));
-    dbuf<uint8_t> tmp(tmp_bytes);
+    scratch<uint8_t> tmp(tmp_bytes, st);
     ABHSF_CUDA(cub::DeviceScan::InclusiveSum(tmp.get(), tmp_bytes, head.get(), run_of.get(), nnz, st));
     const int64_t runs = read_scalar(run_of.get() + nnz - 1, st);
     start.alloc(runs + 1);
@@ -428,7 +429,7 @@ void exclusive_scan(int64_t* in, int64_t* out, int64_t count, cudaStream_t st)
 {
     size_t tmp_bytes = 0;
     ABHSF_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tmp_bytes, in, out, count, st));
-    dbuf<uint8_t> tmp(tmp_bytes);
+    scratch<uint8_t> tmp(tmp_bytes, st);
     ABHSF_CUDA(cub::DeviceScan::ExclusiveSum(tmp.get(), tmp_bytes, in, out, count, st));
 }
 
@@ -450,7 +451,7 @@ void exclusive_scan_i64(const int64_t* in, int64_t* out, int64_t count, cudaStre
 {
     size_t tmp_bytes = 0;
     ABHSF_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tmp_bytes, in, out, count, st));
-    dbuf<uint8_t> tmp(tmp_bytes);
+    scratch<uint8_t> tmp(tmp_bytes, st);
     ABHSF_CUDA(cub::DeviceScan::ExclusiveSum(tmp.get(), tmp_bytes, in, out, count, st));
 }
 
@@ -458,7 +459,7 @@ void inclusive_scan_i64(const int64_t* in, int64_t* out, int64_t count, cudaStre
 {
     size_t tmp_bytes = 0;
     ABHSF_CUDA(cub::DeviceScan::InclusiveSum(nullptr, tmp_bytes, in, out, count, st));
-    dbuf<uint8_t> tmp(tmp_bytes);
+    scratch<uint8_t> tmp(tmp_bytes, st);
     ABHSF_CUDA(cub::DeviceScan::InclusiveSum(tmp.get(), tmp_bytes, in, out, count, st));
 }
 
@@ -516,8 +517,8 @@ void finish_stats(abhsf_matrix& a, const scheme_params& sp, const int64_t* tile_
     const int64_t hl = (int64_t)a.s * a.s + 1;
     std::vector<uint64_t> h(hl, 0);
     if (a.T) {
-        dbuf<unsigned long long> dh(hl);
-        dbuf<int> err(1);
+        scratch<unsigned long long> dh(hl, st);
+        scratch<int> err(1, st);
         ABHSF_CUDA(cudaMemsetAsync(dh.get(), 0, hl * sizeof(unsigned long long), st));
         if (hl <= 8192)
             k_len_hist_shared<<<std::min(grid_for(a.T), 148u * 4), kThreads, hl * sizeof(unsigned int), st>>>(
@@ -605,7 +606,7 @@ void build_matrix(const int64_t* rows, const int64_t* cols, const double* vals, 
         fail(ABHSF_ERROR_OUT_OF_MEMORY, "more than 2^32 elements");
 
     // totals the host reads, together: error bits, tiles, stored values, payload bytes
-    dbuf<int64_t> totals(4);
+    scratch<int64_t> totals(4, st);
     ABHSF_CUDA(cudaMemsetAsync(totals.get(), 0, 4 * sizeof(int64_t), st));
     int* err = reinterpret_cast<int*>(totals.get());
     int64_t tot[4] = {0, 0, 0, 0};
@@ -614,9 +615,9 @@ void build_matrix(const int64_t* rows, const int64_t* cols, const double* vals, 
         ABHSF_CUDA(cudaStreamSynchronize(st));
         raise_err((int)tot[0]);
     };
-    dbuf<int64_t> tile_row, stored, pay;
-    dbuf<uint64_t> keys_in, keys;
-    dbuf<uint32_t> place_in, place;
+    scratch<int64_t> tile_row(st), stored(st), pay(st);
+    scratch<uint64_t> keys_in(st), keys(st);
+    scratch<uint32_t> place_in(st), place(st);
     int64_t* tile_start = nullptr;
     std::unique_ptr<coo_inputs> in;
     const int shift = 2 * lg;
@@ -641,7 +642,7 @@ void build_matrix(const int64_t* rows, const int64_t* cols, const double* vals, 
                                                    nnz, begin_bit, key_bits, st));
         tile_start = reinterpret_cast<int64_t*>(keys_in.get());  // the unsorted keys' memory, once they are sorted
         ABHSF_CUDA(cub::DeviceSelect::If(nullptr, b2, all, tile_start, totals.get() + 1, nnz, head, st));
-        dbuf<uint8_t> tmp(std::max(b1, b2));
+        scratch<uint8_t> tmp(std::max(b1, b2), st);
         ABHSF_CUDA(cub::DeviceRadixSort::SortPairs(tmp.get(), b1, keys_in.get(), keys.get(), place_in.get(),
                                                    place.get(), nnz, begin_bit, key_bits, st));
         ABHSF_CUDA(cub::DeviceSelect::If(tmp.get(), b2, all, tile_start, totals.get() + 1, nnz, head, st));
@@ -700,6 +701,7 @@ void build_matrix(const int64_t* rows, const int64_t* cols, const double* vals, 
     place.reset();
     prepare_tree(a, st);
     prepare_ring(a, st);
+    ABHSF_CUDA(cudaStreamSynchronize(st));  // the handle may be used on any stream from here on
 }
 
 void block_histogram(const int64_t* rows, const int64_t* cols, int64_t nnz, int64_t m, int64_t n, int r, int s,
@@ -722,9 +724,9 @@ void block_histogram(const int64_t* rows, const int64_t* cols, int64_t nnz, int6
     if (!rows || !cols)
         fail(ABHSF_ERROR_INVALID_VALUE, "rows and cols must be non-NULL");
     coo_inputs in(rows, cols, nullptr, nnz, on_device, st);
-    dbuf<int> err(1);
+    scratch<int> err(1, st);
     ABHSF_CUDA(cudaMemsetAsync(err.get(), 0, sizeof(int), st));
-    dbuf<uint64_t> keys(nnz), keys_out(nnz);
+    scratch<uint64_t> keys(nnz, st), keys_out(nnz, st);
     k_block_keys<<<grid_for(nnz), kThreads, 0, st>>>(in.rows, in.cols, nnz, m, n, k, l, keys.get(), err.get());
     check_launch("k_block_keys");
     raise_err(read_scalar(err.get(), st));
@@ -732,13 +734,13 @@ void block_histogram(const int64_t* rows, const int64_t* cols, int64_t nnz, int6
     size_t tmp_bytes = 0;
     ABHSF_CUDA(cub::DeviceRadixSort::SortKeys(nullptr, tmp_bytes, keys.get(), keys_out.get(), nnz, 0, end_bit, st));
     {
-        dbuf<uint8_t> tmp(tmp_bytes);
+        scratch<uint8_t> tmp(tmp_bytes, st);
         ABHSF_CUDA(cub::DeviceRadixSort::SortKeys(tmp.get(), tmp_bytes, keys.get(), keys_out.get(), nnz, 0, end_bit,
                                                   st));
     }
-    dbuf<int64_t> start;
+    scratch<int64_t> start(st);
     const int64_t B = segment_runs(keys_out.get(), nnz, st, start);
-    dbuf<unsigned long long> dh(hist_len);
+    scratch<unsigned long long> dh(hist_len, st);
     ABHSF_CUDA(cudaMemsetAsync(dh.get(), 0, hist_len * sizeof(unsigned long long), st));
     // few counters: added up in shared memory first (most blocks hold one of a
     // few counts, and 32,768 threads adding to one address wait on each other)

@@ -43,7 +43,7 @@ void spmm_dispatch(const abhsf_matrix& a, int k, const double* X, int64_t ldx, d
         spmv_dispatch(a, X, Y, st);
         return;
     }
-    dbuf<double> xc(a.n), yc(a.m);
+    scratch<double> xc(a.n, st), yc(a.m, st);
     for (int j = 0; j < k; ++j) {
         ABHSF_CUDA(cudaMemcpy2DAsync(xc.get(), sizeof(double), X + j, ldx * sizeof(double), sizeof(double), a.n,
                                      cudaMemcpyDeviceToDevice, st));

@@ -320,8 +320,8 @@ void spmv_t(const abhsf_matrix& a, const float* x, float* y, cudaStream_t st) { 
 
 template <typename T>
 struct cg_work {
-    dbuf<T> r, p, ap;
-    explicit cg_work(int64_t n) : r(n), p(n), ap(n) {}
+    scratch<T> r, p, ap;
+    cg_work(int64_t n, cudaStream_t cs) : r(n, cs), p(n, cs), ap(n, cs) {}
 };
 
 // r = b - A x (xn: scratch)
@@ -504,9 +504,9 @@ void cg_solve(const abhsf_matrix& a, const double* b, double* x, double rtol, in
     const int64_t n = a.n;
     solve_stream ss(user);
     cudaStream_t cs = ss.cs;
-    cg_work<double> w(n);
-    dbuf<double> xn(n), partial(2 * kRedBlocks);
-    dbuf<cg_state> st_d(1);
+    cg_work<double> w(n, cs);
+    scratch<double> xn(n, cs), partial(2 * kRedBlocks, cs);
+    scratch<cg_state> st_d(1, cs);
     cg_state st_h{};
     const double bb = norm2(b, n, partial.get(), st_d.get(), &st_h, cs);
     residual<double>(a, b, x, w.r.get(), xn.get(), n, cs);
@@ -531,10 +531,10 @@ void cg_solve_mixed(const abhsf_matrix& a64, const abhsf_matrix& a32, const doub
     const double f2 = update_factor * update_factor;
     solve_stream ss(user);
     cudaStream_t cs = ss.cs;
-    dbuf<double> r64(n), xn(n), partial(2 * kRedBlocks);
-    cg_work<float> w(n);
-    dbuf<float> d(n);  // the f32 solution since the last update
-    dbuf<cg_state> st_d(1), st64_d(1);
+    scratch<double> r64(n, cs), xn(n, cs), partial(2 * kRedBlocks, cs);
+    cg_work<float> w(n, cs);
+    scratch<float> d(n, cs);  // the f32 solution since the last update
+    scratch<cg_state> st_d(1, cs), st64_d(1, cs);
     cg_state st_h{};
     const double bb = norm2(b, n, partial.get(), st64_d.get(), &st_h, cs);
     const double tol2 = rtol * rtol * bb;

@@ -67,21 +67,24 @@ inline std::atomic<int64_t>& dbuf_allocations()
     return count;
 }
 
-// Device memory (alloc.cu): usable on any stream at once, given back after the
-// device has been waited for.
+// Device memory (alloc.cu).
 struct device_block {
-    int dev = -1;      // the device whose pool it came from (-1: cudaMalloc)
+    bool scratch = false;         // allocated and freed in the order of st
+    cudaStream_t st = nullptr;
+    int dev = -1;                 // the device whose pool it came from (-1: cudaMalloc)
     size_t bytes = 0;
 };
 void* device_alloc(size_t bytes, device_block& block);
 void device_free(void* ptr, const device_block& block) noexcept;
+// Waits for the device where a dbuf was freed, and gives its memory back.
+void settle_released() noexcept;
 
-// Owning device allocation.
+// Owning device allocation of a handle: usable on any stream at once, set aside
+// when freed until settle_released.
 template <typename T>
 class dbuf {
   public:
     dbuf() = default;
-    explicit dbuf(size_t count) { alloc(count); }
     ~dbuf() { reset(); }
     dbuf(const dbuf&) = delete;
     dbuf& operator=(const dbuf&) = delete;
@@ -114,10 +117,29 @@ class dbuf {
     T* get() const { return p_; }
     size_t size() const { return n_; }
 
+  protected:
+    device_block block_;
+
   private:
     T* p_ = nullptr;
     size_t n_ = 0;
-    device_block block_;
+};
+
+// Device memory of one call, used on the stream st alone.
+template <typename T>
+class scratch : public dbuf<T> {
+  public:
+    explicit scratch(cudaStream_t st)
+    {
+        this->block_.scratch = true;
+        this->block_.st = st;
+    }
+    scratch(size_t count, cudaStream_t st) : scratch(st) { this->alloc(count); }
+};
+
+// A handle's first member, which goes after its buffers.
+struct settles_released {
+    ~settles_released() { settle_released(); }
 };
 
 // Plain view of a built matrix passed to kernels by value.
@@ -171,6 +193,7 @@ __host__ __device__ inline int64_t tile_payload_bytes(int scheme, int64_t s, int
 
 // The handle behind abhsf_matrix*.
 struct abhsf_matrix {
+    abhsf::settles_released settles;
     int64_t m = 0, n = 0, nnz = 0;
     int32_t s = 0, lg = 0, value_type = ABHSF_VALUE_F64, matrix_type = ABHSF_MATRIX_REAL;
     int64_t M = 0, N = 0, T = 0, n_values = 0, payload_bytes = 0;
@@ -278,6 +301,7 @@ constexpr int kBatchMax = 1 << (32 - kBatchColBits);
 }  // namespace abhsf
 
 struct abhsf_batch {
+    abhsf::settles_released settles;
     std::vector<const abhsf_matrix*> mats;
     int32_t s = 0;
     int device = 0;

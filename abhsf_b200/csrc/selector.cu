@@ -246,7 +246,7 @@ void selector_features(const int64_t* rows, const int64_t* cols, int64_t nnz, in
         fail(ABHSF_ERROR_INVALID_VALUE, "rows and cols must be non-NULL");
     if (!out)
         fail(ABHSF_ERROR_INVALID_VALUE, "out must be non-NULL");
-    dbuf<int64_t> r_d, c_d;
+    scratch<int64_t> r_d(st), c_d(st);
     const int64_t* r = rows;
     const int64_t* c = cols;
     if (!on_device && nnz > 0) {
@@ -257,9 +257,9 @@ void selector_features(const int64_t* rows, const int64_t* cols, int64_t nnz, in
         r = r_d.get();
         c = c_d.get();
     }
-    dbuf<unsigned int> count(m);
-    dbuf<feat_acc> acc(1);
-    dbuf<double> var(1);
+    scratch<unsigned int> count(m, st);
+    scratch<feat_acc> acc(1, st);
+    scratch<double> var(1, st);
     ABHSF_CUDA(cudaMemsetAsync(count.get(), 0, m * sizeof(unsigned int), st));
     ABHSF_CUDA(cudaMemsetAsync(acc.get(), 0, sizeof(feat_acc), st));
     ABHSF_CUDA(cudaMemsetAsync(var.get(), 0, sizeof(double), st));
@@ -335,7 +335,7 @@ int mlp_predict(const float* model_host, const float features[ABHSF_FEATURES], c
     if (!features)
         fail(ABHSF_ERROR_INVALID_VALUE, "features must be non-NULL");
     const float* model = model_host ? model_host : kBuiltinModel;
-    dbuf<float> p(ABHSF_MLP_PARAMS), x(F), probs(C);
+    scratch<float> p(ABHSF_MLP_PARAMS, st), x(F, st), probs(C, st);
     ABHSF_CUDA(cudaMemcpyAsync(p.get(), model, ABHSF_MLP_PARAMS * sizeof(float), cudaMemcpyHostToDevice, st));
     ABHSF_CUDA(cudaMemcpyAsync(x.get(), features, F * sizeof(float), cudaMemcpyHostToDevice, st));
     mlp_forward(p.get(), x.get(), 1, probs.get(), nullptr, st);

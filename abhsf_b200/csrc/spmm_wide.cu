@@ -313,7 +313,7 @@ void prepare_wide(abhsf_matrix& a, cudaStream_t st)
     if (a.value_type != ABHSF_VALUE_F64 || a.sum_order != ABHSF_SUM_REFERENCE ||
         (a.s != 16 && a.s != 32 && a.s != 64) || a.T == 0 || a.tree_nrows == 0)
         return;
-    dbuf<unsigned long long> most(1);
+    scratch<unsigned long long> most(1, st);
     ABHSF_CUDA(cudaMemsetAsync(most.get(), 0, sizeof(unsigned long long), st));
     const unsigned g = (unsigned)std::max<int64_t>(1, std::min<int64_t>((a.T + 255) / 256, 1024));
     k_tile_bytes_max<<<g, 256, 0, st>>>(a.T, a.tile_idx_off.get(), a.tile_val_off.get(), most.get());

@@ -476,7 +476,7 @@ void prepare_tree(abhsf_matrix& a, cudaStream_t st)
     }
     a.tree_ctas = nsm * per_sm;
     a.tree_counter.alloc(1);
-    dbuf<int64_t> flag(a.M + 1), pos(a.M + 1);
+    scratch<int64_t> flag(a.M + 1, st), pos(a.M + 1, st);
     ABHSF_CUDA(cudaMemsetAsync(flag.get() + a.M, 0, sizeof(int64_t), st));
     const unsigned g = (unsigned)std::max<int64_t>(1, std::min<int64_t>((a.M + 255) / 256, 4096));
     k_nonempty_flags<<<g, 256, 0, st>>>(a.M, a.brow_ptr.get(), flag.get());
@@ -496,8 +496,8 @@ void prepare_tree(abhsf_matrix& a, cudaStream_t st)
     // warps finish close together.  The sort is stable (ties keep ascending
     // row order), so the order is deterministic; it does not affect results,
     // since each block row is summed by one warp on its own.
-    dbuf<uint32_t> asc(nr);
-    dbuf<uint64_t> w(nr), w_sorted(nr);
+    scratch<uint32_t> asc(nr, st);
+    scratch<uint64_t> w(nr, st), w_sorted(nr, st);
     k_nonempty_scatter<<<g, 256, 0, st>>>(a.M, a.brow_ptr.get(), pos.get(), asc.get());
     ABHSF_CUDA(cudaGetLastError());
     const unsigned gw = (unsigned)std::max<int64_t>(1, std::min<int64_t>((nr + 255) / 256, 4096));
@@ -506,7 +506,7 @@ void prepare_tree(abhsf_matrix& a, cudaStream_t st)
     size_t tmp_bytes = 0;
     ABHSF_CUDA(cub::DeviceRadixSort::SortPairsDescending(nullptr, tmp_bytes, w.get(), w_sorted.get(), asc.get(),
                                                          a.tree_rows.get(), nr, 0, 64, st));
-    dbuf<uint8_t> tmp(std::max<size_t>(tmp_bytes, 1));
+    scratch<uint8_t> tmp(std::max<size_t>(tmp_bytes, 1), st);
     ABHSF_CUDA(cub::DeviceRadixSort::SortPairsDescending(tmp.get(), tmp_bytes, w.get(), w_sorted.get(), asc.get(),
                                                          a.tree_rows.get(), nr, 0, 64, st));
     ABHSF_CUDA(cudaStreamSynchronize(st));

@@ -1480,7 +1480,7 @@ void tune_ring(abhsf_matrix& a, cudaStream_t st)
     using T = typename val_traits<VT>::T;
     if (forced_variant(a.ring_layout, a.ring_bulk))
         return;
-    dbuf<T> x(a.n), y(a.m);
+    scratch<T> x(a.n, st), y(a.m, st);
     ABHSF_CUDA(cudaMemsetAsync(x.get(), 0, a.n * sizeof(T), st));
     ABHSF_CUDA(cudaMemsetAsync(y.get(), 0, a.m * sizeof(T), st));
     int layout = 0, bulk = 0;
@@ -1517,15 +1517,15 @@ bool build_ring_schedule(const std::vector<const abhsf_matrix*>& mats, int col_b
     std::vector<uint64_t> wt;
     int64_t total_tiles = 0;
     unsigned int mpv = 0;
-    dbuf<unsigned int> max_pv(1);
+    scratch<unsigned int> max_pv(1, st);
     for (size_t i = 0; i < mats.size(); ++i) {
         const abhsf_matrix& a = *mats[i];
         const int64_t nr = a.tree_nrows;
         if (nr == 0)
             continue;
         total_tiles += a.T;
-        dbuf<uint64_t> w_d(nr);
-        dbuf<uint32_t> n_d(nr);
+        scratch<uint64_t> w_d(nr, st);
+        scratch<uint32_t> n_d(nr, st);
         const unsigned g = (unsigned)std::max<int64_t>(1, std::min<int64_t>((nr + 255) / 256, 4096));
         k_ring_weight<<<g, 256, 0, st>>>(nr, a.tree_rows.get(), a.view(), s, vsize, w_d.get(), n_d.get());
         ABHSF_CUDA(cudaGetLastError());
@@ -1631,8 +1631,8 @@ bool build_ring_schedule(const std::vector<const abhsf_matrix*>& mats, int col_b
         const int64_t n = (int64_t)m_rows[i].size();
         if (n == 0)
             continue;
-        dbuf<uint32_t> rows_d(n);
-        dbuf<int64_t> base_d(n);
+        scratch<uint32_t> rows_d(n, st);
+        scratch<int64_t> base_d(n, st);
         ABHSF_CUDA(cudaMemcpyAsync(rows_d.get(), m_rows[i].data(), n * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
         ABHSF_CUDA(cudaMemcpyAsync(base_d.get(), m_base[i].data(), n * sizeof(int64_t), cudaMemcpyHostToDevice, st));
         const uint32_t col_or = col_bits >= 32 ? 0u : (uint32_t)i << col_bits;
@@ -1779,13 +1779,13 @@ void prepare_batch(abhsf_batch& b, cudaStream_t st)
             mx = std::max(mx, a->n);
             my = std::max(my, a->m);
         }
-        dbuf<double> x(mx), y(my);
+        scratch<double> x(mx, st), y(my, st);
         ABHSF_CUDA(cudaMemsetAsync(x.get(), 0, mx * sizeof(double), st));
         ABHSF_CUDA(cudaMemsetAsync(y.get(), 0, my * sizeof(double), st));
         std::vector<const double*> xs(b.mats.size(), x.get());
         std::vector<double*> ys(b.mats.size(), y.get());
-        dbuf<const double*> xs_d(xs.size());
-        dbuf<double*> ys_d(ys.size());
+        scratch<const double*> xs_d(xs.size(), st);
+        scratch<double*> ys_d(ys.size(), st);
         ABHSF_CUDA(cudaMemcpyAsync(xs_d.get(), xs.data(), xs.size() * sizeof(double*), cudaMemcpyHostToDevice, st));
         ABHSF_CUDA(cudaMemcpyAsync(ys_d.get(), ys.data(), ys.size() * sizeof(double*), cudaMemcpyHostToDevice, st));
         int layout = 0, bulk = 0;

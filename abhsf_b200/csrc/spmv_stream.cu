@@ -995,8 +995,11 @@ void deal_slices(const std::vector<const abhsf_matrix*>& mats, dbuf<uint8_t>& sc
         }
     }
     wbeg[W] = (int64_t)out.size();
-    sched.alloc(out.size() * sizeof(dc_slice));
-    wbeg_d.alloc(W + 1);
+    // (a second deal of the same slices fits the first one's memory)
+    if (sched.size() < out.size() * sizeof(dc_slice))
+        sched.alloc(out.size() * sizeof(dc_slice));
+    if (wbeg_d.size() < (size_t)W + 1)
+        wbeg_d.alloc(W + 1);
     ABHSF_CUDA(cudaMemcpyAsync(sched.get(), out.data(), out.size() * sizeof(dc_slice), cudaMemcpyHostToDevice, st));
     ABHSF_CUDA(cudaMemcpyAsync(wbeg_d.get(), wbeg.data(), (W + 1) * sizeof(int64_t), cudaMemcpyHostToDevice, st));
     ABHSF_CUDA(cudaStreamSynchronize(st));
@@ -1036,8 +1039,8 @@ void prepare_stream(abhsf_matrix& a, float avg, cudaStream_t st)
     if (avg <= 0.f || a.tree_nrows == 0 || a.sum_order != ABHSF_SUM_REFERENCE || (uint64_t)a.n > (uint64_t(1) << 32))
         return;
     const int64_t nr = a.tree_nrows;
-    dbuf<uint8_t> ok(nr);
-    dbuf<int64_t> elems(nr), fbytes(nr);
+    scratch<uint8_t> ok(nr, st);
+    scratch<int64_t> elems(nr, st), fbytes(nr, st);
     const int vsize = (int)value_size(a.value_type);
     k_dc_classify<<<grid_of(nr), 256, 0, st>>>(nr, a.tree_rows.get(), a.view(), avg, vsize, ok.get(), elems.get(),
                                                 fbytes.get());
@@ -1071,8 +1074,8 @@ void prepare_stream(abhsf_matrix& a, float avg, cudaStream_t st)
         sidx_h[sel[k].first] = (int32_t)k;
         ebase[k + 1] = ebase[k] + eh[sel[k].second];
     }
-    dbuf<int32_t> sidx(a.M);
-    dbuf<unsigned int> cnt(ns * s);
+    scratch<int32_t> sidx(a.M, st);
+    scratch<unsigned int> cnt(ns * s, st);
     ABHSF_CUDA(cudaMemcpyAsync(sidx.get(), sidx_h.data(), a.M * sizeof(int32_t), cudaMemcpyHostToDevice, st));
     ABHSF_CUDA(cudaMemsetAsync(cnt.get(), 0, ns * s * sizeof(unsigned int), st));
     k_dc_row_counts<<<grid_of(8 * a.T), 256, 0, st>>>(a.T, a.view(), s, lg, sidx.get(), cnt.get());
@@ -1090,8 +1093,9 @@ void prepare_stream(abhsf_matrix& a, float avg, cudaStream_t st)
     std::vector<uint32_t> selrow_h(ns);
     for (int64_t k = 0; k < ns; ++k)
         selrow_h[k] = sel[k].first;
-    dbuf<uint32_t> selrow(ns), sq(R), sq2(R), cq(E / kChainMin + 1), skey(R), skey2(R);
-    dbuf<int64_t> seg_d(nseg + 1), begin_d(nseg + 1), first_d(nseg + 1), found(2), rstart(R + 1), slot0(R);
+    scratch<uint32_t> selrow(ns, st), sq(R, st), sq2(R, st), cq(E / kChainMin + 1, st), skey(R, st), skey2(R, st);
+    scratch<int64_t> seg_d(nseg + 1, st), begin_d(nseg + 1, st), first_d(nseg + 1, st), found(2, st), rstart(R + 1, st),
+        slot0(R, st);
     ABHSF_CUDA(cudaMemcpyAsync(selrow.get(), selrow_h.data(), ns * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
     ABHSF_CUDA(cudaMemcpyAsync(seg_d.get(), seg.data(), (nseg + 1) * sizeof(int64_t), cudaMemcpyHostToDevice, st));
     std::vector<int64_t> begin(nseg + 1, 0), first(nseg + 1, 0);
@@ -1109,7 +1113,7 @@ void prepare_stream(abhsf_matrix& a, float avg, cudaStream_t st)
         ABHSF_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, b3, skey.get(), skey2.get(), sq.get(), sq2.get(), R, 0, kb,
                                                    st));
         ABHSF_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, b4, cnt.get(), rstart.get(), R, st));
-        dbuf<uint8_t> tmp(std::max(std::max(b1, b2), std::max(b3, b4)));
+        scratch<uint8_t> tmp(std::max(std::max(b1, b2), std::max(b3, b4)), st);
         ABHSF_CUDA(cub::DeviceSelect::If(tmp.get(), b1, all, sq.get(), found.get(), R, is_sliced{cnt.get()}, st));
         ABHSF_CUDA(cub::DeviceSelect::If(tmp.get(), b2, all, cq.get(), found.get() + 1, R, is_chain{cnt.get()}, st));
         ABHSF_CUDA(cub::DeviceScan::ExclusiveSum(tmp.get(), b4, cnt.get(), rstart.get(), R, st));
@@ -1131,7 +1135,7 @@ void prepare_stream(abhsf_matrix& a, float avg, cudaStream_t st)
         if (n2[1]) {
             chain_q.resize(n2[1]);
             ABHSF_CUDA(cudaMemcpyAsync(chain_q.data(), cq.get(), n2[1] * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-            dbuf<unsigned int> cl(n2[1]);
+            scratch<unsigned int> cl(n2[1], st);
             k_dc_gather<<<grid_of(n2[1]), 256, 0, st>>>(n2[1], cq.get(), cnt.get(), cl.get());
             ABHSF_CUDA(cudaGetLastError());
             chain_len.resize(n2[1]);
@@ -1149,7 +1153,7 @@ void prepare_stream(abhsf_matrix& a, float avg, cudaStream_t st)
     first[nseg] = nslices;
     std::vector<uint32_t> steps(nslices);
     if (nS) {
-        dbuf<uint32_t> steps_d(nslices);
+        scratch<uint32_t> steps_d(nslices, st);
         ABHSF_CUDA(cudaMemcpyAsync(first_d.get(), first.data(), (nseg + 1) * sizeof(int64_t), cudaMemcpyHostToDevice,
                                    st));
         k_dc_steps<<<grid_of(nS), 256, 0, st>>>(nS, skey2.get(), begin_d.get(), first_d.get(), steps_d.get());
@@ -1201,7 +1205,7 @@ void prepare_stream(abhsf_matrix& a, float avg, cudaStream_t st)
     }
     a.dc_lane.alloc(std::max<int64_t>(32 * nslices, 1));
     if (nS) {
-        dbuf<int64_t> base_d(nslices);
+        scratch<int64_t> base_d(nslices, st);
         ABHSF_CUDA(cudaMemcpyAsync(base_d.get(), base.data(), nslices * sizeof(int64_t), cudaMemcpyHostToDevice, st));
         ABHSF_CUDA(cudaMemsetAsync(a.dc_lane.get(), 0, 32 * nslices * sizeof(uint32_t), st));
         k_dc_lanes<<<grid_of(nS), 256, 0, st>>>(nS, skey2.get(), sq2.get(), selrow.get(), seg_d.get(), begin_d.get(),
@@ -1210,7 +1214,7 @@ void prepare_stream(abhsf_matrix& a, float avg, cudaStream_t st)
         ABHSF_CUDA(cudaStreamSynchronize(st));
     }
     if (!chain_q.empty()) {
-        dbuf<int64_t> slot_d(chain_q.size());
+        scratch<int64_t> slot_d(chain_q.size(), st);
         ABHSF_CUDA(cudaMemcpyAsync(slot_d.get(), chain_slot.data(), chain_q.size() * sizeof(int64_t),
                                    cudaMemcpyHostToDevice, st));
         k_dc_chain_slots<<<grid_of(chain_q.size()), 256, 0, st>>>((int64_t)chain_q.size(), cq.get(), slot_d.get(),
@@ -1219,8 +1223,8 @@ void prepare_stream(abhsf_matrix& a, float avg, cudaStream_t st)
         ABHSF_CUDA(cudaStreamSynchronize(st));
     }
     // the elements row by row: sort by (block row, row), stable in format order
-    dbuf<uint32_t> key(E), pos(E), key2(E), pos2(E), colv(E);
-    dbuf<int64_t> vidx(E), ebase_d(ns + 1);
+    scratch<uint32_t> key(E, st), pos(E, st), key2(E, st), pos2(E, st), colv(E, st);
+    scratch<int64_t> vidx(E, st), ebase_d(ns + 1, st);
     ABHSF_CUDA(cudaMemcpyAsync(ebase_d.get(), ebase.data(), (ns + 1) * sizeof(int64_t), cudaMemcpyHostToDevice, st));
     k_dc_expand<<<grid_of(8 * a.T), 256, 0, st>>>(a.T, a.view(), s, lg, sidx.get(), ebase_d.get(), key.get(), pos.get(),
                                               colv.get(), vidx.get());
@@ -1232,7 +1236,7 @@ void prepare_stream(abhsf_matrix& a, float avg, cudaStream_t st)
     ABHSF_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tb, key.get(), key2.get(), pos.get(), pos2.get(), (int)E, 0,
                                                bits, st));
     {
-        dbuf<uint8_t> tmp(tb);
+        scratch<uint8_t> tmp(tb, st);
         ABHSF_CUDA(cub::DeviceRadixSort::SortPairs(tmp.get(), tb, key.get(), key2.get(), pos.get(), pos2.get(),
                                                    (int)E, 0, bits, st));
         ABHSF_CUDA(cudaStreamSynchronize(st));  // before tmp goes

@@ -37,6 +37,11 @@ ABHSF_API abhsf_status abhsf_test_ring_variant(abhsf_matrix* a, int32_t set, int
  * nothing keeps that promise. */
 ABHSF_API int64_t abhsf_test_device_allocations(void);
 
+/* Blocks of released handles that are not given back yet, because the device
+ * could not be waited for when the handle went (a stream capture in global
+ * mode forbids it): the next release that can wait gives them back. */
+ABHSF_API int64_t abhsf_test_blocks_set_aside(void);
+
 /* The device Matrix Market parser's decimal conversion, run on the host on
  * the len bytes at text: 0 = converted (*value, *used bytes read), 1 = left to
  * the host's parser (not a plain decimal, more than 19 significant digits, a
