@@ -93,11 +93,18 @@ constexpr uint32_t kFirst = 1u << 30, kLast = 1u << 31, kRowMask = kFirst - 1;
 // a COO tile of more than 32 elements whose rows hold one element each
 constexpr uint32_t kDistinctRows = 1u << 26;
 
-// Matrices of up to so many tiles: the ring serves every block row, one launch an
-// SpMV, where a launch is most of the time (banded, 46 to 1,405 tiles: 9.0 us
+// Matrices of up to kSoloTiles tiles: the ring serves every block row, one launch
+// an SpMV, where a launch is most of the time (banded, 46 to 1,405 tiles: 9.0 us
 // against 11.3 with the slices beside; a mixture of 1,866 16.6 against 18.5, of
 // 6,244 20.5 against 21.5; banded of 4,687 12.3 either way).
+// Not where a block row of the slices has more than kSoloRowTiles tiles: one CTA
+// walks a block row, 0.2 to 1.3 us a tile, which the slices' lanes share.  A block
+// row of 4 tiles of 1 to 250 elements each took 9.3 to 12.4 us against 11.3 to
+// 13.1 with the slices (700 such beside 1,000 dense ones: 12.4 against 12.1 to
+// 12.5); of 6 tiles of 100, 12.4 against 11.8; of 16, 24.7 against 11.8; one of
+// 3,900 single elements 1,028 against 13.8.
 constexpr int64_t kSoloTiles = 4096;
+constexpr uint32_t kSoloRowTiles = 4;
 
 // test hooks (abhsf_test_set_hooks)
 int64_t g_drop_desc = -1;
@@ -1472,8 +1479,9 @@ void time_variants(F&& run, int s, cudaStream_t st, int& layout, int& bulk)
     bulk = best.bulk;
 }
 
-// Times the single-right-hand-side variants on zero x and y and keeps the
-// fastest for the matrix (each gives the same y bit for bit).
+// Times the single-right-hand-side variants, on the schedule that an SpMV of this
+// matrix runs and zero x and y, and keeps the fastest for the matrix (each gives
+// the same y bit for bit).
 template <int S, int VT>
 void tune_ring(abhsf_matrix& a, cudaStream_t st)
 {
@@ -1489,7 +1497,11 @@ void tune_ring(abhsf_matrix& a, cudaStream_t st)
             a.ring_layout = tm;
             a.ring_bulk = bk;
             beside bs;
-            launch_ring<S, 1, VT>(bs, a, x.get(), 1, y.get(), 1, st, true);
+            if (a.solo_ctas)
+                launch_ring<S, 1, VT>(bs, a, x.get(), 1, y.get(), 1, st, true, a.solo_desc.get(), a.solo_wbeg.get(),
+                                      a.solo_ctas);
+            else
+                launch_ring<S, 1, VT>(bs, a, x.get(), 1, y.get(), 1, st, true);
         },
         S, st, layout, bulk);
     a.ring_layout = layout;
@@ -1502,7 +1514,8 @@ void tune_ring(abhsf_matrix& a, cudaStream_t st)
 // and value type) over the ring kernel's grid, longest processing time first,
 // and writes every CTA's tile descriptors, matrix i's columns tagged with
 // i << col_bits.  Returns false when a CTA would get more tiles than its
-// counters hold.
+// counters hold.  with_slices: the block rows the slices serve, too -- false where
+// one of them has more than kSoloRowTiles tiles.
 bool build_ring_schedule(const std::vector<const abhsf_matrix*>& mats, int col_bits, dbuf<uint8_t>& desc,
                          dbuf<int64_t>& wbeg_d, int& ctas_out, int& max_pv_out, cudaStream_t st, int64_t brow_lo = 0,
                          int64_t brow_hi = INT64_MAX, bool with_slices = false)
@@ -1558,9 +1571,13 @@ bool build_ring_schedule(const std::vector<const abhsf_matrix*>& mats, int col_b
             if (nr == 0)
                 continue;
             for (int64_t k = 0; k < nr; ++k, ++o)
-                if (!with_slices && (size_t)k < f.size() && f[k]) {
-                    skip[o] = 1;
-                    any_skip = true;
+                if ((size_t)k < f.size() && f[k]) {
+                    if (with_slices && ntiles[o] > kSoloRowTiles)
+                        return false;
+                    if (!with_slices) {
+                        skip[o] = 1;
+                        any_skip = true;
+                    }
                 }
         }
     }

@@ -1,0 +1,70 @@
+"""Small matrices whose SpMV is one launch of the ring kernel over every block
+row, the sliced ones among them: which matrices that is, and y bitwise the
+reference order's either way."""
+import numpy as np
+import pytest
+
+from abhsf_b200 import AbhsfMatrix
+from oracle import oracle
+
+pytestmark = pytest.mark.gpu
+
+
+def _matrix(s, dense, wide, z, seed):
+    """`dense` diagonal tiles about 30% full (bitmaps), then a block row of
+    `wide` tiles of z elements (COO, at the wide end z = 1), ragged at the end."""
+    rng = np.random.default_rng(seed)
+    nb = max(dense + 1, wide)
+    n = nb * s - 3
+    rows, cols = [], []
+    for d in range(dense):
+        k = np.nonzero(rng.random(s * s) < 0.3)[0]
+        rows.append(d * s + k // s)
+        cols.append(d * s + k % s)
+    for J in rng.choice(nb, wide, replace=False):
+        k = rng.choice(s * s, z, replace=False)
+        rows.append(dense * s + k // s)
+        cols.append(J * s + k % s)
+    r, c = np.concatenate(rows), np.concatenate(cols)
+    ok = (r < n) & (c < n)
+    key = np.unique(r[ok].astype(np.int64) * n + c[ok])
+    return key // n, key % n, rng.standard_normal(key.size), n
+
+
+def _check(r, c, v, n, s, vt, kernels):
+    import torch
+    rng = np.random.default_rng(5)
+    A = AbhsfMatrix.from_elements(r, c, v, n, n, block_size=s, value_type=vt)
+    assert A.kernels() == kernels
+    x, y0 = rng.uniform(-1, 1, n), rng.standard_normal(n)
+    if vt == "f64":
+        y = torch.from_numpy(y0.copy()).cuda()
+        A.spmv(torch.from_numpy(x).cuda(), y)
+        ref = oracle.spmv_elements(r, c, v, x, y0.copy())
+    else:
+        x, y0 = x.astype(np.float32), y0.astype(np.float32)
+        stored = torch.from_numpy(v).float()
+        if vt == "bf16":
+            stored = stored.bfloat16().float()
+        y = torch.from_numpy(y0.copy()).cuda()
+        A.spmv_f32(torch.from_numpy(x).cuda(), y)
+        ref = oracle.spmv_elements_f32(r, c, stored.numpy(), x, y0.copy())
+    assert np.array_equal(y.cpu().numpy(), ref)
+    return A
+
+
+@pytest.mark.parametrize("vt", ["f64", "f32", "bf16"])
+@pytest.mark.parametrize("s", [32, 64])
+@pytest.mark.parametrize("wide,z", [(1, 30), (4, 40), (5, 40), (300, 8), (3000, 1)])
+def test_a_wide_sliced_block_row_keeps_its_slices(gpu, s, vt, wide, z):
+    """One CTA of the ring sums a whole block row: up to four tiles of a sliced
+    one are walked there, a wide one stays with the slices."""
+    r, c, v, n = _matrix(s, 9, wide, z, seed=wide)
+    _check(r, c, v, n, s, vt, 1 if wide <= 4 else 2)
+
+
+@pytest.mark.parametrize("tiles,kernels", [(4096, 1), (4097, 2)])
+def test_tiles_of_a_one_launch_matrix(gpu, tiles, kernels):
+    r, c, v, n = _matrix(32, tiles - 2, 2, 20, seed=1)
+    A = _check(r, c, v, n, 32, "f64", kernels)
+    assert A.stats()["tiles"] == tiles
