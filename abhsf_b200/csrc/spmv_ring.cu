@@ -1755,6 +1755,8 @@ void prepare_ring(abhsf_matrix& a, cudaStream_t st)
     if (a.dc_warps > 0 && a.dc_cwarps == 0 && a.T <= kSoloTiles &&
         !build_ring_schedule({&a}, 32, a.solo_desc, a.solo_wbeg, a.solo_ctas, mpv, st, 0, INT64_MAX, true))
         a.solo_ctas = 0;
+    if (a.solo_ctas)
+        a.stats.spmv_bytes = a.stats.format_bytes;  // no slice is read
     if (a.value_type == ABHSF_VALUE_F64)
         a.s == 32 ? tune_ring<32, ABHSF_VALUE_F64>(a, st) : tune_ring<64, ABHSF_VALUE_F64>(a, st);
     else if (a.value_type == ABHSF_VALUE_F32)

@@ -214,7 +214,8 @@ typedef struct abhsf_stats {
     int64_t spmv_bytes;     /* what one reference-order SpMV reads of the matrix (x and y excluded): the
                                format bytes of the block rows the tile kernel sums, and for the block
                                rows in row slices their words, values, lane records and slice records
-                               (format_bytes when no block row is in slices) */
+                               (format_bytes when no block row is in slices, or when one launch of
+                               the tile kernel serves a small matrix's every block row) */
 } abhsf_stats;
 
 /* Fills the defaults: s = 64, f64, CSR allowed, REAL, minimum storage, host
@@ -232,8 +233,9 @@ ABHSF_API abhsf_status abhsf_build(const int64_t* rows, const int64_t* cols, con
 
 /* How many kernels one abhsf_spmv of this matrix launches (the tile kernel
  * or the streaming kernel for the block rows it serves, the row-slice kernel
- * and the chain kernel for those in slices).  No counterpart in the
- * reference. */
+ * and the chain kernel for those in slices; the tile kernel alone for some
+ * matrices of up to 4,096 tiles, the block rows in slices among them).  No
+ * counterpart in the reference. */
 ABHSF_API abhsf_status abhsf_spmv_kernels(const abhsf_matrix* a, int32_t* kernels);
 
 /* y += A x, x[n] and y[m] float64 in device memory; matrix stored as f64.

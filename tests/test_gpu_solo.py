@@ -68,3 +68,21 @@ def test_tiles_of_a_one_launch_matrix(gpu, tiles, kernels):
     r, c, v, n = _matrix(32, tiles - 2, 2, 20, seed=1)
     A = _check(r, c, v, n, 32, "f64", kernels)
     assert A.stats()["tiles"] == tiles
+
+
+@pytest.mark.parametrize("wide", [4, 300])
+def test_bytes_an_spmv_reads(gpu, wide):
+    """One launch reads the format and no slice; else the block row of `wide`
+    tiles is read as slices (word and value an element, 32 bytes a slice, a lane
+    record a row) in place of its share of the format (row pointer, 25 bytes of
+    header and 16 of COO keys a tile, 8 an element)."""
+    r, c, v, n = _matrix(64, 9, wide, 8, seed=2)
+    A = AbhsfMatrix.from_elements(r, c, v, n, n, block_size=64)
+    st, sl = A.stats(), A.slices()
+    assert sl["block_rows"] == 1
+    if A.kernels() == 1:
+        assert st["spmv_bytes"] == st["format_bytes"]
+        return
+    share = 8 + (st["tiles"] - 9) * (25 + 16) + 8 * sl["elements"]
+    assert st["spmv_bytes"] == st["format_bytes"] - share + 12 * sl["elements"] + 32 * sl["slices"] + \
+        4 * int(sl["lanes"].sum())
