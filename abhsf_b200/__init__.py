@@ -13,6 +13,7 @@ _EXPORTS = {
     "read_mtx_device": "matrix",
     "read_mm": "matrix", "write_mm": "matrix", "mtx2mm": "matrix", "expand_symmetric": "matrix", "block_histograms_all": "matrix", "block_scheme_bits": "matrix",
     "block_select_scheme": "matrix", "mmf_line": "matrix", "cg": "matrix", "cg_mixed": "matrix",
+    "trim_device_memory": "matrix",
     "ShardedMatrix": "sharded",
 }
 

@@ -129,6 +129,7 @@ PROTOTYPES = {
     "abhsf_cg_mixed": (C.c_int, [_vp, _vp, _vp, _vp, C.c_double, _i32, C.c_double, _i32, C.POINTER(CgInfo),
                                  _vp]),
     "abhsf_release": (C.c_int, [_vp]),
+    "abhsf_trim_device_memory": (C.c_int, [C.POINTER(_i64)]),
     "abhsf_stats_get": (C.c_int, [_vp, C.POINTER(Stats)]),
     "abhsf_export_host": (C.c_int, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp]),
     "abhsf_block_histogram": (C.c_int, [_vp, _vp, _i64, _i64, _i64, _i32, _i32, _i32, _vp, _u64p, _i64,

@@ -268,6 +268,14 @@ class AbhsfMatrix:
         return out
 
 
+def trim_device_memory() -> int:
+    """Gives back the device memory that the library keeps for its next calls (up
+    to 2 GB a device), so that other allocators can have it: how many bytes."""
+    n = C.c_int64()
+    capi.check(capi.lib.abhsf_trim_device_memory(C.byref(n)))
+    return n.value
+
+
 # ---------------------------------------------------------------------- block statistics
 def block_histogram(rows, cols, m: int, n: int, r: int, s: int, stream=None) -> dict[int, int]:
     """block nnz -> number of r x s blocks, computed on the GPU

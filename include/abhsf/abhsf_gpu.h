@@ -13,7 +13,8 @@
  * Conventions: every call returns abhsf_status and never throws; the reason
  * for the last failure on the calling thread is abhsf_last_error_string().
  * Indices are 0-based (matrix_market_reader.h:135-136).  A handle owns all of
- * its device memory.  Calls taking a stream are ordered on it; a NULL stream
+ * its device memory.  What calls and released handles leave is kept for the
+ * next ones, up to 2 GB a device (abhsf_trim_device_memory).  Calls taking a stream are ordered on it; a NULL stream
  * is the legacy default stream.  abhsf_stats_get may be called from several
  * threads at once.  abhsf_spmv keeps a work counter in the handle: SpMVs on
  * one handle must not overlap on the GPU (queue them on one stream, or order
@@ -320,6 +321,14 @@ ABHSF_API abhsf_status abhsf_spmv_host(abhsf_matrix* a, const double* x, double*
 
 /* Frees the handle and its device memory (release(), spmv/bottlenecks/spmv.cpp:125-133). */
 ABHSF_API abhsf_status abhsf_release(abhsf_matrix* a);
+
+/* Gives back the device memory that the library keeps for its next calls, on
+ * every device it has used, after waiting for the device; handles in use stay as
+ * they are.  For a program that is done building and whose next allocations
+ * come from elsewhere.  bytes (may be NULL): how much it was.  The library does
+ * this by itself where an allocation of its own finds no memory.  No reference
+ * counterpart. */
+ABHSF_API abhsf_status abhsf_trim_device_memory(int64_t* bytes);
 
 /* Format statistics, including the reference's per-scheme storage totals. */
 ABHSF_API abhsf_status abhsf_stats_get(const abhsf_matrix* a, abhsf_stats* out);

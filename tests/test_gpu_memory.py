@@ -8,7 +8,7 @@ import time
 import numpy as np
 import pytest
 
-from abhsf_b200 import AbhsfMatrix, capi, cg, cg_mixed
+from abhsf_b200 import AbhsfMatrix, capi, cg, cg_mixed, read_mtx_device, trim_device_memory
 from abhsf_b200 import workloads as W
 from oracle import oracle
 
@@ -150,3 +150,51 @@ def test_release_while_a_capture_forbids_waiting(gpu):
     y = torch.zeros(coo.m, dtype=torch.float64, device="cuda")
     build().spmv(torch.from_numpy(x).cuda(), y)
     assert np.array_equal(y.cpu().numpy(), _reference(coo, x))
+
+
+def test_unused_memory_is_given_back(gpu):
+    """What builds and releases leave is kept for the next call, and goes back
+    to the device on request; a matrix in use stays as it is."""
+    import torch
+    coo = W.random_blocky(900, 900, 64, 80, seed=73)
+    x = W.rhs(coo.n, 11)
+    A = AbhsfMatrix.from_elements(coo.rows, coo.cols, coo.vals, coo.m, coo.n)
+    big = W.random_uniform(400000, 400000, 6_000_000, seed=74)
+
+    def build():
+        AbhsfMatrix.from_elements(big.rows, big.cols, big.vals, big.m, big.n).release()
+
+    build()  # the kernels' code and stacks are on the device from here on
+    trim_device_memory()
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    build()
+    kept = free - torch.cuda.mem_get_info()[0]
+    assert 0 < kept <= (2 << 30) + (64 << 20)
+    back = trim_device_memory()
+    assert back > 0.9 * kept - (64 << 20) and free - torch.cuda.mem_get_info()[0] <= 64 << 20
+    y = torch.zeros(coo.m, dtype=torch.float64, device="cuda")
+    A.spmv(torch.from_numpy(x).cuda(), y)
+    assert np.array_equal(y.cpu().numpy(), _reference(coo, x))
+
+
+def test_the_reader_gets_what_the_library_keeps(gpu, tmp_path):
+    """The device reader's memory does not come from the library's pool; on a
+    card that others have filled it gets what the pool holds unused."""
+    import torch
+    coo = W.random_uniform(30000, 30000, 400_000, seed=75)
+    path = tmp_path / "a.mtx"
+    with open(path, "w") as f:
+        f.write("%%%%MatrixMarket matrix coordinate real general\n%d %d %d\n" % (coo.m, coo.n, coo.nnz))
+        f.writelines("%d %d %.17g\n" % (r + 1, c + 1, v) for r, c, v in zip(coo.rows, coo.cols, coo.vals))
+    want = [t.cpu() for t in read_mtx_device(str(path))[:3]]
+    big = W.random_uniform(400000, 400000, 6_000_000, seed=76)
+    AbhsfMatrix.from_elements(big.rows, big.cols, big.vals, big.m, big.n).release()
+    torch.cuda.empty_cache()
+    fill = torch.empty(torch.cuda.mem_get_info()[0] - (24 << 20), dtype=torch.uint8, device="cuda")
+    try:
+        got = [t.cpu() for t in read_mtx_device(str(path))[:3]]
+    finally:
+        del fill
+        torch.cuda.empty_cache()
+    assert all(torch.equal(a, b) for a, b in zip(want, got))
