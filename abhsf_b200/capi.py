@@ -108,6 +108,7 @@ PROTOTYPES = {
     "abhsf_device_status": (C.c_int, [_vp, _vp, _i32, C.POINTER(_i32)]),
     "abhsf_test_set_hooks": (None, [_i64, C.c_uint32]),
     "abhsf_test_ring_variant": (C.c_int, [_vp, _i32, C.POINTER(_i32), C.POINTER(_i32)]),
+    "abhsf_test_pick_variant": (_i32, [_i32, C.POINTER(C.c_float), _i32, C.POINTER(_i32), C.POINTER(_i32)]),
     "abhsf_test_device_allocations": (_i64, []),
     "abhsf_test_blocks_set_aside": (_i64, []),
     "abhsf_slices_info": (C.c_int, [_vp] + [C.POINTER(_i64)] * 5),

@@ -1429,17 +1429,33 @@ bool forced_variant(int& layout, int& bulk)
     return true;
 }
 
+// The clock of time_variants: intervals of st's time.
+struct stream_clock {
+    cudaStream_t st;
+    std::vector<event_pair> ev;
+    stream_clock(cudaStream_t s, int intervals) : st(s), ev(intervals) {}
+    void begin(int k) { ABHSF_CUDA(cudaEventRecord(ev[k].a, st)); }
+    void end(int k) { ABHSF_CUDA(cudaEventRecord(ev[k].b, st)); }
+    float ms(int k)
+    {
+        float t = 0.f;
+        ABHSF_CUDA(cudaEventSynchronize(ev[k].b));
+        ABHSF_CUDA(cudaEventElapsedTime(&t, ev[k].a, ev[k].b));
+        return t;
+    }
+};
+
 // The variant (consumer layout, bulk x / y copies or not) whose launches of
-// run(layout, bulk) take least time on st: each is launched twice, the second
-// launch timed, and the three fastest three times more, their best launches
-// compared (25 launches: on a matrix of 60M elements, six of every variant took
-// 5.2 ms of a build's 11.7 ms of GPU time).  At s = 32 layout 3 is layout 1 and
+// run(layout, bulk) take least time: each is launched twice, and the three
+// fastest by their better launch three times more, their best launches compared
+// (25 launches: on a matrix of 60M elements, six of every variant took 5.2 ms of a
+// build's 11.7 ms of GPU time).  Every launch is timed, so one that something
+// else disturbed costs no variant its place.  At s = 32 layout 3 is layout 1 and
 // is skipped.
-template <typename F>
-void time_variants(F&& run, int s, cudaStream_t st, int& layout, int& bulk)
+constexpr int kFirstCut = 2, kFinal = 3, kReps = 3, kIntervals = kFirstCut * 2 * kLayouts + kFinal * kReps;
+template <typename F, typename C>
+void time_variants(F&& run, int s, C&& clock, int& layout, int& bulk)
 {
-    constexpr int kFinal = 3, kReps = 3, kAll = 2 * kLayouts;
-    event_pair ev[kAll + kFinal * kReps];
     struct variant {
         int layout, bulk;
         float ms;
@@ -1448,31 +1464,29 @@ void time_variants(F&& run, int s, cudaStream_t st, int& layout, int& bulk)
     for (int tm = 0; tm < kLayouts; ++tm)
         for (int bk = 0; bk <= 1; ++bk)
             if (!(s == 32 && tm == 3))
-                v.push_back({tm, bk, 0.f});
-    auto timed = [&](const variant& a, event_pair& e) {
-        ABHSF_CUDA(cudaEventRecord(e.a, st));
+                v.push_back({tm, bk, 3.4e38f});
+    int k = 0;  // interval
+    auto timed = [&](const variant& a) {
+        clock.begin(k);
         run(a.layout, a.bulk);
-        ABHSF_CUDA(cudaEventRecord(e.b, st));
+        clock.end(k++);
     };
-    auto read = [&](event_pair& e) {
-        float ms = 0.f;
-        ABHSF_CUDA(cudaEventSynchronize(e.b));
-        ABHSF_CUDA(cudaEventElapsedTime(&ms, e.a, e.b));
-        return ms;
-    };
-    for (size_t i = 0; i < v.size(); ++i) {
-        run(v[i].layout, v[i].bulk);
-        timed(v[i], ev[i]);
-    }
-    for (size_t i = 0; i < v.size(); ++i)
-        v[i].ms = read(ev[i]);
+    for (const variant& a : v)
+        for (int r = 0; r < kFirstCut; ++r)
+            timed(a);
+    k = 0;
+    for (variant& a : v)
+        for (int r = 0; r < kFirstCut; ++r)
+            a.ms = std::min(a.ms, clock.ms(k++));
     std::stable_sort(v.begin(), v.end(), [](const variant& a, const variant& b) { return a.ms < b.ms; });
+    const int k0 = k;
     for (int r = 0; r < kReps; ++r)
         for (int i = 0; i < kFinal; ++i)
-            timed(v[i], ev[kAll + r * kFinal + i]);
+            timed(v[i]);
+    k = k0;
     for (int r = 0; r < kReps; ++r)
         for (int i = 0; i < kFinal; ++i)
-            v[i].ms = std::min(v[i].ms, read(ev[kAll + r * kFinal + i]));
+            v[i].ms = std::min(v[i].ms, clock.ms(k++));
     const variant best = *std::min_element(v.begin(), v.begin() + kFinal,
                                            [](const variant& a, const variant& b) { return a.ms < b.ms; });
     layout = best.layout;
@@ -1503,7 +1517,7 @@ void tune_ring(abhsf_matrix& a, cudaStream_t st)
             else
                 launch_ring<S, 1, VT>(bs, a, x.get(), 1, y.get(), 1, st, true);
         },
-        S, st, layout, bulk);
+        S, stream_clock(st, kIntervals), layout, bulk);
     a.ring_layout = layout;
     a.ring_bulk = bulk;
     ABHSF_CUDA(cudaMemsetAsync(a.dev_status.get(), 0, sizeof(int), st));
@@ -1816,7 +1830,7 @@ void prepare_batch(abhsf_batch& b, cudaStream_t st)
                     beside bs;
                     batch_launch(bs, b, xs_d.get(), ys_d.get(), st, true);
                 },
-                b.s, st, layout, bulk);
+                b.s, stream_clock(st, kIntervals), layout, bulk);
         b.layout = layout;
         b.bulk = bulk;
         ABHSF_CUDA(cudaMemsetAsync(b.dev_status.get(), 0, sizeof(int), st));
@@ -2027,6 +2041,24 @@ extern "C" void abhsf_test_set_hooks(int64_t drop_desc, uint32_t spin_limit)
 {
     abhsf::g_drop_desc = drop_desc < 0 ? -1 : drop_desc;
     abhsf::g_spin_limit = spin_limit;
+}
+
+extern "C" int32_t abhsf_test_pick_variant(int32_t s, const float* ms, int32_t disturbed, int32_t* layout, int32_t* bulk)
+{
+    struct script {
+        const float* ms;
+        int disturbed, launches = 0;
+        float now = 0.f, t[abhsf::kIntervals] = {};
+        void run(int l, int b) { now = ms[2 * l + b] * (launches++ == disturbed ? 10.f : 1.f); }
+    } sc{ms, disturbed};
+    struct clock {
+        script& sc;
+        void begin(int) {}
+        void end(int k) { sc.t[k] = sc.now; }
+        float ms(int k) { return sc.t[k]; }
+    };
+    abhsf::time_variants([&](int l, int b) { sc.run(l, b); }, s, clock{sc}, *layout, *bulk);
+    return sc.launches;
 }
 
 extern "C" int64_t abhsf_test_device_allocations(void) { return abhsf::dbuf_allocations().load(); }

@@ -32,6 +32,12 @@ ABHSF_API void abhsf_test_set_hooks(int64_t drop_desc, uint32_t spin_limit);
  * thread-safe with SpMVs of the same matrix. */
 ABHSF_API abhsf_status abhsf_test_ring_variant(abhsf_matrix* a, int32_t set, int32_t* layout, int32_t* bulk);
 
+/* The choice of a launch variant (block size s) with scripted times: variant
+ * (layout, bulk) takes ms[2 layout + bulk], launch number `disturbed` ten times as
+ * long (-1: none).  Returns the number of launches made.  Runs on the host. */
+ABHSF_API int32_t abhsf_test_pick_variant(int32_t s, const float* ms, int32_t disturbed, int32_t* layout,
+                                          int32_t* bulk);
+
 /* Device allocations (cudaMalloc or pool) the library has made since it was loaded,
  * so that a test can check that an entry point which promises to allocate
  * nothing keeps that promise. */
