@@ -1093,7 +1093,8 @@ void prepare_stream(abhsf_matrix& a, float avg, cudaStream_t st)
     std::vector<uint32_t> selrow_h(ns);
     for (int64_t k = 0; k < ns; ++k)
         selrow_h[k] = sel[k].first;
-    scratch<uint32_t> selrow(ns, st), sq(R, st), sq2(R, st), cq(E / kChainMin + 1, st), skey(R, st), skey2(R, st);
+    const int64_t L = std::min(R, E);  // rows with elements, at most: far fewer than R where block rows hold a few
+    scratch<uint32_t> selrow(ns, st), sq(L, st), sq2(L, st), cq(E / kChainMin + 1, st), skey(L, st), skey2(L, st);
     scratch<int64_t> seg_d(nseg + 1, st), begin_d(nseg + 1, st), first_d(nseg + 1, st), found(2, st), rstart(R + 1, st),
         slot0(R, st);
     ABHSF_CUDA(cudaMemcpyAsync(selrow.get(), selrow_h.data(), ns * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
@@ -1110,7 +1111,7 @@ void prepare_stream(abhsf_matrix& a, float avg, cudaStream_t st)
             ++kb;
         ABHSF_CUDA(cub::DeviceSelect::If(nullptr, b1, all, sq.get(), found.get(), R, is_sliced{cnt.get()}, st));
         ABHSF_CUDA(cub::DeviceSelect::If(nullptr, b2, all, cq.get(), found.get() + 1, R, is_chain{cnt.get()}, st));
-        ABHSF_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, b3, skey.get(), skey2.get(), sq.get(), sq2.get(), R, 0, kb,
+        ABHSF_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, b3, skey.get(), skey2.get(), sq.get(), sq2.get(), L, 0, kb,
                                                    st));
         ABHSF_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, b4, cnt.get(), rstart.get(), R, st));
         scratch<uint8_t> tmp(std::max(std::max(b1, b2), std::max(b3, b4)), st);

@@ -198,3 +198,18 @@ def test_the_reader_gets_what_the_library_keeps(gpu, tmp_path):
         del fill
         torch.cuda.empty_cache()
     assert all(torch.equal(a, b) for a, b in zip(want, got))
+
+
+def test_scratch_of_block_rows_with_one_element(gpu):
+    """200,000 block rows of 64 rows and one element each: the build's scratch
+    is 20 bytes a row (counts, row starts, slots), what goes with the rows that
+    hold elements comes on top (here 1/64 of them)."""
+    k = 200_000
+    rows = np.arange(k, dtype=np.int64) * 640 + 3
+    cols = np.random.default_rng(1).integers(0, 1000, k)
+    trim_device_memory()
+    A = AbhsfMatrix.from_elements(rows, cols, np.ones(k), 640 * k, 1000, block_size=64)
+    assert A.slices()["block_rows"] == k
+    A.release()
+    back = trim_device_memory()
+    assert 20 * 64 * k <= back <= 30 * 64 * k
