@@ -8,9 +8,12 @@
 //
 // The pool keeps at most kPoolKept bytes that nobody uses: its release threshold
 // (CUDA gives back what the pool holds above it at the next synchronisation) is
-// moved along with the bytes in use.  All that is unused is given back when an
-// allocation of the library fails and when the caller asks for it
-// (abhsf_trim_device_memory): nobody else in the process can take it otherwise.
+// moved along with the bytes in use.  The driver takes unused memory out of the
+// pool where another allocation of the process finds no other (a torch.empty of
+// 256 MB more than what is free, 1.7 GB unused here: it succeeds).  What it does
+// not take is given back when an allocation of the library fails, and all of it
+// when the caller asks (abhsf_trim_device_memory): other processes cannot have it
+// otherwise.
 //
 // Both limits from a build with one product of 60M elements, which needs 2 GB of
 // scratch (ms, in a new process and then again and again, B200):
@@ -274,15 +277,6 @@ void settle_released() noexcept
         if (any)
             settle(dev);
     }
-}
-
-bool trim_unused()
-{
-    int dev = 0;
-    device_pool* p = cudaGetDevice(&dev) == cudaSuccess ? pool_of(dev) : nullptr;
-    if (p)
-        trim(*p, dev);
-    return p != nullptr;
 }
 
 }  // namespace abhsf

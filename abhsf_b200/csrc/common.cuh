@@ -78,22 +78,6 @@ void* device_alloc(size_t bytes, device_block& block);
 void device_free(void* ptr, const device_block& block) noexcept;
 // Waits for the device where a dbuf was freed, and gives its memory back.
 void settle_released() noexcept;
-// Gives the current device's unused pool memory back (true where there is a pool).
-bool trim_unused();
-
-// Runs an allocation that is not the pool's own, a second time without the
-// pool's unused memory where the first found none left.
-template <typename F>
-void alloc_checked(F&& f, const char* what)
-{
-    cudaError_t e = f();
-    if (e == cudaErrorMemoryAllocation) {
-        cudaGetLastError();
-        if (trim_unused())
-            e = f();
-    }
-    cuda_check(e, what);
-}
 
 // Owning device allocation of a handle: usable on any stream at once, set aside
 // when freed until settle_released.

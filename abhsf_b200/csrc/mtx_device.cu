@@ -412,8 +412,7 @@ class sbuf {
   public:
     sbuf(size_t count, cudaStream_t st) : st_(st)
     {
-        alloc_checked([&] { return cudaMallocAsync(reinterpret_cast<void**>(&p_), std::max<size_t>(count, 1) * sizeof(T), st); },
-                      "cudaMallocAsync");
+        ABHSF_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&p_), std::max<size_t>(count, 1) * sizeof(T), st));
         dbuf_allocations().fetch_add(1, std::memory_order_relaxed);
     }
     ~sbuf() { cudaFreeAsync(p_, st_); }
@@ -463,9 +462,9 @@ void host_fallback(const char* path, cudaStream_t st, abhsf_coo_device& out)
     out.stored_triangle = h.stored_triangle;
     out.host_parsed = h.nnz;
     const size_t k = (size_t)std::max<int64_t>(h.nnz, 1);
-    alloc_checked([&] { return cudaMalloc(&out.rows, k * sizeof(int64_t)); }, "cudaMalloc");
-    alloc_checked([&] { return cudaMalloc(&out.cols, k * sizeof(int64_t)); }, "cudaMalloc");
-    alloc_checked([&] { return cudaMalloc(&out.vals, k * sizeof(double)); }, "cudaMalloc");
+    ABHSF_CUDA(cudaMalloc(&out.rows, k * sizeof(int64_t)));
+    ABHSF_CUDA(cudaMalloc(&out.cols, k * sizeof(int64_t)));
+    ABHSF_CUDA(cudaMalloc(&out.vals, k * sizeof(double)));
     if (h.nnz > 0) {
         ABHSF_CUDA(cudaMemcpyAsync(out.rows, h.rows, h.nnz * sizeof(int64_t), cudaMemcpyHostToDevice, st));
         ABHSF_CUDA(cudaMemcpyAsync(out.cols, h.cols, h.nnz * sizeof(int64_t), cudaMemcpyHostToDevice, st));
@@ -586,9 +585,9 @@ void read_mtx_device(const char* path, cudaStream_t st, abhsf_coo_device& out)
         if (hd.nnz > 0)
             fail(ABHSF_ERROR_INVALID_VALUE, "could not read matrix element (fewer entries than declared)");
         out.stored_triangle = hd.symmetry == ABHSF_SYMMETRY_GENERAL ? 0 : 2;
-        alloc_checked([&] { return cudaMalloc(&out.rows, sizeof(int64_t)); }, "cudaMalloc");
-        alloc_checked([&] { return cudaMalloc(&out.cols, sizeof(int64_t)); }, "cudaMalloc");
-        alloc_checked([&] { return cudaMalloc(&out.vals, sizeof(double)); }, "cudaMalloc");
+        ABHSF_CUDA(cudaMalloc(&out.rows, sizeof(int64_t)));
+        ABHSF_CUDA(cudaMalloc(&out.cols, sizeof(int64_t)));
+        ABHSF_CUDA(cudaMalloc(&out.vals, sizeof(double)));
         return;
     }
     // the lines
@@ -710,12 +709,9 @@ void read_mtx_device(const char* path, cudaStream_t st, abhsf_coo_device& out)
     const int64_t kept = select_flagged(flag.get(), L, idx.get(), st);
     out.nnz = kept;
     const size_t k = (size_t)std::max<int64_t>(kept, 1);
-    alloc_checked([&] { return cudaMallocAsync(reinterpret_cast<void**>(&out.rows), k * sizeof(int64_t), st); },
-                  "cudaMallocAsync");
-    alloc_checked([&] { return cudaMallocAsync(reinterpret_cast<void**>(&out.cols), k * sizeof(int64_t), st); },
-                  "cudaMallocAsync");
-    alloc_checked([&] { return cudaMallocAsync(reinterpret_cast<void**>(&out.vals), k * sizeof(double), st); },
-                  "cudaMallocAsync");
+    ABHSF_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&out.rows), k * sizeof(int64_t), st));
+    ABHSF_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&out.cols), k * sizeof(int64_t), st));
+    ABHSF_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&out.vals), k * sizeof(double), st));
     if (kept > 0) {
         k_gather<<<grid_for(kept), 256, 0, st>>>(kept, idx.get(), ri.get(), ci.get(), vi.get(), out.rows, out.cols,
                                                  out.vals);

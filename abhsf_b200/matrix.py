@@ -270,7 +270,8 @@ class AbhsfMatrix:
 
 def trim_device_memory() -> int:
     """Gives back the device memory that the library keeps for its next calls (up
-    to 2 GB a device), so that other allocators can have it: how many bytes."""
+    to 2 GB a device), so that other processes can have it (this one's allocations
+    get it without the call): how many bytes."""
     n = C.c_int64()
     capi.check(capi.lib.abhsf_trim_device_memory(C.byref(n)))
     return n.value

@@ -324,10 +324,10 @@ ABHSF_API abhsf_status abhsf_release(abhsf_matrix* a);
 
 /* Gives back the device memory that the library keeps for its next calls, on
  * every device it has used, after waiting for the device; handles in use stay as
- * they are.  For a program that is done building and whose next allocations
- * come from elsewhere.  bytes (may be NULL): how much it was.  The library does
- * this by itself where an allocation of its own finds no memory.  No reference
- * counterpart. */
+ * they are.  For a program that is done building and shares the device with other
+ * processes: allocations of its own process get that memory without the call,
+ * the driver takes it where it finds no other.  bytes (may be NULL): how much it
+ * was.  No reference counterpart. */
 ABHSF_API abhsf_status abhsf_trim_device_memory(int64_t* bytes);
 
 /* Format statistics, including the reference's per-scheme storage totals. */

@@ -8,7 +8,7 @@ import time
 import numpy as np
 import pytest
 
-from abhsf_b200 import AbhsfMatrix, capi, cg, cg_mixed, read_mtx_device, trim_device_memory
+from abhsf_b200 import AbhsfMatrix, capi, cg, cg_mixed, trim_device_memory
 from abhsf_b200 import workloads as W
 from oracle import oracle
 
@@ -178,26 +178,20 @@ def test_unused_memory_is_given_back(gpu):
     assert np.array_equal(y.cpu().numpy(), _reference(coo, x))
 
 
-def test_the_reader_gets_what_the_library_keeps(gpu, tmp_path):
-    """The device reader's memory does not come from the library's pool; on a
-    card that others have filled it gets what the pool holds unused."""
+def test_other_allocations_get_what_the_library_keeps(gpu):
+    """Memory that the library keeps unused is there for the process's other
+    allocations: one of more than what is reported free succeeds."""
     import torch
-    coo = W.random_uniform(30000, 30000, 400_000, seed=75)
-    path = tmp_path / "a.mtx"
-    with open(path, "w") as f:
-        f.write("%%%%MatrixMarket matrix coordinate real general\n%d %d %d\n" % (coo.m, coo.n, coo.nnz))
-        f.writelines("%d %d %.17g\n" % (r + 1, c + 1, v) for r, c, v in zip(coo.rows, coo.cols, coo.vals))
-    want = [t.cpu() for t in read_mtx_device(str(path))[:3]]
     big = W.random_uniform(400000, 400000, 6_000_000, seed=76)
+    trim_device_memory()
     AbhsfMatrix.from_elements(big.rows, big.cols, big.vals, big.m, big.n).release()
     torch.cuda.empty_cache()
-    fill = torch.empty(torch.cuda.mem_get_info()[0] - (24 << 20), dtype=torch.uint8, device="cuda")
     try:
-        got = [t.cpu() for t in read_mtx_device(str(path))[:3]]
+        t = torch.empty(torch.cuda.mem_get_info()[0] + (128 << 20), dtype=torch.uint8, device="cuda")
+        assert t.data_ptr()
+        del t
     finally:
-        del fill
         torch.cuda.empty_cache()
-    assert all(torch.equal(a, b) for a, b in zip(want, got))
 
 
 def test_scratch_of_block_rows_with_one_element(gpu):
