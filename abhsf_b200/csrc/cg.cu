@@ -357,13 +357,12 @@ void dot(const T* a, const T* b, int64_t n, double* partial, cudaStream_t st, co
     launch_after(aligned16(a) && aligned16(b) ? k_dot<T, true> : k_dot<T, false>, st, n, a, b, partial, done);
 }
 
-// p = r, Ap = 0 and the state from r . r: the start of a CG recurrence.
+// p = r and the state from r . r: the start of a CG recurrence.
 template <typename T>
 void cg_start(cg_work<T>& w, int64_t n, cg_state* st_d, double* partial, double tol2, int max_iters,
               cudaStream_t cs)
 {
     ABHSF_CUDA(cudaMemcpyAsync(w.p.get(), w.r.get(), n * sizeof(T), cudaMemcpyDeviceToDevice, cs));
-    ABHSF_CUDA(cudaMemsetAsync(w.ap.get(), 0, n * sizeof(T), cs));
     dot<T>(w.r.get(), w.r.get(), n, partial, cs);
     k_cg_init<<<1, kRedThreads, 0, cs>>>(partial, st_d, tol2, max_iters);
     ABHSF_CUDA(cudaGetLastError());
@@ -376,7 +375,7 @@ class cg_graph {
   public:
     // partial: 2 kRedBlocks
     cg_graph(const abhsf_matrix& a, T* x, cg_work<T>& w, int64_t n, cg_state* st_d, double* partial, cudaStream_t cs)
-        : heeds_(spmv_sets_y(a))
+        : heeds_(spmv_sets_y(a)), ap_(w.ap.get()), n_(n)
     {
         ABHSF_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&seen_), 2 * sizeof(cg_state), cudaHostAllocDefault));
         cudaGraph_t graph = nullptr;
@@ -410,8 +409,14 @@ class cg_graph {
     // Replays chunks until the state says done; returns the iteration count.
     // Where a chunk after the last is a no-op throughout, it is queued before
     // the state is read, so that the GPU does not wait for the host.
+    // An SpMV that adds finds Ap = 0, left by the residual kernel of the
+    // iteration before -- but behind the last iteration of a recurrence the
+    // chunk's remaining products still add onto it, and a recurrence that is
+    // resumed (the mixed solver's) must not start from that.
     int run(const cg_state* st_d, cudaStream_t cs)
     {
+        if (!heeds_)
+            ABHSF_CUDA(cudaMemsetAsync(ap_, 0, n_ * sizeof(T), cs));
         for (int k = 0;; ++k) {
             if (heeds_ || k > 0)
                 ABHSF_CUDA(cudaGraphLaunch(exec_, cs));
@@ -457,6 +462,8 @@ class cg_graph {
     }
 
     const bool heeds_;  // the SpMV sets y and heeds the done flag
+    T* const ap_;
+    const int64_t n_;
     cg_state* seen_ = nullptr;  // pinned: the state after the last two chunks
     cudaEvent_t ev_[2] = {nullptr, nullptr};
     cudaGraphExec_t exec_ = nullptr;
