@@ -429,7 +429,14 @@ __device__ __forceinline__ void seq_block_row(const tiles_view& A, const void* x
     __syncwarp();
 }
 
-template <int S, int VT, bool B = false>
+// BEHIND: queued behind the product's chains, for whose end one thread waits.  A
+// kernel of its own: with that wait after the loop the loop is compiled slower
+// (banded matrix of 200,000 rows, 121 elements each, s = 256: bf16 541 us against
+// 460, f32 431 against 345; of a million rows, 17 each, s = 16: FP64 115 against
+// 103, f32 111 against 99).
+// Eight CTAs an SM at s = 16 (64 registers a thread, no spill; six leave 80): tiled
+// mixture FP64 305 -> 278 us, bf16 274 -> 254, f32 256 either way.
+template <int S, int VT, bool B, bool BEHIND>
 __global__ void __launch_bounds__(kWarps * 32, S == 16 && !B ? 8 : kMinCtasPerSm) k_spmv_seq(seq_args P)
 {
     using T = typename seq_t<VT>::T;
@@ -452,7 +459,8 @@ __global__ void __launch_bounds__(kWarps * 32, S == 16 && !B ? 8 : kMinCtasPerSm
         }
         k = __shfl_sync(kFull, next, 0);
     }
-    beside_end();
+    if constexpr (BEHIND)
+        beside_end();
 }
 
 // (the work counter is cleared by the caller before the product's first kernel:
@@ -465,11 +473,12 @@ void launch_seq(beside& bs, const abhsf_matrix& a, const uint32_t* rows, int64_t
     int dev = 0, nsm = 0, per_sm = 0;
     ABHSF_CUDA(cudaGetDevice(&dev));
     ABHSF_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    ABHSF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_spmv_seq<S, VT>, kWarps * 32, 0));
+    const auto kern = bs.any ? k_spmv_seq<S, VT, false, true> : k_spmv_seq<S, VT, false, false>;
+    ABHSF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kWarps * 32, 0));
     seq_args P{a.view(), rows, nrows, a.tree_counter.get(), x, y, nullptr, nullptr, nullptr, nullptr};
     const int64_t ctas = (nrows + kWarps - 1) / kWarps;
     const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(ctas, (int64_t)nsm * std::max(per_sm, 1)));
-    launch_beside(bs, k_spmv_seq<S, VT, false>, grid, kWarps * 32, 0, st, P);
+    launch_beside(bs, kern, grid, kWarps * 32, 0, st, P);
 }
 
 template <int VT>
@@ -495,14 +504,13 @@ void seq_any(const abhsf_matrix& a, const void* x, void* y, cudaStream_t st)
     const bool slices = a.dc_rows > 0 && a.sum_order == ABHSF_SUM_REFERENCE && a.s != 32 && a.s != 64;
     beside bs;
     dc_plan p;
-    const uint32_t* rows = a.tree_rows.get();
-    int64_t nrows = a.tree_nrows;
-    ABHSF_CUDA(cudaMemsetAsync(a.tree_counter.get(), 0, sizeof(unsigned int), st));
+    const uint32_t* rows = slices ? a.seq_rows.get() : a.tree_rows.get();
+    const int64_t nrows = slices ? a.seq_nrows : a.tree_nrows;
+    if (nrows > 0)
+        ABHSF_CUDA(cudaMemsetAsync(a.tree_counter.get(), 0, sizeof(unsigned int), st));
     if (slices) {
         p = plan_of(a);
         slices_begin(bs, a, p, x, 1, y, 1, st);
-        rows = a.seq_rows.get();
-        nrows = a.seq_nrows;
     }
     if (a.value_type == ABHSF_VALUE_F64)
         launch_seq_vt<ABHSF_VALUE_F64>(bs, a, rows, nrows, x, y, st);
@@ -575,7 +583,7 @@ void launch_batch_seq(beside& bs, const abhsf_batch& b, const double* const* xs,
     int dev = 0, nsm = 0, per_sm = 0;
     ABHSF_CUDA(cudaGetDevice(&dev));
     ABHSF_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    auto kern = k_spmv_seq<S, ABHSF_VALUE_F64, true>;
+    const auto kern = bs.any ? k_spmv_seq<S, ABHSF_VALUE_F64, true, true> : k_spmv_seq<S, ABHSF_VALUE_F64, true, false>;
     ABHSF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kWarps * 32, 0));
     seq_args P{};
     P.nrows = b.seq_nitems;
