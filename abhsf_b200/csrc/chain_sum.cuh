@@ -95,6 +95,32 @@ __device__ __forceinline__ T run_segment(T a, const T (&p)[L], bool& inside, boo
     return a;
 }
 
+// The exponent of v as an integer that compares like |v| (inf and NaN above all).
+template <typename T>
+__device__ __forceinline__ uint32_t exponent(T v)
+{
+    using B = typename bits_of<T>::B;
+    return (B::key(v) >> B::kKeyMant) & (uint32_t)B::kExpMax;
+}
+
+// Whether few of a group's segments will cross a binade, by a sample of its
+// products (a quarter of each lane's): they are of one sign (the sum doubles a few
+// times at most), or y is 2^kAbove times as large.  Sums near zero of products of
+// both signs would have most segments run again.
+template <int kAbove, int L, typename T>
+__device__ __forceinline__ bool calm(T y, const T (&p)[L])
+{
+    uint32_t most = 0, signs = 0;
+#pragma unroll
+    for (int i = 1; i < L; i += 4) {
+        const uint32_t e = exponent(p[i]);
+        most = max(most, e);
+        signs |= e == 0 ? 0u : p[i] < T(0) ? 1u : 2u;
+    }
+    return __reduce_or_sync(0xffffffffu, signs) != 3u ||
+           exponent(y) >= __reduce_max_sync(0xffffffffu, most) + (uint32_t)kAbove;
+}
+
 // p[0 .. L-1] added onto a in turn, and nothing else.
 template <int L, typename T>
 __device__ __forceinline__ T add_segment(T a, const T (&p)[L])
@@ -107,11 +133,11 @@ __device__ __forceinline__ T add_segment(T a, const T (&p)[L])
 
 // Adds the products of 32 / STRIDE segments of L each onto y, in order: lane
 // STRIDE g + h holds segment g of chain h in p (STRIDE chains at once, each
-// lane of a chain holding its y).  False, y unchanged, where more than kAgain
-// segments would have to be run again one after another: the caller adds in
-// turn.
+// lane of a chain holding its y).  Returns how many steps of running segments
+// again it took; -1, y unchanged, where more than kAgain would have to be run one
+// after another: the caller adds in turn.
 template <int STRIDE, int L, typename T>
-__device__ __forceinline__ bool sum_group(T& y, const T (&p)[L], int lane)
+__device__ __forceinline__ int sum_group(T& y, const T (&p)[L], int lane)
 {
     using B = typename bits_of<T>::B;
     using I = typename B::I;
@@ -143,7 +169,7 @@ __device__ __forceinline__ bool sum_group(T& y, const T (&p)[L], int lane)
     T end = run_segment<L>(start, p, inside, tie);
     const unsigned outside = __ballot_sync(full, !inside);
     if (__any_sync(full, __popc(outside & mine) > kAgain))
-        return false;
+        return -1;
     const long long gap = (long long)B::bits(__shfl_up_sync(full, end, STRIDE)) - (long long)B::bits(start);
     const bool far = gap >= kFar || gap <= -kFar;
     int off = g > 0 && !far ? (int)gap : 0;  // spacings from the start to the true start
@@ -163,10 +189,10 @@ __device__ __forceinline__ bool sum_group(T& y, const T (&p)[L], int lane)
         const T moved = B::value(B::bits(end) + (I)off);  // the true end
         if (bad == 0) {
             y = __shfl_sync(full, moved, 32 - STRIDE + h);
-            return true;
+            return again;
         }
         if (again == kAgain)
-            return false;
+            return -1;
         // this chain's first segment that the rule does not cover, from its
         // true start; the later segments' distances move by as much as its end did
         const T again_end = add_segment<L>(__shfl_up_sync(full, moved, STRIDE), p);
@@ -174,7 +200,7 @@ __device__ __forceinline__ bool sum_group(T& y, const T (&p)[L], int lane)
         const int b = bad & mine ? (__ffs(bad & mine) - 1) / STRIDE : g;
         const int more = __shfl_sync(full, shift < kFar && shift > -kFar ? (int)shift - off : INT_MIN, b * STRIDE + h);
         if (__any_sync(full, (bad & mine) && more == INT_MIN))
-            return false;
+            return -1;
         if (bad & mine) {
             first = b;
             if (g == b) {

@@ -56,7 +56,6 @@ constexpr int kChainCtasPerSm = 4;  // register bound of the chain kernel (128 a
 constexpr int kChainGridPerSm = 1;  // chain CTAs per SM in the grid: the rest of the SM is left to the others
 constexpr int kSliceGridPerSm = 3;  // sliced-row CTAs per SM beside chains
 constexpr int kChainGroup = 512;  // chain: elements a warp sums at a time, 16 a lane
-constexpr int kChainTurn = 4;     // chain: a last group of so few segments of 16 is added in turn
 constexpr int kMmCols = 4;        // columns a warp of the SpMM kernels serves
 constexpr int kMmWarps = 2, kMmCtas = 10;  // sliced-row SpMM: warps a CTA (small ones fit beside the chains), CTAs an SM
 constexpr int kMmAhead = 2;       // steps a lane of the sliced-row SpMM loads at a time
@@ -156,53 +155,6 @@ __device__ __forceinline__ bool begin(const dc_args& P)
         asm volatile("griddepcontrol.wait;" ::: "memory");
     beside_begin();
     return P.skip && *reinterpret_cast<const volatile int*>(P.skip) != 0;
-}
-
-// Eight consecutive values from shared memory (16-byte aligned), in two or
-// four 16-byte loads.
-__device__ __forceinline__ void load8(const double* q, double (&t)[8])
-{
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        const double2 u = reinterpret_cast<const double2*>(q)[k];
-        t[2 * k] = u.x;
-        t[2 * k + 1] = u.y;
-    }
-}
-__device__ __forceinline__ void load8(const float* q, float (&t)[8])
-{
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-        const float4 u = reinterpret_cast<const float4*>(q)[k];
-        t[4 * k] = u.x;
-        t[4 * k + 1] = u.y;
-        t[4 * k + 2] = u.z;
-        t[4 * k + 3] = u.w;
-    }
-}
-
-// Adds nseg runs of 16 products, `stride` values apart in shared memory, onto
-// run one after another (every lane the same: broadcast loads).  Eight
-// products are loaded while the eight before them are added, so that nothing
-// but the adds lies on the chain.
-template <typename T>
-__device__ __forceinline__ T add_in_turn(T run, const T* q, int stride, int nseg)
-{
-    T t[8], u[8];
-    load8(q, t);
-#pragma unroll 1
-    for (int b = 0; b < nseg; ++b, q += stride) {
-        load8(q + 8, u);
-#pragma unroll
-        for (int k = 0; k < 8; ++k)
-            run = dadd(run, t[k]);
-        if (b + 1 < nseg)
-            load8(q + stride, t);
-#pragma unroll
-        for (int k = 0; k < 8; ++k)
-            run = dadd(run, u[k]);
-    }
-    return run;
 }
 
 // Sliced rows.  A warp sums its dealt slices one after another, each lane
@@ -322,6 +274,81 @@ __device__ __forceinline__ void load16(const V* q, V (&t)[16])
     }
 }
 
+// ... and back.
+template <typename V>
+__device__ __forceinline__ void store16(V* q, const V (&t)[16])
+{
+    constexpr int N = 16 / (int)sizeof(V);
+#pragma unroll
+    for (int k = 0; k < 16 / N; ++k) {
+        union {
+            uint4 u;
+            V v[N];
+        } c;
+#pragma unroll
+        for (int i = 0; i < N; ++i)
+            c.v[i] = t[N * k + i];
+        reinterpret_cast<uint4*>(q)[k] = c.u;
+    }
+}
+
+// Eight consecutive values from shared memory (16-byte aligned), in two or
+// four 16-byte loads.
+__device__ __forceinline__ void load8(const double* q, double (&t)[8])
+{
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const double2 u = reinterpret_cast<const double2*>(q)[k];
+        t[2 * k] = u.x;
+        t[2 * k + 1] = u.y;
+    }
+}
+__device__ __forceinline__ void load8(const float* q, float (&t)[8])
+{
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        const float4 u = reinterpret_cast<const float4*>(q)[k];
+        t[4 * k] = u.x;
+        t[4 * k + 1] = u.y;
+        t[4 * k + 2] = u.z;
+        t[4 * k + 3] = u.w;
+    }
+}
+
+// Adds nseg runs of 16 products, `stride` values apart in shared memory, onto
+// run one after another (every lane the same: broadcast loads).  Eight
+// products are loaded while the eight before them are added, so that nothing
+// but the adds lies on the chain; eight runs at a time (one at a time a lone row
+// of 60,000 took 152 us in f32, 137 so).
+template <typename T>
+__device__ __forceinline__ T add_in_turn(T run, const T* q, int stride, int nseg)
+{
+    T t[8], u[8];
+    load8(q, t);
+    auto add_run = [&](bool more) {
+        load8(q + 8, u);
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+            run = dadd(run, t[k]);
+        q += stride;
+        if (more)
+            load8(q, t);
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+            run = dadd(run, u[k]);
+    };
+    int b = nseg;
+#pragma unroll 1
+    for (; b > 8; b -= 8)
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+            add_run(true);
+#pragma unroll 1
+    for (; b > 0; --b)
+        add_run(b > 1);
+    return run;
+}
+
 // A chain as a warp walks it, kChainGroup elements at a time.
 template <typename T, typename V>
 struct chain_pos {
@@ -349,19 +376,26 @@ __device__ __forceinline__ void chain_at(const dc_args& P, const dc_slice& sl, c
 // The chains: one warp per row, the row's elements in order (each word the
 // absolute column), 512 at a time.  Lane l holds elements 16 l .. 16 l + 15 of
 // a group: its segment of chain::sum_group, which adds the group in order
-// without a chain of 512 additions (8.2 cycles each in FP64).  Where that gives
-// up -- a sum that keeps crossing binades, near zero -- every lane adds the
-// products in turn from shared memory.  A warp's rows form one stream of
+// without a chain of 512 additions (8.2 cycles each in FP64, 4 in f32).  Where
+// that would not pay -- few segments, or a sum near zero that keeps crossing
+// binades (chain::calm) -- or gives up, every lane adds the products in turn
+// from shared memory.  A warp's rows form one stream of
 // groups: while one is summed, the values and gathered x of the next are on
 // their way into the other half of the warp's shared buffer (cp.async: they
 // take no registers), and so are the words of the one after, whichever rows
 // they belong to.  The places of a group past its row's end hold -0, which
 // leaves any sum as it is.
-// Bound by latency: one warp issues 408 instructions a group, 4.8 cycles each
-// (a lone row of 98,304 ones 0.49 -> 0.20 ms, of N(0,1) products 0.49 -> 0.37,
-// against additions in turn).  R-MAT scale 22 (chains and sliced rows
-// together) 0.574 -> 0.357 ms, the 256-matrix batch 0.861 -> 0.790 ms.  Two
-// CTAs an SM, or the sliced rows two, were slower on the batch (0.87 ms).
+// Bound by latency: one warp issues 408 instructions a group, 4.8 cycles each,
+// and some 500 cycles more for a segment run again.  So the time depends on the
+// values.  R-MAT scale 22 (chains and sliced rows together; us, against additions
+// in turn): N(0,1) x U[-1,1] products onto a y that has grown 570 -> 370, onto
+// y = 0 583 -> 580 to 627, all products positive onto y = 0 581 -> 415; f32 442 ->
+// 310 to 340, 456 -> 402, 457 -> 368.  A lone row of 60,000: FP64 229 -> 90, onto 0
+// 241 -> 183; f32 136 -> 81, 149 -> 162.  200 rows of 20,000: FP64 118 -> 87, onto 0
+// 131 -> 139; f32 63 -> 66, 75 -> 88.  Rows of 260 to 600: 20 to 40% off either way.
+// Without the two rules (segments, calm) a y = 0 took 604 to 635 on R-MAT scale
+// 22 and 153 (f32 111) on the 200 rows.  Two CTAs an SM, or the sliced rows two,
+// were slower on the 256-matrix batch (0.87 ms against 0.79).
 template <int S, int VT, bool B>
 __global__ void __launch_bounds__(32 * kChainWarps, kChainCtasPerSm) k_spmv_chains(dc_args P)
 {
@@ -369,6 +403,12 @@ __global__ void __launch_bounds__(32 * kChainWarps, kChainCtasPerSm) k_spmv_chai
     using V = typename vt_of<VT>::V;
     constexpr int L = 16, G = kChainGroup;
     static_assert(G == 32 * L, "a segment a lane");
+    // A group goes in turn at once where that is faster: up to kTurn segments (in
+    // f32 an addition takes half as long), or where the sum is not kAbove binades
+    // above the products (2 fewer: 200 rows of 20,000 onto 0 146 -> 152 us; 1 more:
+    // onto a y that has grown 85 -> 92) unless the row's group before was settled
+    // without a segment run again.
+    constexpr int kTurn = sizeof(T) == 8 ? 12 : 19, kAbove = sizeof(T) == 8 ? 4 : 5;
     // segments 16 bytes apart, so that the lanes' 16-byte reads meet no bank twice
     constexpr int STX = L + 16 / (int)sizeof(T), STV = L + 16 / (int)sizeof(V);
     extern __shared__ __align__(16) uint8_t chain_smem[];
@@ -444,7 +484,7 @@ __global__ void __launch_bounds__(32 * kChainWarps, kChainCtasPerSm) k_spmv_chai
     if (ahead.si < s1)
         load_words();
     T run = T(0);
-    int half = 0;
+    int half = 0, again = -1;  // again: segments run again in the row's group before (-1: added in turn)
 #pragma unroll 1
     for (;;) {
         cur = nxt;
@@ -484,11 +524,12 @@ __global__ void __launch_bounds__(32 * kChainWarps, kChainCtasPerSm) k_spmv_chai
                 p[i] = i < have ? p[i] : T(-0.0);
         }
         const int nseg = min(32, (cur.len - cur.b0 + L - 1) / L);
-        // a short last group is as fast in turn
-        if (nseg <= kChainTurn || !chain::sum_group<1, L>(run, p, lane)) {
-#pragma unroll
-            for (int i = 0; i < L; ++i)
-                xs[i] = p[i];
+        if (cur.b0 == 0)
+            again = -1;
+        if (nseg <= kTurn || !(again == 0 || chain::calm<kAbove>(run, p)) ||
+            (again = chain::sum_group<1, L>(run, p, lane)) < 0) {
+            again = -1;
+            store16(xs, p);
             __syncwarp();
             run = add_in_turn(run, xb + half * 32 * STX, STX, nseg);
         }
@@ -643,7 +684,7 @@ __global__ void __launch_bounds__(32 * kChainWarps, kChainCtasPerSm) k_spmm_chai
                 v[j] = ld_stream(Vv + min(b0 + G + e0 + kMmCols * j, len - 1));
                 w[j] = ld_stream(W + min(b0 + 2 * G + e0 + kMmCols * j, len - 1));
             }
-            if (!chain::sum_group<kMmCols, L>(run, p, lane)) {
+            if (chain::sum_group<kMmCols, L>(run, p, lane) < 0) {
                 const int nseg = min(8, (len - b0 + L - 1) / L);
 #pragma unroll 1
                 for (int s = 0; s < nseg; ++s) {
