@@ -249,6 +249,7 @@ struct abhsf_matrix {
     abhsf::dbuf<int64_t> dc_cwbeg;
     int dc_cwarps = 0;
     int64_t dc_elements = 0, dc_rows = 0, dc_slots = 0, dc_lane_records = 0;
+    int64_t dc_steps = 0, dc_longest = 0;  // steps of the sliced rows' slices: in all, of the longest
     float dc_avg = 0.f;                  // largest mean elements per tile of a slice block row (0: none)
     abhsf::dbuf<int> dev_status;  // ABHSF_DEVSTAT_* bits set by kernels
     // staging for abhsf_spmv_host

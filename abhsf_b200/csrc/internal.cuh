@@ -131,9 +131,10 @@ struct dc_plan {
     const uint8_t* csched = nullptr;
     const int64_t* cwbeg = nullptr;
     int cwarps = 0;
+    int64_t steps = 0, longest = 0;  // SpMM: steps of the slices, in all and of the longest
 };
 dc_plan plan_of(const abhsf_matrix& a);
-// cols > 1 (FP64 only): Y += A X over that many columns in one launch, each
+// cols > 1 (FP64 only): Y += A X over that many columns, each
 // column bitwise its SpMV.
 void slices_begin(beside& bs, const abhsf_matrix& a, const dc_plan& p, const void* x, int64_t ldx, void* y,
                   int64_t ldy, cudaStream_t st, int cols = 1);

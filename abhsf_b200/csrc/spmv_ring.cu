@@ -2014,7 +2014,7 @@ bool spmm_f64_ring(const abhsf_matrix& a, int k, const double* X, int64_t ldx, d
         else
             spmm_ring<64>(bs, a, k, X, ldx, Y, ldy, st);
     }
-    slices_begin(bs, a, p, X, ldx, Y, ldy, st, k);  // the slice rows, every column in one launch
+    slices_begin(bs, a, p, X, ldx, Y, ldy, st, k);  // the slice rows, all columns
     slices_end(bs, a, p, X, ldx, Y, ldy, st, k);
     return true;
 }

@@ -57,8 +57,9 @@ constexpr int kChainGridPerSm = 1;  // chain CTAs per SM in the grid: the rest o
 constexpr int kSliceGridPerSm = 3;  // sliced-row CTAs per SM beside chains
 constexpr int kChainGroup = 512;  // chain: elements a warp sums at a time, 16 a lane
 constexpr int kMmCols = 4;        // columns a warp of the SpMM kernels serves
-constexpr int kMmWarps = 2, kMmCtas = 10;  // sliced-row SpMM: warps a CTA (small ones fit beside the chains), CTAs an SM
-constexpr int kMmAhead = 2;       // steps a lane of the sliced-row SpMM loads at a time
+constexpr int kMmWide = 16;       // ... and of the sliced-row one where there are as many and no chains
+constexpr int kMmWarps = 2;       // sliced-row SpMM: warps a CTA (small ones fit beside the chains)
+constexpr int kMmCtas = 16, kMmLateCtas = 10;  // ... and CTAs an SM where warps count, and where latency does
 constexpr uint32_t kChain = 1u;   // dc_slice::geo: a one-row chain
 constexpr int kMidShift = 20;     // dc_slice::geo: matrix index of a batch
 constexpr int kLenBits = 8;       // lane record: row offset << kLenBits | (length - 1)
@@ -544,25 +545,36 @@ __global__ void __launch_bounds__(32 * kChainWarps, kChainCtasPerSm) k_spmv_chai
     beside_end();
 }
 
-// Y += A X over k > 1 columns (FP64), kMmCols = 4 of them a warp (blockIdx.x
-// names the four): one 32-byte sector of a row of X.  Lane (g, h) = (lane / 4,
-// lane % 4) keeps the sums of column h for rows g, g + 8, g + 16, g + 24 of
-// the slice and reads those rows' words and values itself (four lanes the same
-// address: a broadcast), so nothing is exchanged between lanes.  The next
-// kMmAhead steps' words and values are in flight while the gathers of the
-// current ones return.  Every (row, column) sum adds its products in the
-// row's column order from Y's value: column j of Y is bitwise the SpMV of
-// column j of X.
-// Bound by the latency of the gathers (eight a lane in flight); one launch
-// whatever k is.  R-MAT scale 18, 7 columns: passes of 4, 2 and 1 columns, each
-// with up to four gathers a lane in flight and column and value by shuffles,
-// took 415 us of kernel time, this 78 us (with the chains: 1,305 -> 98 us).
-template <int S>
-__global__ void __launch_bounds__(32 * kMmWarps, kMmCtas) k_spmm_slices(dc_args P)
+// Y += A X over k > 1 columns (FP64).  A unit of blockIdx.x is C columns of G R
+// of a slice's rows: 4 columns (one 32-byte sector of a row of X) of all 32, or
+// 16 (a whole line) of a quarter.  Lane (g, h) = (lane / C, lane % C) keeps the
+// sums of column h for rows g, g + G, g + 2 G, g + 3 G of them and reads those
+// rows' words and values itself (C lanes the same address: a broadcast), so
+// nothing is exchanged between lanes.  The next U steps' words and values are in
+// flight while the gathers of the current ones return.  Every (row, column) sum
+// adds its products in the row's column order from Y's value: column j of Y is
+// bitwise the SpMV of column j of X.
+// Beside chains, or where the longest slice takes longer than a warp's share of
+// all, bound by the latency of the gathers: ten CTAs an SM and eight gathers a
+// lane in flight.  R-MAT scale 18, 7 columns: passes of 4, 2
+// and 1 columns, each with up to four gathers a lane in flight and column and
+// value by shuffles, took 415 us of kernel time, this 78 us (with the chains:
+// 1,305 -> 98 us; 88 with sixteen CTAs instead of 85); scale 10, no chains, 16
+// columns 54 us against 87 the other way.
+// Else bound by the lines a gather touches (4 columns a warp: eight a
+// load, 16: two) and by the warps to hide them: sixteen CTAs (64 registers, 48 to
+// 64 bytes spilled), and 16 columns a warp where there are as many, a step at a
+// time.  3D Laplacian 120^3, 2 / 8 / 16 / 32 columns: 118 / 237 / 445 / 866 us with
+// ten CTAs and 4 columns a warp, 93 / 183 / 335 / 653 so (113 / 256 / 353 / 1,527
+// in passes of 2, 8, 16 and 32 columns before either).
+template <int S, int C, int CTAS>
+__global__ void __launch_bounds__(32 * kMmWarps, CTAS) k_spmm_slices(dc_args P)
 {
-    constexpr int R = kMmCols, U = kMmAhead;  // rows a lane (32 rows x 4 columns over 32 lanes); steps a round
+    constexpr int R = kMmCols, U = C == kMmWide ? 1 : 2;  // rows a lane; steps a round
+    constexpr int G = 32 / C, Q = C / R;                  // rows side by side; parts of a slice's 32 rows
+    static_assert(G * R * Q == 32, "a unit of the grid is G R rows by C columns");
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int g = lane / kMmCols, h = blockIdx.x * kMmCols + lane % kMmCols;
+    const int g = G * R * (blockIdx.x % Q) + lane / C, h = blockIdx.x / Q * C + lane % C;
     const int gw = blockIdx.y * kMmWarps + warp;
     beside_begin();
     if (gw >= P.warps || h >= P.cols)
@@ -582,7 +594,7 @@ __global__ void __launch_bounds__(32 * kMmWarps, kMmCtas) k_spmm_slices(dc_args 
         double v[U][R];
 #pragma unroll
         for (int i = 0; i < R; ++i) {
-            const int r = g + 8 * i;
+            const int r = g + G * i;
             const uint32_t rec = r < (int)sl.lanes ? P.A.lane[sl.meta + r] : 0u;
             len[i] = r < (int)sl.lanes ? (int)(rec & kLenMask) + 1 : 0;
             y[i] = Y + ((int64_t)sl.brow * S + (int64_t)(rec >> kLenBits)) * P.ldy;
@@ -592,14 +604,16 @@ __global__ void __launch_bounds__(32 * kMmWarps, kMmCtas) k_spmm_slices(dc_args 
         for (int u = 0; u < U; ++u)
 #pragma unroll
             for (int i = 0; i < R; ++i) {
-                w[u][i] = u < len[i] ? __ldg(W + 32 * u + 8 * i) : 0u;
-                v[u][i] = u < len[i] ? __ldg(Vv + 32 * u + 8 * i) : 0.0;
+                w[u][i] = u < len[i] ? __ldg(W + 32 * u + G * i) : 0u;
+                v[u][i] = u < len[i] ? __ldg(Vv + 32 * u + G * i) : 0.0;
             }
 #pragma unroll
         for (int i = 0; i < R; ++i)
             acc[i] = len[i] ? *y[i] : 0.0;
+        // the longest of the warp's rows is its first (all 32 lanes are here where Q > 1)
+        const int steps = Q > 1 ? __shfl_sync(0xffffffffu, len[0], 0) : (int)sl.steps;
 #pragma unroll 1
-        for (int k0 = 0; k0 < (int)sl.steps; k0 += U) {
+        for (int k0 = 0; k0 < steps; k0 += U) {
             double x[U][R];
 #pragma unroll
             for (int u = 0; u < U; ++u)
@@ -607,7 +621,7 @@ __global__ void __launch_bounds__(32 * kMmWarps, kMmCtas) k_spmm_slices(dc_args 
                 for (int i = 0; i < R; ++i) {
                     col[i] += w[u][i];
                     x[u][i] = k0 + u < len[i] ? __ldg(X + (int64_t)col[i] * P.ldx) : 0.0;
-                    w[u][i] = k0 + U + u < len[i] ? __ldg(W + 32 * (k0 + U + u) + 8 * i) : 0u;
+                    w[u][i] = k0 + U + u < len[i] ? __ldg(W + 32 * (k0 + U + u) + G * i) : 0u;
                 }
 #pragma unroll
             for (int u = 0; u < U; ++u)
@@ -615,7 +629,7 @@ __global__ void __launch_bounds__(32 * kMmWarps, kMmCtas) k_spmm_slices(dc_args 
                 for (int i = 0; i < R; ++i) {
                     if (k0 + u < len[i])
                         acc[i] = dadd(acc[i], dmul(v[u][i], x[u][i]));
-                    v[u][i] = k0 + U + u < len[i] ? __ldg(Vv + 32 * (k0 + U + u) + 8 * i) : 0.0;
+                    v[u][i] = k0 + U + u < len[i] ? __ldg(Vv + 32 * (k0 + U + u) + G * i) : 0.0;
                 }
         }
 #pragma unroll
@@ -1075,7 +1089,7 @@ void prepare_stream(abhsf_matrix& a, float avg, cudaStream_t st)
     a.dc_tree_flag.assign((size_t)a.tree_nrows, 0);
     a.dc_warps = a.dc_cwarps = 0;
     a.dc_every_row = false;
-    a.dc_elements = a.dc_rows = a.dc_slots = a.dc_lane_records = 0;
+    a.dc_elements = a.dc_rows = a.dc_slots = a.dc_lane_records = a.dc_steps = a.dc_longest = 0;
     const int s = a.s, lg = a.lg;
     if (avg <= 0.f || a.tree_nrows == 0 || a.sum_order != ABHSF_SUM_REFERENCE || (uint64_t)a.n > (uint64_t(1) << 32))
         return;
@@ -1315,6 +1329,10 @@ void prepare_stream(abhsf_matrix& a, float avg, cudaStream_t st)
     a.dc_every_row = ns == a.tree_nrows && nS + (int64_t)chain_q.size() == a.m;
     a.dc_slots = slots;
     a.dc_lane_records = 32 * nslices;
+    for (uint32_t t : steps) {
+        a.dc_steps += t;
+        a.dc_longest = std::max<int64_t>(a.dc_longest, t);
+    }
     deal_slices({&a}, a.dc_sched, a.dc_wbeg, a.dc_warps, st, 0, INT64_MAX, kDealSliced);
     deal_slices({&a}, a.dc_csched, a.dc_cwbeg, a.dc_cwarps, st, 0, INT64_MAX, kDealChains);
 }
@@ -1421,19 +1439,37 @@ dc_args batch_args(const abhsf_batch& b, const uint8_t* sched, const int64_t* wb
 // Column groups first in the grid: the groups of one slice run side by side
 // and share its words and values in L2.
 template <int S>
-void launch_mm(beside& bs, bool chains, const dc_args& P, cudaStream_t st)
+void launch_mm(beside& bs, bool chains, bool late, const dc_args& P, cudaStream_t st)
 {
     same_carveout<k_spmm_chains<S>>();
-    same_carveout<k_spmm_slices<S>>();
-    const unsigned groups = (unsigned)((P.cols + kMmCols - 1) / kMmCols);
+    same_carveout<k_spmm_slices<S, kMmCols, kMmLateCtas>>();
     const int per = chains ? kChainWarps : kMmWarps;
-    const dim3 grid(groups, (unsigned)((P.warps + per - 1) / per));
-    launch_beside(bs, chains ? k_spmm_chains<S> : k_spmm_slices<S>, grid, 32u * per, 0, st, P);
+    auto grid = [&](int cols) {
+        return dim3((unsigned)((cols + kMmCols - 1) / kMmCols), (unsigned)((P.warps + per - 1) / per));
+    };
+    if (chains) {
+        launch_beside(bs, k_spmm_chains<S>, grid(P.cols), 32u * per, 0, st, P);
+        return;
+    }
+    if (late) {
+        launch_beside(bs, k_spmm_slices<S, kMmCols, kMmLateCtas>, grid(P.cols), 32u * per, 0, st, P);
+        return;
+    }
+    dc_args R = P;
+    R.cols = P.cols / kMmWide * kMmWide;
+    if (R.cols > 0)
+        launch_beside(bs, k_spmm_slices<S, kMmWide, kMmCtas>, grid(R.cols), 32u * per, 0, st, R);
+    if (R.cols == P.cols)
+        return;
+    R.x = static_cast<const double*>(P.x) + R.cols;
+    R.y = static_cast<double*>(P.y) + R.cols;
+    R.cols = P.cols - R.cols;
+    launch_beside(bs, k_spmm_slices<S, kMmCols, kMmCtas>, grid(R.cols), 32u * per, 0, st, R);
 }
 
 // P.cols columns: the SpMV kernels for one, the SpMM ones (FP64) for more and
 // for one that is a column of a wider X or Y.
-void launch_cols(beside& bs, int s, int vt, bool chains, const dc_args& P, cudaStream_t st)
+void launch_cols(beside& bs, int s, int vt, bool chains, bool late, const dc_args& P, cudaStream_t st)
 {
     if (P.warps == 0)
         return;
@@ -1442,11 +1478,11 @@ void launch_cols(beside& bs, int s, int vt, bool chains, const dc_args& P, cudaS
         return;
     }
     switch (s) {
-    case 16: launch_mm<16>(bs, chains, P, st); break;
-    case 32: launch_mm<32>(bs, chains, P, st); break;
-    case 64: launch_mm<64>(bs, chains, P, st); break;
-    case 128: launch_mm<128>(bs, chains, P, st); break;
-    default: launch_mm<256>(bs, chains, P, st); break;
+    case 16: launch_mm<16>(bs, chains, late, P, st); break;
+    case 32: launch_mm<32>(bs, chains, late, P, st); break;
+    case 64: launch_mm<64>(bs, chains, late, P, st); break;
+    case 128: launch_mm<128>(bs, chains, late, P, st); break;
+    default: launch_mm<256>(bs, chains, late, P, st); break;
     }
 }
 
@@ -1461,6 +1497,8 @@ dc_plan plan_of(const abhsf_matrix& a)
     p.csched = a.dc_csched.get();
     p.cwbeg = a.dc_cwbeg.get();
     p.cwarps = a.dc_cwarps;
+    p.steps = a.dc_steps;
+    p.longest = a.dc_longest;
     return p;
 }
 
@@ -1468,14 +1506,17 @@ void slices_begin(beside& bs, const abhsf_matrix& a, const dc_plan& p, const voi
                   int64_t ldy, cudaStream_t st, int cols)
 {
     if (p.cwarps)
-        launch_cols(bs, a.s, a.value_type, true, args_of(a, p.csched, p.cwbeg, p.cwarps, x, ldx, y, ldy, cols), st);
+        launch_cols(bs, a.s, a.value_type, true, false, args_of(a, p.csched, p.cwbeg, p.cwarps, x, ldx, y, ldy, cols), st);
 }
 
 void slices_end(beside& bs, const abhsf_matrix& a, const dc_plan& p, const void* x, int64_t ldx, void* y, int64_t ldy,
                 cudaStream_t st, int cols)
 {
+    // 148 x 10 x 2 warps of the SpMM kernel share the steps of every four columns
+    const bool late = p.cwarps > 0 || p.longest * (148 * kMmLateCtas * kMmWarps) > p.steps * ((cols + 3) / 4);
     if (p.warps)
-        launch_cols(bs, a.s, a.value_type, false, args_of(a, p.sched, p.wbeg, p.warps, x, ldx, y, ldy, cols), st);
+        launch_cols(bs, a.s, a.value_type, false, late,
+                    args_of(a, p.sched, p.wbeg, p.warps, x, ldx, y, ldy, cols), st);
 }
 
 bool spmv_sets_y(const abhsf_matrix& a) { return a.dc_every_row; }
