@@ -97,14 +97,16 @@ constexpr uint32_t kDistinctRows = 1u << 26;
 // an SpMV, where a launch is most of the time (banded, 46 to 1,405 tiles: 9.0 us
 // against 11.3 with the slices beside; a mixture of 1,866 16.6 against 18.5, of
 // 6,244 20.5 against 21.5; banded of 4,687 12.3 either way).
-// Not where a block row of the slices has more than kSoloRowTiles tiles: one CTA
-// walks a block row, 0.2 to 1.3 us a tile, which the slices' lanes share.  A block
-// row of 4 tiles of 1 to 250 elements each took 9.3 to 12.4 us against 11.3 to
-// 13.1 with the slices (700 such beside 1,000 dense ones: 12.4 against 12.1 to
-// 12.5); of 6 tiles of 100, 12.4 against 11.8; of 16, 24.7 against 11.8; one of
-// 3,900 single elements 1,028 against 13.8.
+// Not where a block row of the slices takes long to walk: one CTA does, 0.2 us a
+// tile of one or two elements, 1 us from 30 on, which the slices' lanes share.  The
+// bound counts 8 and up to 32 elements a tile: 23 tiles of one, 5 of 32 or more.
+// A block row of 12 tiles of 8 (192) took 9.4 to 10.4 us against 11.7 with the
+// slices, 6 of 30 (228) 10.2 to 10.4, 8 of 30 (304) 12.4, 24 of one (216) 10.4 to
+// 12.4, 4 of 100 (160) 10.4, 6 of 100 (240) 12.4, 16 of 100 24.7; 700 of 4 of 50 to
+// 220 beside 1,000 dense ones 12.4 against 12.1 to 12.5; one of 3,900 single
+// elements 1,028 against 13.8.
 constexpr int64_t kSoloTiles = 4096;
-constexpr uint32_t kSoloRowTiles = 4;
+constexpr uint32_t kSoloWalk = 208, kSoloTileWalk = 8, kSoloNnzWalk = 32;
 
 // test hooks (abhsf_test_set_hooks)
 int64_t g_drop_desc = -1;
@@ -1248,6 +1250,17 @@ __global__ void k_ring_weight(int64_t nr, const uint32_t* __restrict__ rows, til
     }
 }
 
+// How long a CTA walks a block row (kSoloWalk).
+__global__ void k_solo_walk(int64_t nr, const uint32_t* __restrict__ rows, tiles_view A, uint32_t* __restrict__ walk)
+{
+    for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < nr; k += (int64_t)gridDim.x * blockDim.x) {
+        uint32_t w = 0;
+        for (int64_t t = A.brow_ptr[rows[k]]; t < A.brow_ptr[rows[k] + 1]; ++t)
+            w += kSoloTileWalk + min(A.tile_nnz[t], kSoloNnzWalk);
+        walk[k] = w;
+    }
+}
+
 __global__ void k_ring_fill(int64_t nitems, const uint32_t* __restrict__ rows, const int64_t* __restrict__ base,
                             tiles_view A, int s, uint32_t col_or, ring_desc* __restrict__ out)
 {
@@ -1529,7 +1542,7 @@ void tune_ring(abhsf_matrix& a, cudaStream_t st)
 // and writes every CTA's tile descriptors, matrix i's columns tagged with
 // i << col_bits.  Returns false when a CTA would get more tiles than its
 // counters hold.  with_slices: the block rows the slices serve, too -- false where
-// one of them has more than kSoloRowTiles tiles.
+// one of them takes longer than kSoloWalk to walk.
 bool build_ring_schedule(const std::vector<const abhsf_matrix*>& mats, int col_bits, dbuf<uint8_t>& desc,
                          dbuf<int64_t>& wbeg_d, int& ctas_out, int& max_pv_out, cudaStream_t st, int64_t brow_lo = 0,
                          int64_t brow_hi = INT64_MAX, bool with_slices = false)
@@ -1540,7 +1553,7 @@ bool build_ring_schedule(const std::vector<const abhsf_matrix*>& mats, int col_b
     ABHSF_CUDA(cudaGetDevice(&dev));
     ABHSF_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
     const int per_sm = ring_per_sm(s, vt);
-    std::vector<uint32_t> mid, rows, ntiles;
+    std::vector<uint32_t> mid, rows, ntiles, walk;
     std::vector<uint64_t> wt;
     int64_t total_tiles = 0;
     unsigned int mpv = 0;
@@ -1566,6 +1579,14 @@ bool build_ring_schedule(const std::vector<const abhsf_matrix*>& mats, int col_b
         wt.resize(o + nr);
         mid.resize(o + nr, (uint32_t)i);
         unsigned int m_pv = 0;
+        if (with_slices) {
+            walk.resize(o + nr);
+            scratch<uint32_t> walk_d(nr, st);
+            k_solo_walk<<<g, 256, 0, st>>>(nr, a.tree_rows.get(), a.view(), walk_d.get());
+            ABHSF_CUDA(cudaGetLastError());
+            ABHSF_CUDA(cudaMemcpyAsync(walk.data() + o, walk_d.get(), nr * sizeof(uint32_t), cudaMemcpyDeviceToHost,
+                                       st));
+        }
         ABHSF_CUDA(cudaMemcpyAsync(rows.data() + o, a.tree_rows.get(), nr * sizeof(uint32_t), cudaMemcpyDeviceToHost,
                                    st));
         ABHSF_CUDA(cudaMemcpyAsync(wt.data() + o, w_d.get(), nr * sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
@@ -1586,7 +1607,7 @@ bool build_ring_schedule(const std::vector<const abhsf_matrix*>& mats, int col_b
                 continue;
             for (int64_t k = 0; k < nr; ++k, ++o)
                 if ((size_t)k < f.size() && f[k]) {
-                    if (with_slices && ntiles[o] > kSoloRowTiles)
+                    if (with_slices && walk[o] > kSoloWalk)
                         return false;
                     if (!with_slices) {
                         skip[o] = 1;

@@ -14,14 +14,14 @@ def _matrix(s, dense, wide, z, seed):
     """`dense` diagonal tiles about 30% full (bitmaps), then a block row of
     `wide` tiles of z elements (COO, at the wide end z = 1), ragged at the end."""
     rng = np.random.default_rng(seed)
-    nb = max(dense + 1, wide)
+    nb = max(dense + 2, wide + 1)  # the last block row and column, cut by three, stay empty
     n = nb * s - 3
     rows, cols = [], []
     for d in range(dense):
         k = np.nonzero(rng.random(s * s) < 0.3)[0]
         rows.append(d * s + k // s)
         cols.append(d * s + k % s)
-    for J in rng.choice(nb, wide, replace=False):
+    for J in rng.choice(nb - 1, wide, replace=False):
         k = rng.choice(s * s, z, replace=False)
         rows.append(dense * s + k // s)
         cols.append(J * s + k % s)
@@ -55,12 +55,14 @@ def _check(r, c, v, n, s, vt, kernels):
 
 @pytest.mark.parametrize("vt", ["f64", "f32", "bf16"])
 @pytest.mark.parametrize("s", [32, 64])
-@pytest.mark.parametrize("wide,z", [(1, 30), (4, 40), (5, 40), (300, 8), (3000, 1)])
-def test_a_wide_sliced_block_row_keeps_its_slices(gpu, s, vt, wide, z):
-    """One CTA of the ring sums a whole block row: up to four tiles of a sliced
-    one are walked there, a wide one stays with the slices."""
-    r, c, v, n = _matrix(s, 9, wide, z, seed=wide)
-    _check(r, c, v, n, s, vt, 1 if wide <= 4 else 2)
+@pytest.mark.parametrize("wide,z,kernels", [(1, 30, 1), (5, 40, 1), (6, 40, 2), (13, 8, 1), (14, 8, 2), (23, 1, 1),
+                                            (24, 1, 2), (300, 8, 2), (3000, 1, 2)])
+def test_a_wide_sliced_block_row_keeps_its_slices(gpu, s, vt, wide, z, kernels):
+    """One CTA of the ring sums a whole block row: a sliced one is walked there
+    while its tiles at 8 and up to 32 elements each are no more than 208, a wider
+    one stays with the slices."""
+    r, c, v, n = _matrix(s, 30, wide, z, seed=wide)
+    _check(r, c, v, n, s, vt, kernels)
 
 
 @pytest.mark.parametrize("tiles,kernels", [(4096, 1), (4097, 2)])
