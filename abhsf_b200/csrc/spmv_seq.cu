@@ -436,6 +436,8 @@ __device__ __forceinline__ void seq_block_row(const tiles_view& A, const void* x
 // 103, f32 111 against 99).
 // Eight CTAs an SM at s = 16 (64 registers a thread, no spill; six leave 80): tiled
 // mixture FP64 305 -> 278 us, bf16 274 -> 254, f32 256 either way.
+// (bf16 at s = 16 is the other way round: 83 us with the wait after the loop, 92
+// without, on a tiled mixture of 20,000 rows: it always has it.)
 template <int S, int VT, bool B, bool BEHIND>
 __global__ void __launch_bounds__(kWarps * 32, S == 16 && !B ? 8 : kMinCtasPerSm) k_spmv_seq(seq_args P)
 {
@@ -473,7 +475,8 @@ void launch_seq(beside& bs, const abhsf_matrix& a, const uint32_t* rows, int64_t
     int dev = 0, nsm = 0, per_sm = 0;
     ABHSF_CUDA(cudaGetDevice(&dev));
     ABHSF_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    const auto kern = bs.any ? k_spmv_seq<S, VT, false, true> : k_spmv_seq<S, VT, false, false>;
+    constexpr bool kWait = S == 16 && VT == ABHSF_VALUE_BF16;  // (see k_spmv_seq)
+    const auto kern = bs.any ? k_spmv_seq<S, VT, false, true> : k_spmv_seq<S, VT, false, kWait>;
     ABHSF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kWarps * 32, 0));
     seq_args P{a.view(), rows, nrows, a.tree_counter.get(), x, y, nullptr, nullptr, nullptr, nullptr};
     const int64_t ctas = (nrows + kWarps - 1) / kWarps;
