@@ -59,6 +59,7 @@ constexpr int kChainGroup = 512;  // chain: elements a warp sums at a time, 16 a
 constexpr int kMmCols = 4;        // columns a warp of the SpMM kernels serves
 constexpr int kMmWide = 16;       // ... and of the sliced-row one where there are as many and no chains
 constexpr int kMmWarps = 2;       // sliced-row SpMM: warps a CTA (small ones fit beside the chains)
+constexpr int64_t kMmManySteps = 40;  // ... steps a warp from which on warps count for four columns
 constexpr int kMmCtas = 16, kMmLateCtas = 10;  // ... and CTAs an SM where warps count, and where latency does
 constexpr uint32_t kChain = 1u;   // dc_slice::geo: a one-row chain
 constexpr int kMidShift = 20;     // dc_slice::geo: matrix index of a batch
@@ -563,8 +564,10 @@ __global__ void __launch_bounds__(32 * kChainWarps, kChainCtasPerSm) k_spmv_chai
 // columns 54 us against 87 the other way.
 // Else bound by the lines a gather touches (4 columns a warp: eight a
 // load, 16: two) and by the warps to hide them: sixteen CTAs (64 registers, 48 to
-// 64 bytes spilled), and 16 columns a warp where there are as many, a step at a
-// time.  3D Laplacian 120^3, 2 / 8 / 16 / 32 columns: 118 / 237 / 445 / 866 us with
+// 64 bytes spilled; with four columns a warp from kMmManySteps on: 3D Laplacian
+// 60^3, 32 a warp at 8 columns, 34.5 us with ten and 38 with sixteen, 2D 700^2,
+// 52, 56 and 46), and 16 columns a warp where there are as many, a step at a time.
+// 3D Laplacian 120^3, 2 / 8 / 16 / 32 columns: 118 / 237 / 445 / 866 us with
 // ten CTAs and 4 columns a warp, 93 / 183 / 335 / 653 so (113 / 256 / 353 / 1,527
 // in passes of 2, 8, 16 and 32 columns before either).
 template <int S, int C, int CTAS>
@@ -1439,7 +1442,7 @@ dc_args batch_args(const abhsf_batch& b, const uint8_t* sched, const int64_t* wb
 // Column groups first in the grid: the groups of one slice run side by side
 // and share its words and values in L2.
 template <int S>
-void launch_mm(beside& bs, bool chains, bool late, const dc_args& P, cudaStream_t st)
+void launch_mm(beside& bs, bool chains, bool late, bool many, const dc_args& P, cudaStream_t st)
 {
     same_carveout<k_spmm_chains<S>>();
     same_carveout<k_spmm_slices<S, kMmCols, kMmLateCtas>>();
@@ -1451,7 +1454,7 @@ void launch_mm(beside& bs, bool chains, bool late, const dc_args& P, cudaStream_
         launch_beside(bs, k_spmm_chains<S>, grid(P.cols), 32u * per, 0, st, P);
         return;
     }
-    if (late) {
+    if (late) {  // (k_spmm_slices)
         launch_beside(bs, k_spmm_slices<S, kMmCols, kMmLateCtas>, grid(P.cols), 32u * per, 0, st, P);
         return;
     }
@@ -1464,12 +1467,13 @@ void launch_mm(beside& bs, bool chains, bool late, const dc_args& P, cudaStream_
     R.x = static_cast<const double*>(P.x) + R.cols;
     R.y = static_cast<double*>(P.y) + R.cols;
     R.cols = P.cols - R.cols;
-    launch_beside(bs, k_spmm_slices<S, kMmCols, kMmCtas>, grid(R.cols), 32u * per, 0, st, R);
+    launch_beside(bs, many ? k_spmm_slices<S, kMmCols, kMmCtas> : k_spmm_slices<S, kMmCols, kMmLateCtas>, grid(R.cols),
+                  32u * per, 0, st, R);
 }
 
 // P.cols columns: the SpMV kernels for one, the SpMM ones (FP64) for more and
 // for one that is a column of a wider X or Y.
-void launch_cols(beside& bs, int s, int vt, bool chains, bool late, const dc_args& P, cudaStream_t st)
+void launch_cols(beside& bs, int s, int vt, bool chains, bool late, bool many, const dc_args& P, cudaStream_t st)
 {
     if (P.warps == 0)
         return;
@@ -1478,11 +1482,11 @@ void launch_cols(beside& bs, int s, int vt, bool chains, bool late, const dc_arg
         return;
     }
     switch (s) {
-    case 16: launch_mm<16>(bs, chains, late, P, st); break;
-    case 32: launch_mm<32>(bs, chains, late, P, st); break;
-    case 64: launch_mm<64>(bs, chains, late, P, st); break;
-    case 128: launch_mm<128>(bs, chains, late, P, st); break;
-    default: launch_mm<256>(bs, chains, late, P, st); break;
+    case 16: launch_mm<16>(bs, chains, late, many, P, st); break;
+    case 32: launch_mm<32>(bs, chains, late, many, P, st); break;
+    case 64: launch_mm<64>(bs, chains, late, many, P, st); break;
+    case 128: launch_mm<128>(bs, chains, late, many, P, st); break;
+    default: launch_mm<256>(bs, chains, late, many, P, st); break;
     }
 }
 
@@ -1506,16 +1510,17 @@ void slices_begin(beside& bs, const abhsf_matrix& a, const dc_plan& p, const voi
                   int64_t ldy, cudaStream_t st, int cols)
 {
     if (p.cwarps)
-        launch_cols(bs, a.s, a.value_type, true, false, args_of(a, p.csched, p.cwbeg, p.cwarps, x, ldx, y, ldy, cols), st);
+        launch_cols(bs, a.s, a.value_type, true, false, false, args_of(a, p.csched, p.cwbeg, p.cwarps, x, ldx, y, ldy, cols), st);
 }
 
 void slices_end(beside& bs, const abhsf_matrix& a, const dc_plan& p, const void* x, int64_t ldx, void* y, int64_t ldy,
                 cudaStream_t st, int cols)
 {
-    // 148 x 10 x 2 warps of the SpMM kernel share the steps of every four columns
-    const bool late = p.cwarps > 0 || p.longest * (148 * kMmLateCtas * kMmWarps) > p.steps * ((cols + 3) / 4);
+    // SpMM: 148 x 10 x 2 warps share the steps of every four columns
+    const int64_t warps = 148 * kMmLateCtas * kMmWarps, steps = p.steps * ((cols + 3) / 4);
+    const bool late = p.cwarps > 0 || p.longest * warps > steps, many = steps >= kMmManySteps * warps;
     if (p.warps)
-        launch_cols(bs, a.s, a.value_type, false, late,
+        launch_cols(bs, a.s, a.value_type, false, late, many,
                     args_of(a, p.sched, p.wbeg, p.warps, x, ldx, y, ldy, cols), st);
 }
 
