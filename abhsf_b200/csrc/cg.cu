@@ -15,10 +15,11 @@
 // the state's `done` flag turns the rest of the chunk into no-ops; where the
 // SpMV heeds the flag too, a chunk is queued before the state after the one
 // before it has been read.
-// Bound by memory for large systems (the vector kernels move eight vectors an
-// iteration: dot 2, residual 3, direction 5, less one the SpMV need not read,
-// where a kernel each for x and r, and for p, moved eleven) and by the launches
-// for small ones.
+// Bound by memory for large systems and by the launches for small ones.  The
+// vector kernels move ten vectors an iteration (dot 2, residual 3, direction 5),
+// and the SpMV that sets y does not read it; where it adds, the residual kernel
+// clears Ap too, eleven.  A kernel each for the dot, for x and r, and for p moved
+// twelve.
 #include <cmath>
 #include <vector>
 

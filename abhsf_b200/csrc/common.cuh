@@ -238,7 +238,7 @@ struct abhsf_matrix {
     std::vector<uint8_t> dc_tree_flag;   // per non-empty block row (tree_rows order): served by the slices
     abhsf::dbuf<uint32_t> dc_words;      // one word per slot (delta-coded columns)
     abhsf::dbuf<uint8_t> dc_vals;        // the values in slot order
-    abhsf::dbuf<uint32_t> dc_lane;       // lane records: row << 24 | length
+    abhsf::dbuf<uint32_t> dc_lane;       // lane records: row offset << 8 | length - 1
     abhsf::dbuf<uint8_t> dc_sched;       // the matrix's own launch: sliced rows in warp order
     abhsf::dbuf<int64_t> dc_wbeg;
     int dc_warps = 0;

@@ -1862,7 +1862,7 @@ void prepare_batch(abhsf_batch& b, cudaStream_t st)
 void batch_spmv(const abhsf_batch& b, const double* const* xs, double* const* ys, cudaStream_t st)
 {
     beside bs;
-// The ring first: a chain CTA's 73 KB would keep two of the ring's five CTAs
+    // The ring first: a chain CTA's 73 KB would keep two of the ring's five CTAs
     // from an SM (chains first 844 us, ring first 791, on the 256-matrix batch).
     if (b.ctas > 0)
         batch_launch(bs, b, xs, ys, st, false);

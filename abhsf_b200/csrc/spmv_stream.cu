@@ -26,11 +26,12 @@
 // running sum of the deltas, x gathered through L2 -- and adds each product
 // onto its row's sum in column order, starting from y: the order of the
 // reference CSR's spmv_naive (spmv/bottlenecks/spmv.cpp:58-64), so y is
-// bitwise the same.  A chain (its own kernel, queued first and run beside the
-// others): 512 products at a time,
-// a segment a lane, added in order to the bit by the rule of chain_sum.cuh.
-// Slices and chains are dealt to warps at preparation time, longest first.  No waits: nothing here can stall on
-// another warp.
+// bitwise the same.  A chain (its own kernel, beside the others): 512 products
+// at a time, in turn or a segment a lane by the rule of chain_sum.cuh, which
+// gives the same bits.  For one matrix the chains are queued first (the longest
+// bounds the product), in a batch behind the ring kernel, whose CTAs they would
+// keep from an SM.  Slices and chains are dealt to warps at preparation time,
+// longest first.  Nothing here stalls on another warp.
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
